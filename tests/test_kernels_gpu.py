@@ -85,6 +85,19 @@ def test_gemm_simt(kernels, dtype, m, n, k):
         assert torch.equal(kernels.gemm_simt(a[m // 2 : m // 2 + 1].contiguous(), w), kernels.gemm_simt(a, w)[m // 2 : m // 2 + 1])
 
 
+@pytest.mark.parametrize("n,k", [(31, 4), (64, 32), (129, 100), (300, 1028), (37900, 36)])
+def test_gemm_simt_forms_agree_bit_for_bit(kernels, n, k):
+    """Few rows, every size of tile, rows that do not start on 16 bytes: every output is the same chain of fused multiply-adds over k."""
+    a, w = rand((600, k), torch.float32, 8), rand((n, k), torch.float32, 9)
+    wide = torch.zeros((600, k + 1), device="cuda")
+    wide[:, 1:] = a
+    rows = kernels.gemm_simt(wide[:, 1:], w)                # neither an aligned row nor a whole stride: an element at a time
+    want = a.double().cpu() @ w.double().cpu().T
+    close(rows, want, torch.float32, "gemm an element at a time", scale=k * 2.0 ** -23 / 2e-6 + 1)      # as in test_gemm_simt
+    for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 33, 127, 600):
+        assert torch.equal(kernels.gemm_simt(a[:m], w), rows[:m]), f"{m} rows"
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nq,nkv,d,rot,page", [(4, 2, 16, 16, 16), (6, 1, 32, 32, 8), (5, 5, 48, 32, 4), (8, 2, 128, 128, 16), (3, 1, 80, 80, 32)])
 def test_qk_norm_rope_cache(kernels, dtype, nq, nkv, d, rot, page):

@@ -290,6 +290,32 @@ def test_paged_attention_mixed_rows(kernels, dtype, window, nq, nkv, d, page):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("window", [None, 1, 40])
+@pytest.mark.parametrize("nq,nkv,d,page", [(4, 4, 4, 16), (6, 2, 20, 8), (32, 1, 64, 16), (10, 2, 100, 16), (16, 8, 128, 16)])
+def test_paged_attention_forms_agree_bit_for_bit(kernels, dtype, window, nq, nkv, d, page):
+    """A block of many rows and a block of one token make the same sums in the same order: the query's address alone (off a whole piece of
+    four numbers) sends the second call to the form for any sizes. Values that are not finite stay with the rows that see them."""
+    g = torch.Generator().manual_seed(15)
+    lens, news = [33, 1, 97, 300, 7, 64], [33, 1, 40, 1, 2, 64]
+    keys, values = ([torch.randn(n, nkv, d, generator=g).to(dtype).double() for n in lens] for _ in range(2))
+    values[2][-3], values[5][20, 0, 1] = float("inf"), float("nan")
+    positions = [i for n, m in zip(lens, news) for i in range(n - m, n)] + [-1, -1]        # a padding row's tokens at the end
+    rows = [b for b, m in enumerate(news) for _ in range(m)] + [len(lens)] * 2
+    kp, vp, indptr, indices = build_paged(keys, values, page, dtype, num_pages=sum(-(-n // page) for n in lens) + 3, seed=16)
+    if window:
+        release_passed_pages(kp, vp, indptr, indices, lens, news, window, page)
+    indptr = torch.cat([indptr, indptr[-1:]])
+    flat = torch.zeros(len(positions) * nq * d + 1, dtype=dtype, device="cuda")
+    flat[1:] = (torch.randn(len(positions) * nq * d, generator=g) * 1.5).to(dtype).cuda()
+    q = flat[1:].view(len(positions), nq, d)
+    args = (kp, vp, torch.tensor(positions, dtype=torch.int32).cuda(), torch.tensor(rows, dtype=torch.int32).cuda(), indptr, indices, d ** -0.5, window)
+    want = kernels.paged_attention_generic(q, *args)
+    got = kernels.paged_attention_generic(q.clone(), *args)
+    assert torch.equal(got.nan_to_num(nan=-7.0), want.nan_to_num(nan=-7.0))
+    assert torch.isfinite(want).float().mean() > 0.5 and not torch.isfinite(want).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("case", ["far key", "first key", "page edge", "window edge in", "window edge out"])
 def test_paged_attention_finds_the_one_key_that_matters(kernels, dtype, case):
     """Random keys would hide a key that is skipped or read from the wrong slot. Here one key's score stands out by

@@ -331,3 +331,33 @@ def test_the_command_line_writes_a_vamatar_folder_and_generates_from_it(tmp_path
         top = logits[len(prompt) - 1 + j].topk(2)
         if float(top.values[0] - top.values[1]) > 1e-3:
             assert tok == int(top.indices[0]), (j, tok, int(top.indices[0]))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("lengths,channels", [([1, 2, 3, 4, 37], 24), ([3000, 1, 2000], 1032)])
+def test_convolution_forms_agree_bit_for_bit(kernels, dtype, lengths, channels):
+    """Sixteen tokens a thread, one, and a number at a time (columns that start off a whole piece): the same sums."""
+    T = sum(lengths)
+    g = torch.Generator().manual_seed(T)
+    u = torch.randn(T, channels + 16, generator=g).to(dtype).cuda()
+    shifted = torch.zeros_like(u)
+    shifted[:, 9 : 9 + channels] = u[:, 8 : 8 + channels]
+    w, bias = torch.randn(channels, 4, generator=g).cuda(), torch.randn(channels, generator=g).cuda()
+    state = torch.randn(len(lengths) + 1, 8 + 3 * channels, generator=g).cuda()
+    rows = torch.tensor([r for r, n in enumerate(lengths) for _ in range(n)], dtype=torch.int32).cuda()
+    q_indptr = torch.tensor([0] + list(np.cumsum(lengths)), dtype=torch.int32).cuda()
+    slots = torch.arange(len(lengths), 0, -1, dtype=torch.int32).cuda()
+    args = (channels, w, bias, state, 8, rows, q_indptr, slots)
+    assert torch.equal(kernels.mamba2_conv(u, 8, *args), kernels.mamba2_conv(shifted, 9, *args))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("size,groups", [(4, 3), (36, 2), (256, 2), (512, 8), (1024, 1), (1028, 3), (2048, 1), (4100, 1), (8192, 1), (8196, 1), (50, 1)])
+def test_gated_group_norm_at_every_width(kernels, dtype, size, groups):
+    g = torch.Generator().manual_seed(size)
+    y, w = torch.randn(5, size * groups, generator=g).cuda() * 3, torch.randn(size * groups, generator=g).cuda()
+    u = torch.randn(5, size * groups + 4, generator=g).to(dtype).cuda()
+    z = u.double().cpu()[:, : size * groups]
+    v = y.double().cpu() * z * torch.sigmoid(z)
+    want = P.unit_rms(v.reshape(5, groups, size), 1e-6).reshape(5, -1) * w.double().cpu()
+    close(kernels.gated_group_norm(y, u, w, groups, 1e-6, dtype), want, dtype, "gated group norm")

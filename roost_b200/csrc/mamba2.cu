@@ -536,6 +536,13 @@ static void launch_scan(const void* xbc, const void* u, int64_t ld_u, int dt_col
                 a_log, d_skip, state, state_stride, q_indptr, slots, heads, P, N, groups);
 }
 
+namespace roost {
+bool mamba2_chunks_serve(int rows, int tokens, int heads, int head_dim, int state_rows, int groups, int dtype);
+int mamba2_chunks(const void* xbc, const void* u, int64_t ld_u, int dt_col, float* y, const float* dt_bias, const float* a_log, const float* d_skip, float* state,
+                  int64_t state_stride, const int32_t* q_indptr, const int32_t* slots, int rows, int tokens, int heads, int state_rows, int groups, float* ws_state,
+                  float* ws_decay, cudaStream_t stream);
+}  // namespace roost
+
 extern "C" int roost_mamba2_scan(const void* xbc, const void* u, int64_t ld_u, int dt_col, float* y, const float* dt_bias, const float* a_log,
                                  const float* d_skip, float* state, int64_t state_stride, const int32_t* q_indptr, const int32_t* slots,
                                  int rows, int tokens, int heads, int head_dim, int state_rows, int groups, float* ws_state, float* ws_decay,
@@ -546,6 +553,12 @@ extern "C" int roost_mamba2_scan(const void* xbc, const void* u, int64_t ld_u, i
   if (heads > 65535) return fail(ROOST_ERR_UNSUPPORTED, "mamba2_scan: too many heads");
   if (rows == 0) return ROOST_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  if (mamba2_chunks_serve(rows, tokens, heads, head_dim, state_rows, groups, dtype)) {
+    if ((uintptr_t)xbc % 16 == 0 && (uintptr_t)state % 8 == 0 && state_stride % 2 == 0 && (uintptr_t)ws_state % 16 == 0)
+      return mamba2_chunks(xbc, u, ld_u, dt_col, y, dt_bias, a_log, d_skip, state, state_stride, q_indptr, slots, rows, tokens, heads, state_rows, groups, ws_state,
+                           ws_decay, s);
+    ws_state = nullptr;      // sized for the parts of that form
+  }
   {
     // whole 16-byte pieces everywhere: the form that reads shared memory in vectors and prefetches
     const int vec = dtype == ROOST_F32 ? 4 : 8;

@@ -326,6 +326,9 @@ int roost_mamba2_scan(const void* xbc, const void* u, int64_t ld_u, int dt_col, 
  * roost_mamba2_scan_chunks(tokens, rows), roost_mamba2_scan cuts long rows into chunks that run side by side; with null
  * pointers it walks every row in one pass. */
 int roost_mamba2_scan_chunks(int tokens, int rows);
+/* Where roost_mamba2_scan walks a step of these sizes in chunks on the tensor cores (mamba2_chunks.cu): the parts its rows are cut into, to take
+ * the place of `chunks` in the workspaces' sizes (0: none are needed); -1 elsewhere. */
+int roost_mamba2_scan_parts(int rows, int tokens, int heads, int head_dim, int state_rows, int groups, int dtype);
 int roost_gated_group_norm(const float* y, const void* u, int64_t ld_u, const float* w, void* out, int tokens, int inner, int groups,
                            float eps, int dtype, roost_stream_t stream);
 

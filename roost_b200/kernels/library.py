@@ -141,6 +141,7 @@ _SIGNATURES = {
     "roost_mamba2_scan": [c_void_p, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
                           c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p],
     "roost_mamba2_scan_chunks": [c_int, c_int],
+    "roost_mamba2_scan_parts": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
     "roost_gated_group_norm": [c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p],
     "roost_moe_tile_rows": [],
     "roost_moe_router_logits": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
@@ -794,8 +795,10 @@ class KernelLibrary:
         T = xbc.shape[0]
         y = torch.empty((T, heads * head_dim), dtype=torch.float32, device=xbc.device)
         ws_state = ws_decay = None
-        if T >= self.SCAN_CHUNKED_MIN_TOKENS:       # long rows are cut into chunks that run side by side
-            chunks = self._lib.roost_mamba2_scan_chunks(T, slots.numel())
+        chunks = self._lib.roost_mamba2_scan_parts(slots.numel(), T, heads, head_dim, state_rows, groups, dtype_code(xbc.dtype))
+        if chunks < 0:       # long rows are cut into chunks that run side by side
+            chunks = self._lib.roost_mamba2_scan_chunks(T, slots.numel()) if T >= self.SCAN_CHUNKED_MIN_TOKENS else 0
+        if chunks:
             ws_state = torch.empty((chunks * heads * head_dim * state_rows,), dtype=torch.float32, device=xbc.device)
             ws_decay = torch.empty((chunks * heads,), dtype=torch.float32, device=xbc.device)
         self._call("roost_mamba2_scan", _ptr(xbc), _ptr(u), u.stride(0), dt_col, _ptr(y), _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(state),

@@ -333,6 +333,54 @@ def test_the_command_line_writes_a_vamatar_folder_and_generates_from_it(tmp_path
             assert tok == int(top.indices[0]), (j, tok, int(top.indices[0]))
 
 
+def _recurrence_in_64_bits(xbc, dt, dt_bias, a_log, d, state, lengths, heads, N, groups):
+    """y and the states after the rows, token by token; ``state`` [rows, heads, 64, N]."""
+    H, S, at, ys = heads, state.double().cpu().clone(), 0, []
+    x, B, C = xbc.double().cpu().split([H * 64, groups * N, groups * N], -1)
+    x, (B, C) = x.reshape(-1, H, 64), (t.reshape(-1, groups, N).repeat_interleave(H // groups, 1) for t in (B, C))
+    dt = torch.nn.functional.softplus(dt.double().cpu() + dt_bias.double().cpu())
+    fade = torch.exp(-torch.exp(a_log.double().cpu()) * dt)
+    for r, n in enumerate(lengths):
+        for t in range(at, at + n):
+            S[r] = fade[t][:, None, None] * S[r] + (dt[t][:, None] * x[t])[:, :, None] * B[t][:, None]
+            ys.append(torch.einsum("hpn,hn->hp", S[r], C[t]) + d.double().cpu()[:, None] * x[t])
+        at += n
+    return torch.stack(ys).reshape(at, -1), S
+
+
+@pytest.mark.parametrize("odd", [False, True])
+@pytest.mark.parametrize("N,groups,lengths", [(64, 1, [64, 65]), (128, 2, [1, 300, 17]), (128, 4, [63, 128]), (64, 2, [8, 9, 1, 200])])
+def test_recurrence_in_chunks_on_the_tensor_cores(kernels, N, groups, lengths, odd):
+    """Edges of chunks, rows of one token, carried states, decays from none to complete; against 64 bits, and no further from it than the
+    walk in 32 bits over the same numbers. A value that is not finite shows from its own token on and not before."""
+    H, T = 4, sum(lengths)
+    g = torch.Generator().manual_seed(N + len(lengths))
+    xbc = torch.randn(T, H * 64 + 2 * groups * N, generator=g).to(torch.bfloat16)
+    u = torch.zeros(T, 8 + H)
+    u[:, 8:] = torch.randn(T, H, generator=g)
+    u = u.to(torch.bfloat16)
+    dt_bias, d = torch.randn(H, generator=g), torch.randn(H, generator=g)
+    a_log = torch.tensor([-3.0, -1.0, 1.0, 4.0])
+    state = torch.randn(len(lengths), H * 64 * N, generator=g)
+    if odd:
+        xbc[T - 6, 70], u[T - 6, 9] = float("inf"), float("inf")
+    want, S = _recurrence_in_64_bits(xbc, u[:, 8:].float(), dt_bias, a_log, d, state.reshape(len(lengths), H, 64, N), lengths, H, N, groups)
+    q_indptr = torch.tensor([0] + list(np.cumsum(lengths)), dtype=torch.int32).cuda()
+    slots = torch.arange(len(lengths), dtype=torch.int32).cuda()
+    got = {}
+    for dtype in DTYPES:
+        s = state.cuda()
+        y = kernels.mamba2_scan(xbc.to(dtype).cuda(), u.to(dtype).cuda(), 8, dt_bias.cuda(), a_log.cuda(), d.cuda(), s, q_indptr, slots, H, 64, N, groups)
+        got[dtype] = (y.double().cpu(), s.double().cpu().reshape(S.shape))
+    for name, w, k in (("y", want, 0), ("state", S, 1)):
+        fine = torch.isfinite(w)
+        assert torch.equal(torch.isfinite(got[torch.bfloat16][k]), fine) and torch.equal(torch.isfinite(got[torch.float32][k]), fine), name
+        off = {t: float((got[t][k] - w)[fine].norm() / w[fine].norm()) for t in DTYPES}
+        print(f"MEASURED recurrence in chunks {name}: tensor cores {off[torch.bfloat16]:.2e}, walk {off[torch.float32]:.2e}")
+        # float32 sums of up to N and 64 terms: a few units of 2^-24, whichever the order
+        assert off[torch.bfloat16] < max(2 * off[torch.float32], 1e-6), (name, off)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("lengths,channels", [([1, 2, 3, 4, 37], 24), ([3000, 1, 2000], 1032)])
 def test_convolution_forms_agree_bit_for_bit(kernels, dtype, lengths, channels):

@@ -1259,7 +1259,7 @@ bool prefill_tc_serves(int head_dim, int q_heads, int kv_heads, int page_size, l
                        const void* q);
 int launch_prefill_tc(const void* q, long long tokens, void* out, const void* k_pool, const void* v_pool, const int32_t* q_indptr,
                       const int32_t* kv_lens, const int32_t* kv_indptr, const int32_t* kv_indices, const int32_t* work, int items, int tile_rows,
-                      int q_heads, int kv_heads, int head_dim, int page_size, long long pool_pages, float scale, int window, cudaStream_t s);
+                      int q_heads, int kv_heads, int head_dim, int page_size, long long pool_pages, float scale, int window, const float* sinks, cudaStream_t s);
 void set_prefill_tc(bool on);
 int prefill_tc_status();
 
@@ -1422,7 +1422,7 @@ extern "C" int roost_attention_prefill_tile_rows(int head_dim, int q_heads, int 
   return head_dim <= 128 && packed_rows * kv_heads >= kPrefillWideMinRows ? 128 : 64;
 }
 
-// The same for a caller that asks for wide weights (ROOST_ATTENTION_WIDE_WEIGHTS), which the mma.sync kernels serve.
+// The same for a caller that asks for what only the mma.sync kernels serve (a cap on the scores, kept keys).
 extern "C" int roost_attention_prefill_tile_rows_mma(int head_dim, int kv_heads, long long packed_rows) {
   if (!roost_attention_mma_supported(head_dim)) return 0;
   return head_dim <= 128 && packed_rows * kv_heads >= kPrefillWideMinRows ? 128 : 64;
@@ -1470,13 +1470,12 @@ static int attention_prefill(const void* q, long long tokens, void* out, const v
   if (kv_heads > 65535) return fail(ROOST_ERR_UNSUPPORTED, "attention_prefill: more than 65535 key/value heads");
   if (items == 0) return ROOST_OK;
   ROOST_REQUIRE(softcap >= 0.f && (softcap == 0.f || tile_rows != 256), "attention_prefill: a cap on the scores is served by the mma.sync kernels (items of 64 or 128 packed rows)");
-  if ((tile_rows == 128 || tile_rows == 256) && tokens > 0 && !(window & ROOST_ATTENTION_WIDE_WEIGHTS) && softcap == 0.f && sinks == nullptr && keep_first == 0 &&
+  if ((tile_rows == 128 || tile_rows == 256) && tokens > 0 && softcap == 0.f && keep_first == 0 &&
       prefill_tc_serves(head_dim, q_heads, kv_heads, page_size, pool_pages, k_pool, v_pool, q)) {
     return launch_prefill_tc(q, tokens, out, k_pool, v_pool, q_indptr, kv_lens, kv_indptr, kv_indices, work, items, tile_rows, q_heads, kv_heads,
-                             head_dim, page_size, pool_pages, scale, window, (cudaStream_t)stream);
+                             head_dim, page_size, pool_pages, scale, window, sinks, (cudaStream_t)stream);
   }
-  ROOST_REQUIRE(tile_rows != 256 || (!(window & ROOST_ATTENTION_WIDE_WEIGHTS) && sinks == nullptr && keep_first == 0),
-                "attention_prefill: work items of 256 packed rows belong to the tcgen05 kernel, which takes no wide weights, stored sinks or kept keys");
+  ROOST_REQUIRE(tile_rows != 256 || keep_first == 0, "attention_prefill: work items of 256 packed rows belong to the tcgen05 kernel, which takes no kept keys");
   ROOST_REQUIRE(keep_first >= 0, "attention_prefill: the number of kept keys cannot be negative");
   if (tile_rows == 128) {
     switch (head_dim) {

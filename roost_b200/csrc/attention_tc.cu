@@ -23,6 +23,9 @@
 //     against moves only when the new maximum exceeds it by more than 2^8 (the weights then stay below 2^8, well inside
 //     bfloat16's and float32's range, and the quotient at the end is the same): the row of the output accumulator is
 //     rescaled in tensor memory only then.
+// Wide weights (WIDE): a row's weights enter the second product as two bfloat16 operands, their rounding and what it left over, so that 16 bits
+// of the 32-bit weights count: the second operands lie over the other half of the scores' columns, and every product with V is made twice. Rows of 1,500, 500 and 2,048 tokens, 16
+// heads of 128 over 4, with a sink: 64 us, 243 with the mma.sync kernel that served wide weights before.
 // Value rows at positions the request does not hold yet (the rest of its last page) or before the CTA's first visible key
 // are zeroed in shared memory before the second product, so that whatever the pool holds there cannot reach a result;
 // their scores are masked by position. Every wait is bounded (see tma.cuh): a wait given up raises the CTA's abort flag
@@ -64,15 +67,15 @@ struct TcCfg {
 // longest first. Tensor memory and the barriers are set up once; the rings of keys and values, the score columns and the
 // barriers' phases run on from one pair to the next, so the copies of the next pair start while the last tiles of this
 // one are still being computed.
-template <int D, int RPC, int NG>
+template <int D, int RPC, int NG, bool WIDE>
 __global__ void __launch_bounds__(64 + NG * 128, 1)
     attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                 const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out, const int32_t* __restrict__ q_indptr,
                                 const int32_t* __restrict__ kv_lens, const int32_t* __restrict__ kv_indptr,
                                 const int32_t* __restrict__ kv_indices, const int2* __restrict__ work, int items, int q_heads, int kv_heads,
-                                int page_size, float scale_log2, int window) {
-  const float sink = (window & ROOST_ATTENTION_SINK) ? 1.0f : 0.f;     // one more term, 2^(0 - m), in every row's denominator
-  window &= ~(ROOST_ATTENTION_SINK | ROOST_ATTENTION_WIDE_WEIGHTS);      // a caller that wants wide weights is not sent here
+                                int page_size, float scale_log2, int window, const float* __restrict__ sinks) {
+  const float sink = (window & ROOST_ATTENTION_SINK) ? 1.0f : 0.f;     // one more term, 2^(0 - m) or 2^(a head's stored number - m), in every row's denominator
+  window &= ~(ROOST_ATTENTION_SINK | ROOST_ATTENTION_WIDE_WEIGHTS);
   using Cfg = TcCfg<D, NG>;
   constexpr int BM = kTcRows, TK = kTcKeys, KS = Cfg::kKStages, VS = Cfg::kVStages, NP = TK / RPC, CB = D / 64;
   constexpr uint32_t kQBytes = BM * D * 2;                  // one row group's Q tile
@@ -283,6 +286,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
             const uint32_t v_rows = v0 + (uint32_t)((kk * 16) / RPC) * kVPage + (uint32_t)((kk * 16) % RPC) * 128;
             const uint64_t b_desc = umma_desc_mn_major_sw128(v_rows, RPC * 128, 1024);
             tcgen05_mma_f16_ts(tmem_o(g), tmem_s(g, sb) + (uint32_t)(kk * 8), b_desc, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+            if (WIDE) tcgen05_mma_f16_ts(tmem_o(g), tmem_s(g, sb) + (uint32_t)(TK / 2 + kk * 8), b_desc, idesc_o, 1u);
           }
           tcgen05_commit(v_empty((kt0 + i) % VS));  // the values are free (for this group) once these products have read them
           if (p.g_first[g] + j == p.g_last[g]) tcgen05_commit(o_done(g));
@@ -399,13 +403,17 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
         }
         const float msafe = m == -INFINITY ? 0.f : m;  // a row that has seen no key yet: every weight below is 0
         float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t packed[TK / 2];
+        uint32_t packed[TK / 2], rest[WIDE ? TK / 2 : 1];
 #pragma unroll
         for (int e = 0; e < TK; e += 2) {
           const float p0 = ex2(fmaf(s[e], scale_log2, -msafe)), p1 = ex2(fmaf(s[e + 1], scale_log2, -msafe));
           sum4[(e / 2) & 3] += p0 + p1;
           __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
           packed[e / 2] = *reinterpret_cast<uint32_t*>(&pb);
+          if (WIDE) {
+            __nv_bfloat162 rb = __floats2bfloat162_rn(p0 - __uint_as_float(packed[e / 2] << 16), p1 - __uint_as_float(packed[e / 2] & 0xffff0000u));
+            rest[e / 2] = *reinterpret_cast<uint32_t*>(&rb);
+          }
         }
         l = l * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
         // The accumulator holds the pair's tiles 0 .. j - 1 once the second product of tile j - 1 is done. With one set
@@ -444,6 +452,11 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
         // the row's weights, two bfloat16 a column, over the first half of the scores' columns
 #pragma unroll
         for (int c = 0; c < TK / 64; ++c) tcgen05_st_32x32b_x32_nowait(tmem_s(g, sb) + lane_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&packed[c * 32]));
+        if (WIDE) {
+#pragma unroll
+          for (int c = 0; c < TK / 64; ++c)
+            tcgen05_st_32x32b_x32_nowait(tmem_s(g, sb) + lane_addr + TK / 2 + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&rest[WIDE ? c * 32 : 0]));
+        }
         tcgen05_wait_st();
         tcgen05_fence_before();
         __syncwarp();
@@ -453,7 +466,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
       if (ok && my_tiles > 0) ok = mbar_wait_limited(o_done(g), (uint32_t)outs & 1u, abortp, 8, &g_attention_tc_error);
       if (ok && my_tiles > 0) {
         tcgen05_fence_after();
-        l += sink * ex2(-(m == -INFINITY ? 0.f : m));
+        if (sink != 0.f) l += ex2((sinks != nullptr && valid ? sinks[p.kvh * group + pr % group] * kLog2eTc : 0.f) - (m == -INFINITY ? 0.f : m));
         const float inv = l > 0.f ? 1.0f / l : 0.f;
         __nv_bfloat16* dst = valid ? out + ((size_t)(p.q_start + pr / group) * q_heads + p.kvh * group + pr % group) * D : nullptr;
 #pragma unroll 1
@@ -513,12 +526,12 @@ bool prefill_tc_serves(int head_dim, int q_heads, int kv_heads, int page_size, l
   return (uintptr_t)k_pool % 128 == 0 && (q == nullptr || (uintptr_t)q % 16 == 0) && encode_tiled() != nullptr;
 }
 
-template <int D, int RPC, int NG>
+template <int D, int RPC, int NG, bool WIDE>
 static int launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out, const int32_t* q_indptr, const int32_t* kv_lens,
                      const int32_t* kv_indptr, const int32_t* kv_indices, const int32_t* work, int items, int q_heads, int kv_heads,
-                     int page_size, float scale, int window, cudaStream_t s) {
+                     int page_size, float scale, int window, const float* sinks, cudaStream_t s) {
   constexpr size_t smem = TcCfg<D, NG>::kSmem;
-  auto kernel = attention_prefill_tc_kernel<D, RPC, NG>;
+  auto kernel = attention_prefill_tc_kernel<D, RPC, NG, WIDE>;
   static int sms[64] = {};   // per device: its SM count, and that the kernel's shared-memory size has been set there
   int dev = 0;
   cudaGetDevice(&dev);
@@ -534,13 +547,13 @@ static int launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   const long long pairs = (long long)items * kv_heads;
   const int grid = (int)(pairs <= 8LL * sms[dev] ? (pairs < sms[dev] ? pairs : sms[dev]) : pairs);
   launch_kernel(kernel, dim3(grid), dim3(64 + NG * 128), smem, s, mq, mk, mv, (__nv_bfloat16*)out, q_indptr, kv_lens, kv_indptr, kv_indices,
-                (const int2*)work, items, q_heads, kv_heads, page_size, scale * kLog2eTc, window);
+                (const int2*)work, items, q_heads, kv_heads, page_size, scale * kLog2eTc, window, sinks);
   return check_launch("attention_prefill_tc");
 }
 
 int launch_prefill_tc(const void* q, long long tokens, void* out, const void* k_pool, const void* v_pool, const int32_t* q_indptr,
                       const int32_t* kv_lens, const int32_t* kv_indptr, const int32_t* kv_indices, const int32_t* work, int items, int tile_rows,
-                      int q_heads, int kv_heads, int head_dim, int page_size, long long pool_pages, float scale, int window, cudaStream_t s) {
+                      int q_heads, int kv_heads, int head_dim, int page_size, long long pool_pages, float scale, int window, const float* sinks, cudaStream_t s) {
   if (tile_rows != 128 && tile_rows != 256) return fail(ROOST_ERR_INVALID, "attention_prefill: the tcgen05 kernel takes work items of 128 or 256 packed rows");
   const int groups = tile_rows / kTcRows;
   const int group = q_heads / kv_heads;
@@ -580,10 +593,15 @@ int launch_prefill_tc(const void* q, long long tokens, void* out, const void* k_
                                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ROOST_ERR_CUDA, "attention_prefill: cuTensorMapEncodeTiled (values) failed with code " + std::to_string((int)r));
   }
-#define ROOST_TC_CASE(DD, RR, GG)                                                                                                      \
-  if (head_dim == DD && box_rows == RR && groups == GG)                                                                                \
-    return launch_tc<DD, RR, GG>(mq, mk, mv, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items, q_heads, kv_heads, page_size, \
-                                 scale, window, s);
+  const bool wide = (window & ROOST_ATTENTION_WIDE_WEIGHTS) != 0;
+#define ROOST_TC_CASE(DD, RR, GG)                                                                                                            \
+  if (head_dim == DD && box_rows == RR && groups == GG) {                                                                                    \
+    if (wide)                                                                                                                                \
+      return launch_tc<DD, RR, GG, true>(mq, mk, mv, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items, q_heads, kv_heads,          \
+                                         page_size, scale, window, sinks, s);                                                                \
+    return launch_tc<DD, RR, GG, false>(mq, mk, mv, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items, q_heads, kv_heads, page_size, \
+                                        scale, window, sinks, s);                                                                            \
+  }
   ROOST_TC_CASE(128, 16, 1)
   ROOST_TC_CASE(128, 32, 1)
   ROOST_TC_CASE(64, 16, 1)

@@ -38,8 +38,8 @@ extern "C" {
  * entry point's `sinks` (float, one a query head) is not null the term is exp(sinks[h] - maximum) instead. */
 #define ROOST_ATTENTION_SINK (1 << 30)
 /* Also added to `window`: the softmax weights enter the second product as two bfloat16 operands, their rounding and what it left
- * over, so that 16 bits of the 32-bit weights count (the denominator is summed from the 32-bit weights anyway). The mma.sync
- * kernels serve it; plan the prefill's work items with roost_attention_prefill_tile_rows_mma. */
+ * over, so that 16 bits of the 32-bit weights count (the denominator is summed from the 32-bit weights anyway). Where a cap on the scores
+ * or kept keys are asked for too, plan the prefill's work items with roost_attention_prefill_tile_rows_mma. */
 #define ROOST_ATTENTION_WIDE_WEIGHTS (1 << 29)
 int roost_attention_prefill_tile_rows_mma(int head_dim, int kv_heads, long long packed_rows);
 

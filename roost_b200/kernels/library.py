@@ -432,7 +432,7 @@ class KernelLibrary:
         """Packed rows of a prefill work item (64 or 128) for these pools [pages, kv_heads, page_size, head_dim] and a step
         that brings ``packed_rows`` packed rows in all to the prefill kernels."""
         pages, nkv, page, d = k_pool.shape
-        if not tensor_memory:       # the mma.sync kernels' items (a caller that wants wide weights)
+        if not tensor_memory:       # the mma.sync kernels' items (a caller that wants a cap on the scores or kept keys)
             return int(self._lib.roost_attention_prefill_tile_rows_mma(d, nkv, int(packed_rows)))
         return int(self._lib.roost_attention_prefill_tile_rows(d, int(q_heads), nkv, page, pages, _ptr(k_pool), _ptr(v_pool), int(packed_rows)))
 
@@ -451,11 +451,10 @@ class KernelLibrary:
         """Tensor-core attention (bfloat16). ``plan``: an ``AttentionPlan`` whose work lists are on the device. ``sink``: one is
         added to the softmax's denominator (a key of score 0 that has no value), or exp(sinks[h]) of head h with ``sinks`` (float32, one a
         query head). ``wide_weights``: the softmax weights enter P V as two
-        bfloat16 operands (16 bits of the 32-bit weights); the plan's prefill items must then come from
-        ``attention_prefill_tile_rows(..., tensor_memory=False)``. ``softcap`` c > 0: a scaled score s becomes c tanh(s / c); the
+        bfloat16 operands (16 bits of the 32-bit weights). ``softcap`` c > 0: a scaled score s becomes c tanh(s / c); the
         prompt kernels on mma.sync serve it (items from ``tensor_memory=False``), the decode kernels do not: the plan must hold no
-        decode items then. ``keep_first``: with a window, a query also sees its request's first ``keep_first`` keys; the plan's decode
-        items must list them (``attention_work(..., keep_first=)``)."""
+        decode items then. ``keep_first``: with a window, a query also sees its request's first ``keep_first`` keys; the plan's prefill items come from ``tensor_memory=False``
+        then, and its decode items must list them (``attention_work(..., keep_first=)``)."""
         _need(q, "q", torch.bfloat16); _need(k_pool, "k_pool", torch.bfloat16); _need(v_pool, "v_pool", torch.bfloat16)
         T, nq, d = q.shape
         _, nkv, page, d2 = k_pool.shape

@@ -12,7 +12,7 @@ The cache is a paged group. When keys and values have the same size it has two p
 framework's tensor-core attention kernels, which then serve the bfloat16 steps with the sink added at their end; otherwise it
 has one plane whose entries are [key | value] of one key/value head, and the 32-bit kernel, which takes any sizes, reads that.
 On the tensor cores the 32-bit softmax weights enter P V as two bfloat16 operands, their rounding and what it left over (16 bits
-of the weights), which the mma.sync kernels serve; the denominator is summed from the 32-bit weights.
+of the weights); the denominator is summed from the 32-bit weights.
 
 With ``joined_norm_eps`` the kernel before the attention norms all query heads of a token as one row (and the key heads likewise) under
 stored weights instead, without a rotation. With ``keep_first`` a query sees the request's first keys beside its window, and the cache keeps
@@ -131,7 +131,9 @@ class SinkAttention(Mixer):
     def _attend_tensor_cores(self, q, batch, cache, tables):
         s, k = self.spec, self.rt.kernels
         group = s.num_heads // s.num_kv_heads
-        tile_rows = k.attention_prefill_tile_rows(s.num_heads, cache.k_pool, cache.v_pool, batch.num_tokens * group, tensor_memory=False)
+        # prompt portions run on tcgen05 unless the scores are capped or first keys kept, which the mma.sync kernels serve
+        tile_rows = k.attention_prefill_tile_rows(s.num_heads, cache.k_pool, cache.v_pool, batch.num_tokens * group,
+                                                  tensor_memory=not s.softcap and not s.keep_first)
         split_for = getattr(k, "decode_split_for", None)
         kept = {"chunks_of": lambda c: kept_chunks(batch.kv_cap, s.window, s.keep_first, c)} if s.keep_first else {}
         chunk, cluster = split_for(batch.num_rows, batch.kv_cap, cache.k_pool, cache.v_pool, **kept) if split_for and batch.kv_cap else (k.decode_chunk, 0)

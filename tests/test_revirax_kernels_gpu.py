@@ -277,3 +277,44 @@ def test_the_norm_over_all_heads_with_a_weight_and_a_gate(kernels, dtype, width,
     got = kernels.head_norm_gate(o.cuda(), u.cuda(), 5, w.cuda(), 1, 1e-5, dtype, gate=gate)
     gx = u[:, 5:].double()
     close(got.cpu(), P.rms_norm(o.double(), w.double(), 1e-5) * (P.sigmoid(gx) if gate == "sigmoid" else P.silu(gx)), dtype, f"row norm, {gate}")
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,page", [(4, 2, 64, 16), (8, 2, 128, 16), (4, 4, 128, 32), (16, 1, 64, 32)])
+@pytest.mark.parametrize("window", [None, 1, 150])
+def test_wide_weights_on_tcgen05(kernels, heads, kv_heads, dim, page, window):
+    """Prompt portions with stored sinks through the tcgen05 kernel, one and two row groups a CTA, lengths beside the key tiles' edges, scores
+    with a wide spread; against 64 bits, and no further from it than the mma.sync kernel is."""
+    g = torch.Generator().manual_seed(heads + dim)
+    lens, counts = [257, 640], [257, 387]
+    pg = Paged(lens, kv_heads, dim, dim, torch.bfloat16, page, g)
+    group, scale = heads // kv_heads, 3.0 / math.sqrt(dim)
+    q = torch.randn(sum(counts), heads, dim, generator=g).to(torch.bfloat16)
+    kv = torch.randn(2, pg.T, kv_heads, dim, generator=g).to(torch.bfloat16)
+    flat = pg.slots.long().cuda()
+    for pool, x in ((pg.k_pool, kv[0]), (pg.v_pool, kv[1])):
+        pool[flat // page, :, flat % page] = x.cuda()
+    sinks = torch.linspace(-6.0, 6.0, heads)
+    want, at = [], 0
+    for r, (n, m) in enumerate(zip(lens, counts)):
+        rows = slice(sum(lens[:r]), sum(lens[:r]) + n)
+        k, v = (kv[i, rows].double().repeat_interleave(group, 1).transpose(0, 1) for i in (0, 1))
+        s = q[at : at + m].double().transpose(0, 1) @ k.transpose(1, 2) * scale
+        i, j = torch.arange(n - m, n)[:, None], torch.arange(n)[None]
+        s = s.masked_fill((j > i) | (j <= i - window if window else j < 0), -math.inf)
+        e = torch.exp(s)
+        want.append(((e @ v) / (e.sum(-1, keepdim=True) + sinks.double().exp()[:, None, None])).transpose(0, 1).reshape(m, -1))
+        at += m
+    want = torch.cat(want)
+
+    def run(tile_rows):
+        plan = plan_attention([n - m for n, m in zip(lens, counts)], counts, group, window, 256, "cuda", tile_rows)
+        return kernels.attention_mma(q.cuda(), pg.k_pool, pg.v_pool, i32([0, counts[0], sum(counts)]), i32(lens), pg.kv_indptr, pg.kv_indices, plan, scale, window,
+                                     sink=True, wide_weights=True, sinks=sinks.cuda()).double().cpu()
+
+    off = lambda got: float((got - want).norm() / want.norm())
+    mma = off(run(64))
+    for tile_rows in (128, 256):
+        assert kernels.attention_prefill_tile_rows(heads, pg.k_pool, pg.v_pool, 10 ** 6) == 256, "the tcgen05 kernel does not serve these sizes"
+        here = off(run(tile_rows))
+        print(f"MEASURED wide weights, items of {tile_rows}: {here:.3e} on tcgen05, {mma:.3e} on mma.sync")
+        assert here < 1.1 * mma and here < 2.0 ** -8       # the output's own rounding to bfloat16 is all that shows

@@ -26,11 +26,17 @@
 // Wide weights (WIDE): a row's weights enter the second product as two bfloat16 operands, their rounding and what it left over, so that 16 bits
 // of the 32-bit weights count: the second operands lie over the other half of the scores' columns, and every product with V is made twice. Rows of 1,500, 500 and 2,048 tokens, 16
 // heads of 128 over 4, with a sink: 64 us, 243 with the mma.sync kernel that served wide weights before.
+// Keys and values that are not paged (FLAT): entry r * stride + j is row r's token at position j of a dense tensor with the heads side by side, a
+// key/value head a query head, keys wider than values by a part that all heads share (a tensor of its own, as the queries' last numbers are):
+// what prompt portions of a latent attention carry out of their cache (rows of 2,048 and 1,000 tokens, 16 heads of 128 + 64 over a latent of 512:
+// 69 us, with the gather and the two products before it 98; 1,204 in the latent space on mma.sync). The work items follow from q_indptr, the last tiles of a row first.
 // Value rows at positions the request does not hold yet (the rest of its last page) or before the CTA's first visible key
 // are zeroed in shared memory before the second product, so that whatever the pool holds there cannot reach a result;
 // their scores are masked by position. Every wait is bounded (see tma.cuh): a wait given up raises the CTA's abort flag
 // and records a code that roost_attention_status() returns.
 #include "tcgen05.cuh"
+
+#include <initializer_list>
 
 namespace roost {
 
@@ -53,13 +59,19 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-template <int D, int NG>
+template <int DK, int DV, int NG>
 struct TcCfg {
-  // what fits beside NG Q tiles in 227 KB: a key tile and a value tile are 128 x D x 2 bytes each
-  static constexpr int kKStages = D == 128 ? (NG == 1 ? 3 : 2) : 3;
-  static constexpr int kVStages = D == 128 ? 2 : 3;
-  static constexpr uint32_t kTile = kTcKeys * D * 2;
-  static constexpr size_t kSmem = (size_t)NG * kTcRows * D * 2 + (size_t)(kKStages + kVStages) * kTile + 1024;
+  // what fits beside NG Q tiles in 227 KB: a key tile is 128 x DK x 2 bytes, a value tile 128 x DV x 2
+  static constexpr int kKStages = DK == 192 ? 2 : DK == 128 ? (NG == 1 ? 3 : 2) : 3;
+  static constexpr int kVStages = DV == 128 ? 2 : 3;
+  static constexpr uint32_t kKTile = kTcKeys * DK * 2, kVTile = kTcKeys * DV * 2;
+  static constexpr size_t kSmem = (size_t)NG * kTcRows * DK * 2 + (size_t)kKStages * kKTile + (size_t)kVStages * kVTile + 1024;
+  static_assert(kSmem <= 227 * 1024, "shared memory of a CTA");
+};
+
+// What a FLAT launch has instead of pages: entries a row, batch rows, 64-column blocks of a head's own key part, k steps of a score.
+struct TcFlat {
+  int stride, rows, own_blocks, k_steps;
 };
 
 // work[i] = (batch row, first packed row of the item's NG x 128 rows); an item is run once for every key/value head.
@@ -67,24 +79,25 @@ struct TcCfg {
 // longest first. Tensor memory and the barriers are set up once; the rings of keys and values, the score columns and the
 // barriers' phases run on from one pair to the next, so the copies of the next pair start while the last tiles of this
 // one are still being computed.
-template <int D, int RPC, int NG, bool WIDE>
+template <int DK, int DV, int RPC, int NG, bool WIDE, bool FLAT>
 __global__ void __launch_bounds__(64 + NG * 128, 1)
     attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                                const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out, const int32_t* __restrict__ q_indptr,
+                                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_q2,
+                                const __grid_constant__ CUtensorMap map_k2, TcFlat flat, __nv_bfloat16* __restrict__ out, const int32_t* __restrict__ q_indptr,
                                 const int32_t* __restrict__ kv_lens, const int32_t* __restrict__ kv_indptr,
                                 const int32_t* __restrict__ kv_indices, const int2* __restrict__ work, int items, int q_heads, int kv_heads,
                                 int page_size, float scale_log2, int window, const float* __restrict__ sinks) {
   const float sink = (window & ROOST_ATTENTION_SINK) ? 1.0f : 0.f;     // one more term, 2^(0 - m) or 2^(a head's stored number - m), in every row's denominator
   window &= ~(ROOST_ATTENTION_SINK | ROOST_ATTENTION_WIDE_WEIGHTS);
-  using Cfg = TcCfg<D, NG>;
-  constexpr int BM = kTcRows, TK = kTcKeys, KS = Cfg::kKStages, VS = Cfg::kVStages, NP = TK / RPC, CB = D / 64;
-  constexpr uint32_t kQBytes = BM * D * 2;                  // one row group's Q tile
-  constexpr uint32_t kTile = Cfg::kTile;                    // keys, or values, of TK positions
-  constexpr uint32_t kVPage = CB * RPC * 128;               // the values page copy by page copy: [column block][RPC rows][128 B]
+  using Cfg = TcCfg<DK, DV, NG>;
+  constexpr int BM = kTcRows, TK = kTcKeys, KS = Cfg::kKStages, VS = Cfg::kVStages, NP = TK / RPC, CB = DK / 64;
+  constexpr uint32_t kQBytes = BM * DK * 2;                 // one row group's Q tile
+  constexpr uint32_t kKTile = Cfg::kKTile, kVTile = Cfg::kVTile;      // keys, and values, of TK positions
+  constexpr uint32_t kVPage = (DV / 64) * RPC * 128;        // the values page copy by page copy: [column block][RPC rows][128 B]
   constexpr int kOps = NP * (CB + 1);                       // copies a tile takes: per page one per column block of keys, one of values
   static_assert(kOps <= 32, "one lane a copy");
   constexpr int SB = NG == 1 ? 2 : 1;                       // sets of score columns a row group has
-  constexpr uint32_t kGroupCols = SB * TK + D;              // tensor-memory columns of a row group: the scores (the weights over them) and the output
+  constexpr uint32_t kGroupCols = SB * TK + DV;             // tensor-memory columns of a row group: the scores (the weights over them) and the output
   constexpr uint32_t kTmemCols = NG * kGroupCols <= 256 ? 256 : 512;
   static_assert(NG * kGroupCols <= 512, "tensor memory has 512 columns");
   constexpr int kGroupBars = 2 * SB + 1;                    // s_full[SB], p_full[SB], o_done
@@ -93,7 +106,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
   const uint32_t smem_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023u) & ~1023u;
   const uint32_t q_smem = smem_base;
   const uint32_t k_smem = q_smem + NG * kQBytes;
-  const uint32_t v_smem = k_smem + KS * kTile;
+  const uint32_t v_smem = k_smem + KS * kKTile;
   __shared__ __align__(8) uint64_t bars[2 + 2 * KS + 2 * VS + NG * kGroupBars];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
@@ -162,14 +175,29 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
     int t0, ntiles, lo, hi;
   };
   auto load_pair = [&](int wi, Pair& p) -> bool {
-    const int2 w = work[wi / kv_heads];
-    p.b = w.x;
-    p.row0 = w.y;
+    int n;
     p.kvh = wi % kv_heads;
-    if (p.b < 0) return false;  // padding of a fixed-size work list
-    p.q_start = q_indptr[p.b];
-    const int n = q_indptr[p.b + 1] - p.q_start;
-    p.kv_len = kv_lens[p.b];
+    if (FLAT) {
+      int item = wi / kv_heads, tiles = 0;
+      for (p.b = 0; p.b < flat.rows; ++p.b) {
+        p.q_start = q_indptr[p.b];
+        n = q_indptr[p.b + 1] - p.q_start;
+        p.kv_len = kv_lens[p.b];
+        tiles = p.kv_len >= n ? (n + BM - 1) / BM : 0;      // a padding row holds no keys
+        if (item < tiles) break;
+        item -= tiles;
+      }
+      if (p.b == flat.rows) return false;
+      p.row0 = (tiles - 1 - item) * BM;
+    } else {
+      const int2 w = work[wi / kv_heads];
+      p.b = w.x;
+      p.row0 = w.y;
+      if (p.b < 0) return false;  // padding of a fixed-size work list
+      p.q_start = q_indptr[p.b];
+      n = q_indptr[p.b + 1] - p.q_start;
+      p.kv_len = kv_lens[p.b];
+    }
     p.pos0 = p.kv_len - n;
     p.rows_total = n * group;
     // Key tiles of each row group: from its first row's window to its last row's position; a group past the request's
@@ -200,16 +228,16 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
 
   if (warp == 0) {
     // ---- producer
-    const int page_shift = 31 - __clz(page_size);  // a power of two here
+    const int page_shift = FLAT ? 0 : 31 - __clz(page_size);  // a power of two here
     int kt = 0;        // tiles copied so far, over all pairs: the rings run on
     int pairs = 0;     // pairs begun so far
     bool ok = true;
     Pair p;
     for (int round = 0, wi = pair_of(0); wi < total && ok; wi = pair_of(++round)) {
       if (!load_pair(wi, p)) continue;
-      const int32_t* pages = kv_indices + kv_indptr[p.b];
-      const int p_first = (p.t0 * TK) >> page_shift, p_last = p.hi >> page_shift;
-      const int fallback = pages[p_last];
+      const int32_t* pages = FLAT ? nullptr : kv_indices + kv_indptr[p.b];
+      const int p_first = (p.t0 * TK) >> page_shift, p_last = FLAT ? -1 : p.hi >> page_shift;
+      const int fallback = FLAT ? 0 : pages[p_last];
       auto row_of = [&](int pg, int entry) {  // first pool row of page pg of the request, given its block-table entry
         const bool visible = ((pg + 1) << page_shift) > p.lo && (pg << page_shift) <= p.hi;
         return ((visible && entry >= 0 ? entry : fallback) * kv_heads + p.kvh) << page_shift;
@@ -221,8 +249,16 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
         if (pairs >= 1) ok = mbar_wait_limited(q_empty, (uint32_t)(pairs - 1) & 1u, abortp, 12, &g_attention_tc_error);
         if (ok) {
           mbar_expect_tx(q_full, NG * kQBytes);  // rows past the tensor's last token are filled with zeros and counted
+          if constexpr (FLAT) {
 #pragma unroll
-          for (int g = 0; g < NG; ++g) tma_load_5d(q_smem + g * kQBytes, &map_q, q_full, 0, 0, p.kvh, p.q_start + (p.row0 + g * BM) / group, 0);
+            for (int c = 0; c < CB; ++c) {
+              const bool own = c < flat.own_blocks;
+              tma_load_3d(q_smem + c * (BM * 128), own ? &map_q : &map_q2, q_full, own ? c * 64 : 0, p.kvh, p.q_start + p.row0);
+            }
+          } else {
+#pragma unroll
+            for (int g = 0; g < NG; ++g) tma_load_5d(q_smem + g * kQBytes, &map_q, q_full, 0, 0, p.kvh, p.q_start + (p.row0 + g * BM) / group, 0);
+          }
         }
       }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -230,7 +266,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
       for (int i = 0; i < p.ntiles && ok; ++i, ++kt) {
         const int ks = kt % KS, vs = kt % VS;
         const int j = (p.t0 + i) * TK;
-        if ((j >> page_shift) >= batch0 + 32) {  // uniform in the warp
+        if (!FLAT && (j >> page_shift) >= batch0 + 32) {  // uniform in the warp
           batch0 += 32;
           cur = row_of(batch0 + lane, nxt_entry);
           nxt_entry = batch0 + 32 + lane <= p_last ? pages[batch0 + 32 + lane] : -1;
@@ -239,22 +275,24 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
         // A tile never straddles two batches of 32 pages: both start on tile boundaries.
         const int c = lane / (CB + 1), part = lane % (CB + 1);
         const int jc = j + (c < NP ? c : 0) * RPC;
-        const int my_row = __shfl_sync(0xffffffffu, cur, ((jc >> page_shift) - batch0) & 31) + (jc & (page_size - 1));
+        const int my_row = FLAT ? p.b * flat.stride + j : __shfl_sync(0xffffffffu, cur, ((jc >> page_shift) - batch0) & 31) + (jc & (page_size - 1));
         if (lane == 0) {
           if (kt >= KS) ok = mbar_wait_limited(k_empty(ks), (uint32_t)((kt / KS) - 1) & 1u, abortp, 1, &g_attention_tc_error);
-          if (ok) mbar_expect_tx(k_full(ks), kTile);
+          if (ok) mbar_expect_tx(k_full(ks), kKTile);
         }
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;  // also orders the expected bytes before the copies
         if (ok && lane < kOps && part < CB) {
-          tma_load_2d(k_smem + ks * kTile + part * (TK * 128) + c * (RPC * 128), &map_k, k_full(ks), part * 64, my_row);
+          const bool own = !FLAT || part < flat.own_blocks;
+          tma_load_2d(k_smem + ks * kKTile + part * (TK * 128) + c * (RPC * 128), own ? &map_k : &map_k2, k_full(ks),
+                      FLAT ? (own ? (p.kvh * flat.own_blocks + part) * 64 : 0) : part * 64, my_row);
         }
         if (lane == 0 && ok) {
           if (kt >= VS) ok = mbar_wait_limited(v_empty(vs), (uint32_t)((kt / VS) - 1) & 1u, abortp, 9, &g_attention_tc_error);
-          if (ok) mbar_expect_tx(v_full(vs), kTile);
+          if (ok) mbar_expect_tx(v_full(vs), kVTile);
         }
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         if (ok && lane < kOps && part == CB) {
-          tma_load_3d(v_smem + vs * kTile + c * kVPage, &map_v, v_full(vs), 0, my_row, 0);
+          tma_load_3d(v_smem + vs * kVTile + c * kVPage, &map_v, v_full(vs), 0, my_row, FLAT ? p.kvh * (DV / 64) : 0);
         }
       }
     }
@@ -262,7 +300,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
     // ---- issuer
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(BM, TK);
-      constexpr uint32_t idesc_o = umma_idesc_bf16_b_mn(BM, D);
+      constexpr uint32_t idesc_o = umma_idesc_bf16_b_mn(BM, DV);
       int kt0 = 0;            // tiles of the pairs before this one
       int pairs = 0;
       int jt0[NG];            // tiles of each group in the pairs before this one: which score columns, which phase
@@ -280,7 +318,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
           const int jt = jt0[g] + j, sb = jt % SB;
           if (!(ok = mbar_wait_limited(p_full(g, sb), (uint32_t)(jt / SB) & 1u, abortp, 3, &g_attention_tc_error))) return;
           tcgen05_fence_after();
-          const uint32_t v0 = v_smem + ((kt0 + i) % VS) * kTile;
+          const uint32_t v0 = v_smem + ((kt0 + i) % VS) * kVTile;
 #pragma unroll
           for (int kk = 0; kk < TK / 16; ++kk) {
             const uint32_t v_rows = v0 + (uint32_t)((kk * 16) / RPC) * kVPage + (uint32_t)((kk * 16) % RPC) * 128;
@@ -294,9 +332,10 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
         // S_g = Q K^T of the pair's tile i
         auto issue_s = [&](int g, int j, int i) {
           const int jt = jt0[g] + j;
-          const uint32_t k0 = k_smem + ((kt0 + i) % KS) * kTile;
+          const uint32_t k0 = k_smem + ((kt0 + i) % KS) * kKTile;
 #pragma unroll
-          for (int k = 0; k < D / 16; ++k) {
+          for (int k = 0; k < DK / 16; ++k) {
+            if (FLAT && k >= flat.k_steps) break;       // the rest of the shared part's block is padding
             const uint64_t a_desc = umma_desc_k_major_sw128(q_smem + g * kQBytes + (k / 4) * (BM * 128)) + (uint64_t)(2 * (k % 4));
             const uint64_t b_desc = umma_desc_k_major_sw128(k0 + (k / 4) * (TK * 128)) + (uint64_t)(2 * (k % 4));
             tcgen05_mma_f16(tmem_s(g, jt % SB), a_desc, b_desc, idesc_s, k > 0 ? 1u : 0u);
@@ -425,7 +464,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
             tcgen05_fence_after();
           }
 #pragma unroll 1
-          for (int c = 0; c < D / 32; ++c) {
+          for (int c = 0; c < DV / 32; ++c) {
             uint32_t v[32];
             tcgen05_ld_32x32b_x32(tmem_o(g) + lane_addr + c * 32, v);
 #pragma unroll
@@ -438,9 +477,9 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
         // it before its own second product.
         if (j0 + TK > p.kv_len || j0 < p.lo) {
           if (!(ok = mbar_wait_limited(v_full(kt % VS), (uint32_t)(kt / VS) & 1u, abortp, 7, &g_attention_tc_error))) break;
-          const uint32_t v0 = v_smem + (kt % VS) * kTile;
-          for (int idx = tid_g; idx < TK * (D / 8); idx += kGroupThreads) {
-            const int r = idx / (D / 8), ch = idx % (D / 8);
+          const uint32_t v0 = v_smem + (kt % VS) * kVTile;
+          for (int idx = tid_g; idx < TK * (DV / 8); idx += kGroupThreads) {
+            const int r = idx / (DV / 8), ch = idx % (DV / 8);
             if (j0 + r >= p.kv_len || j0 + r < p.lo) {
               const uint32_t addr = v0 + (uint32_t)(r / RPC) * kVPage + (uint32_t)(ch >> 3) * (RPC * 128) + (uint32_t)(r % RPC) * 128 +
                                     (uint32_t)(((ch & 7) ^ (r & 7)) << 4);
@@ -468,9 +507,9 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
         tcgen05_fence_after();
         if (sink != 0.f) l += ex2((sinks != nullptr && valid ? sinks[p.kvh * group + pr % group] * kLog2eTc : 0.f) - (m == -INFINITY ? 0.f : m));
         const float inv = l > 0.f ? 1.0f / l : 0.f;
-        __nv_bfloat16* dst = valid ? out + ((size_t)(p.q_start + pr / group) * q_heads + p.kvh * group + pr % group) * D : nullptr;
+        __nv_bfloat16* dst = valid ? out + ((size_t)(p.q_start + pr / group) * q_heads + p.kvh * group + pr % group) * DV : nullptr;
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
+        for (int c = 0; c < DV / 32; ++c) {
           uint32_t v[32];
           tcgen05_ld_32x32b_x32(tmem_o(g) + lane_addr + c * 32, v);
           if (valid) {
@@ -526,12 +565,12 @@ bool prefill_tc_serves(int head_dim, int q_heads, int kv_heads, int page_size, l
   return (uintptr_t)k_pool % 128 == 0 && (q == nullptr || (uintptr_t)q % 16 == 0) && encode_tiled() != nullptr;
 }
 
-template <int D, int RPC, int NG, bool WIDE>
-static int launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out, const int32_t* q_indptr, const int32_t* kv_lens,
-                     const int32_t* kv_indptr, const int32_t* kv_indices, const int32_t* work, int items, int q_heads, int kv_heads,
-                     int page_size, float scale, int window, const float* sinks, cudaStream_t s) {
-  constexpr size_t smem = TcCfg<D, NG>::kSmem;
-  auto kernel = attention_prefill_tc_kernel<D, RPC, NG, WIDE>;
+template <int DK, int DV, int RPC, int NG, bool WIDE, bool FLAT>
+static int launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mq2, const CUtensorMap& mk2, TcFlat flat, void* out,
+                     const int32_t* q_indptr, const int32_t* kv_lens, const int32_t* kv_indptr, const int32_t* kv_indices, const int32_t* work, int items,
+                     int q_heads, int kv_heads, int page_size, float scale, int window, const float* sinks, cudaStream_t s) {
+  constexpr size_t smem = TcCfg<DK, DV, NG>::kSmem;
+  auto kernel = attention_prefill_tc_kernel<DK, DV, RPC, NG, WIDE, FLAT>;
   static int sms[64] = {};   // per device: its SM count, and that the kernel's shared-memory size has been set there
   int dev = 0;
   cudaGetDevice(&dev);
@@ -546,7 +585,7 @@ static int launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   // list better than the fixed walk (8 x 8192 tokens: 1017 against 885 TFLOP/s).
   const long long pairs = (long long)items * kv_heads;
   const int grid = (int)(pairs <= 8LL * sms[dev] ? (pairs < sms[dev] ? pairs : sms[dev]) : pairs);
-  launch_kernel(kernel, dim3(grid), dim3(64 + NG * 128), smem, s, mq, mk, mv, (__nv_bfloat16*)out, q_indptr, kv_lens, kv_indptr, kv_indices,
+  launch_kernel(kernel, dim3(grid), dim3(64 + NG * 128), smem, s, mq, mk, mv, mq2, mk2, flat, (__nv_bfloat16*)out, q_indptr, kv_lens, kv_indptr, kv_indices,
                 (const int2*)work, items, q_heads, kv_heads, page_size, scale * kLog2eTc, window, sinks);
   return check_launch("attention_prefill_tc");
 }
@@ -594,13 +633,13 @@ int launch_prefill_tc(const void* q, long long tokens, void* out, const void* k_
     if (r != CUDA_SUCCESS) return fail(ROOST_ERR_CUDA, "attention_prefill: cuTensorMapEncodeTiled (values) failed with code " + std::to_string((int)r));
   }
   const bool wide = (window & ROOST_ATTENTION_WIDE_WEIGHTS) != 0;
-#define ROOST_TC_CASE(DD, RR, GG)                                                                                                            \
-  if (head_dim == DD && box_rows == RR && groups == GG) {                                                                                    \
-    if (wide)                                                                                                                                \
-      return launch_tc<DD, RR, GG, true>(mq, mk, mv, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items, q_heads, kv_heads,          \
-                                         page_size, scale, window, sinks, s);                                                                \
-    return launch_tc<DD, RR, GG, false>(mq, mk, mv, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items, q_heads, kv_heads, page_size, \
-                                        scale, window, sinks, s);                                                                            \
+#define ROOST_TC_CASE(DD, RR, GG)                                                                                                              \
+  if (head_dim == DD && box_rows == RR && groups == GG) {                                                                                      \
+    if (wide)                                                                                                                                  \
+      return launch_tc<DD, DD, RR, GG, true, false>(mq, mk, mv, mq, mk, TcFlat{}, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items,  \
+                                                    q_heads, kv_heads, page_size, scale, window, sinks, s);                                    \
+    return launch_tc<DD, DD, RR, GG, false, false>(mq, mk, mv, mq, mk, TcFlat{}, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items,   \
+                                                   q_heads, kv_heads, page_size, scale, window, sinks, s);                                     \
   }
   ROOST_TC_CASE(128, 16, 1)
   ROOST_TC_CASE(128, 32, 1)
@@ -612,6 +651,20 @@ int launch_prefill_tc(const void* q, long long tokens, void* out, const void* k_
   ROOST_TC_CASE(64, 32, 2)
 #undef ROOST_TC_CASE
   return fail(ROOST_ERR_UNSUPPORTED, "attention_prefill: no tcgen05 kernel for these sizes");
+}
+
+static bool flat_serves(int nope, int rope, int vdim) {
+  return (nope == 64 || nope == 128) && (vdim == 64 || vdim == 128) && rope >= 0 && rope <= 64 && rope % 16 == 0 && encode_tiled() != nullptr;
+}
+
+// A tensor map of bfloat16 numbers with 128-byte swizzle; `strides` in bytes, of dimensions 1 ...
+static int flat_map(CUtensorMap* m, const void* base, int rank, std::initializer_list<cuuint64_t> dims, std::initializer_list<cuuint64_t> strides,
+                    std::initializer_list<cuuint32_t> box) {
+  const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
+  const CUresult r = encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims.begin(), strides.begin(), box.begin(), elem,
+                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? ROOST_OK : fail(ROOST_ERR_CUDA, "carried_attention: cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
 }
 
 void set_prefill_tc(bool on) { g_prefill_tc = on; }
@@ -632,5 +685,55 @@ int prefill_tc_status() {
 }
 
 }  // namespace roost
+
+using namespace roost;
+
+extern "C" int roost_carried_attention_tc_supported(int nope, int rope, int vdim) { return flat_serves(nope, rope, vdim) ? 1 : 0; }
+
+// q [tokens, heads x (nope + rope)], rows ld_q apart; keys [rows * stride, heads * nope], values [rows * stride, heads * vdim] and, with rope, the
+// part of a key that all heads share, rope_keys [rows * stride, rope] with rows ld_rope apart: entry r * stride + j is row r's token at position j.
+// A row's queries are its last q_indptr[r + 1] - q_indptr[r] positions before kv_lens[r]; window as in roost_attention_prefill; sinks: null, or
+// exp(sinks[h]) joins head h's denominator. out [tokens, heads * vdim].
+extern "C" int roost_carried_attention_tc(const void* q, int64_t ld_q, void* out, const void* keys, const void* values, const void* rope_keys, int64_t ld_rope,
+                                          const int32_t* q_indptr, const int32_t* kv_lens, int tokens, int rows, int heads, int nope, int rope, int vdim,
+                                          int stride, float scale, int window, const float* sinks, roost_stream_t stream) {
+  ROOST_REQUIRE(tokens >= 0 && rows >= 0 && heads > 0 && stride > 0 && stride % kTcKeys == 0 && scale > 0.f && window >= 0,
+                "carried_attention: sizes and the scale must be positive, a row's entries a multiple of 128");
+  ROOST_REQUIRE(q && out && keys && values && q_indptr && kv_lens && (rope == 0 || rope_keys), "carried_attention: a pointer is null");
+  if (!flat_serves(nope, rope, vdim)) return fail(ROOST_ERR_UNSUPPORTED, "carried_attention: sizes the tcgen05 form does not serve");
+  ROOST_REQUIRE(ld_q >= (int64_t)heads * (nope + rope) && ld_q % 8 == 0 && (rope == 0 || (ld_rope >= rope && ld_rope % 8 == 0)),
+                "carried_attention: rows are too narrow or not whole 16-byte pieces");
+  ROOST_REQUIRE(((uintptr_t)q | (uintptr_t)out | (uintptr_t)keys | (uintptr_t)values | (uintptr_t)rope_keys) % 16 == 0, "carried_attention: a pointer is not aligned");
+  const long long entries = (long long)rows * stride, items = (long long)tokens / kTcRows + rows;
+  if (entries >= (1LL << 31) || items * heads >= (1LL << 30)) return fail(ROOST_ERR_UNSUPPORTED, "carried_attention: too many entries or heads");
+  if (tokens == 0 || rows == 0) return ROOST_OK;
+  const cuuint64_t E = (cuuint64_t)entries, H = (cuuint64_t)heads, head = (cuuint64_t)(nope + rope) * 2;
+  CUtensorMap mq, mk, mv, mq2, mk2;
+  int rc = flat_map(&mq, q, 3, {(cuuint64_t)nope, H, (cuuint64_t)tokens}, {head, (cuuint64_t)ld_q * 2}, {64u, 1u, (cuuint32_t)kTcRows});
+  if (rc == ROOST_OK) rc = flat_map(&mk, keys, 2, {H * nope, E}, {H * nope * 2}, {64u, (cuuint32_t)kTcKeys});
+  if (rc == ROOST_OK) rc = flat_map(&mv, values, 3, {64u, E, H * vdim / 64}, {H * vdim * 2, 128u}, {64u, (cuuint32_t)kTcKeys, (cuuint32_t)vdim / 64});
+  mq2 = mq;
+  mk2 = mk;
+  if (rc == ROOST_OK && rope) {
+    rc = flat_map(&mq2, (const char*)q + nope * 2, 3, {(cuuint64_t)rope, H, (cuuint64_t)tokens}, {head, (cuuint64_t)ld_q * 2}, {64u, 1u, (cuuint32_t)kTcRows});
+    if (rc == ROOST_OK) rc = flat_map(&mk2, rope_keys, 2, {(cuuint64_t)rope, E}, {(cuuint64_t)ld_rope * 2}, {64u, (cuuint32_t)kTcKeys});
+  }
+  if (rc != ROOST_OK) return rc;
+  const TcFlat flat = {stride, rows, nope / 64, (nope + rope) / 16};
+  const int w = window | (sinks != nullptr ? ROOST_ATTENTION_SINK : 0);
+  const int dk = nope + (rope ? 64 : 0);
+#define ROOST_TC_FLAT(KK, VV)                                                                                                                \
+  if (dk == KK && vdim == VV)                                                                                                                \
+    return launch_tc<KK, VV, 128, 1, true, true>(mq, mk, mv, mq2, mk2, flat, out, q_indptr, kv_lens, nullptr, nullptr, nullptr, (int)items,  \
+                                                 heads, heads, 1, scale, w, sinks, (cudaStream_t)stream);
+  ROOST_TC_FLAT(64, 64)
+  ROOST_TC_FLAT(64, 128)
+  ROOST_TC_FLAT(128, 64)
+  ROOST_TC_FLAT(128, 128)
+  ROOST_TC_FLAT(192, 64)
+  ROOST_TC_FLAT(192, 128)
+#undef ROOST_TC_FLAT
+  return fail(ROOST_ERR_UNSUPPORTED, "carried_attention: no tcgen05 kernel for these sizes");
+}
 
 ROOST_TRACE_TU(attention_tc)

@@ -3,8 +3,8 @@
 // [rows * stride, heads * vdim] (made by two products from the rows' gathered latents), entry j of a row being its token at
 // position j. bfloat16 on the tensor cores (mma.sync m16n8k16); scores, running maxima, weights and sums in 32-bit.
 //
-//   latent_gather:  a block an entry: the cached vector of (row, position j) copied to the dense [rows * stride, width] tensor,
-//                   zeros beyond the row's length.
+//   latent_gather:  the cached vector of (row, position j) copied to the dense [rows * stride, width] tensor, a thread a 16-byte piece
+//                   (a number where vectors are not whole pieces); zeros beyond the row's length and where a window has given the page back.
 //   attention:      one block of four warps per (row, 64 of its query tokens, head), a warp 16 query tokens; key tiles of 64 and
 //                   their values come by asynchronous copies a tile ahead; S = Q K^T; a running maximum and denominator a query;
 //                   the weights exp(s - m) enter P V as two bfloat16 operands, their rounding and what it left over (16 bits of
@@ -35,16 +35,19 @@ __device__ __forceinline__ void ca_split_pair(float x, float y, uint32_t& hi, ui
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
-__global__ void latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, __nv_bfloat16* __restrict__ out, const int32_t* __restrict__ kv_lens,
-                                     const int32_t* __restrict__ kv_indptr, const int32_t* __restrict__ kv_indices, int stride, int width,
-                                     int page_size) {
+template <typename P>      // a piece: 16 bytes or one number
+__global__ void __launch_bounds__(256) latent_gather_kernel(const P* pool, P* out, const int32_t* __restrict__ kv_lens, const int32_t* __restrict__ kv_indptr,
+                                                           const int32_t* __restrict__ kv_indices, int stride, int pieces, int page_size) {
   pdl_launch_dependents();
-  const int r = blockIdx.y, j = blockIdx.x;
+  const int r = blockIdx.y;
+  const long long at = (long long)blockIdx.x * 256 + threadIdx.x;
+  const int j = (int)(at / pieces), i = (int)(at % pieces);
+  if (j >= stride) return;
+  const int page = j < kv_lens[r] ? kv_indices[kv_indptr[r] + j / page_size] : -1;
   pdl_wait();
-  __nv_bfloat16* dst = out + ((size_t)r * stride + j) * width;
-  const __nv_bfloat16* src = nullptr;
-  if (j < kv_lens[r]) src = pool + ((size_t)kv_indices[kv_indptr[r] + j / page_size] * page_size + j % page_size) * width;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) dst[i] = src != nullptr ? src[i] : __float2bfloat16_rn(0.f);
+  P v = {};
+  if (page >= 0) v = pool[((size_t)page * page_size + j % page_size) * pieces + i];
+  out[((size_t)r * stride + j) * pieces + i] = v;
 }
 
 __device__ __forceinline__ bool ca_tile_of_block(const int32_t* __restrict__ q_indptr, int rows, int b, int& r, int& k) {
@@ -236,8 +239,15 @@ extern "C" int roost_latent_gather(const void* pool, void* out, const int32_t* k
   ROOST_REQUIRE(pool && out && kv_lens && kv_indptr && kv_indices, "latent_gather: a pointer is null");
   if (rows == 0) return ROOST_OK;
   if (rows > 65535) return fail(ROOST_ERR_UNSUPPORTED, "latent_gather: too many rows");
-  launch_kernel(latent_gather_kernel, dim3(stride, rows), dim3(width >= 256 ? 128 : 64), 0, (cudaStream_t)stream, (const __nv_bfloat16*)pool,
-                (__nv_bfloat16*)out, kv_lens, kv_indptr, kv_indices, stride, width, page_size);
+  const bool whole = width % 8 == 0 && ((uintptr_t)pool | (uintptr_t)out) % 16 == 0;
+  const int pieces = whole ? width / 8 : width;
+  const dim3 grid((unsigned)(((long long)stride * pieces + 255) / 256), rows);
+  if (whole)
+    launch_kernel(latent_gather_kernel<uint4>, grid, dim3(256), 0, (cudaStream_t)stream, (const uint4*)pool, (uint4*)out, kv_lens, kv_indptr, kv_indices, stride,
+                  pieces, page_size);
+  else
+    launch_kernel(latent_gather_kernel<uint16_t>, grid, dim3(256), 0, (cudaStream_t)stream, (const uint16_t*)pool, (uint16_t*)out, kv_lens, kv_indptr, kv_indices,
+                  stride, pieces, page_size);
   return check_launch("latent_gather");
 }
 

@@ -561,6 +561,11 @@ int roost_sigmoid_attention_mma(const void* q, void* out, const void* k_base, co
 /* out [rows * stride, width]: entry r * stride + j is the cached vector of row r's token at position j, zeros from kv_lens[r] on. */
 int roost_latent_gather(const void* pool, void* out, const int32_t* kv_lens, const int32_t* kv_indptr, const int32_t* kv_indices, int rows,
                         int stride, int width, int page_size, roost_stream_t stream);
+/* The tcgen05 form (attention_tc.cu, which says how the tensors lie): keys with a part that all heads share, a window, stored sinks. */
+int roost_carried_attention_tc_supported(int nope, int rope, int vdim);
+int roost_carried_attention_tc(const void* q, int64_t ld_q, void* out, const void* keys, const void* values, const void* rope_keys, int64_t ld_rope,
+                               const int32_t* q_indptr, const int32_t* kv_lens, int tokens, int rows, int heads, int nope, int rope, int vdim, int stride,
+                               float scale, int window, const float* sinks, roost_stream_t stream);
 int roost_carried_attention_supported(int dim, int vdim);   /* multiples of 16 up to 128 */
 /* Causal softmax attention of the step's queries (rows ld_q apart, head h at column h * dim) over keys [rows * stride, heads * dim] and
  * values [rows * stride, heads * vdim] laid out like the gather's output: out [tokens, heads * vdim]. */

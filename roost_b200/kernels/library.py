@@ -187,6 +187,9 @@ _SIGNATURES = {
     "roost_sigmoid_attention_mma": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_int, c_void_p],
     "roost_latent_gather": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+    "roost_carried_attention_tc_supported": [c_int, c_int, c_int],
+    "roost_carried_attention_tc": [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                   c_int, c_int, c_float, c_int, c_void_p, c_void_p],
     "roost_carried_attention_supported": [c_int, c_int],
     "roost_carried_attention": [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                                 c_void_p],
@@ -765,6 +768,34 @@ class KernelLibrary:
         out = torch.empty((T, heads * vdim), dtype=q.dtype, device=q.device)
         self._call("roost_carried_attention", _ptr(q), q.stride(0), _ptr(out), _ptr(keys), _ptr(values), _ptr(positions), _ptr(q_indptr), T, rows, heads,
                    dim, vdim, stride, float(scale), _stream())
+        return out
+
+    def carried_attention_tc_supported(self, nope: int, rope: int, vdim: int) -> bool:
+        return bool(self._lib.roost_carried_attention_tc_supported(int(nope), int(rope), int(vdim)))
+
+    def carried_attention_tc(self, q, keys, values, rope_keys, q_indptr, kv_lens, heads: int, nope: int, rope: int, vdim: int, stride: int, scale: float,
+                             window: int | None = None, sinks: torch.Tensor | None = None) -> torch.Tensor:
+        """The same on tcgen05: a query is [nope | rope] numbers a head, a key the head's ``nope`` numbers of ``keys`` beside ``rope_keys``
+        [rows * stride, rope], which all heads share (None without; rows may lie apart). A row's queries are its last positions before
+        ``kv_lens``. ``window`` and ``sinks`` (exp(sinks[h]) joins the denominator) as in ``latent_attention``."""
+        _need(q, "q", torch.bfloat16); _need(keys, "keys", torch.bfloat16); _need(values, "values", torch.bfloat16)
+        _need(q_indptr, "q_indptr", torch.int32); _need(kv_lens, "kv_lens", torch.int32)
+        T, rows = q.shape[0], q_indptr.numel() - 1
+        if (q.shape[1] < heads * (nope + rope) or tuple(keys.shape) != (rows * stride, heads * nope) or tuple(values.shape) != (rows * stride, heads * vdim)
+                or kv_lens.numel() < rows):
+            raise KernelError("carried_attention_tc: the queries, keys or values do not fit the sizes")
+        if rope:
+            _need_rows(rope_keys, "rope_keys", torch.bfloat16)
+            if tuple(rope_keys.shape) != (rows * stride, rope):
+                raise KernelError("carried_attention_tc: the shared key parts do not fit the sizes")
+        if sinks is not None:
+            _need(sinks, "sinks", torch.float32)
+            if sinks.numel() != heads:
+                raise KernelError("carried_attention_tc: stored sinks are one number a head")
+        out = torch.empty((T, heads * vdim), dtype=q.dtype, device=q.device)
+        self._call("roost_carried_attention_tc", _ptr(q), q.stride(0), _ptr(out), _ptr(keys), _ptr(values), _ptr(rope_keys) if rope else None,
+                   rope_keys.stride(0) if rope else 0, _ptr(q_indptr), _ptr(kv_lens), T, rows, heads, nope, rope, vdim, stride, float(scale),
+                   int(window) if window else 0, _ptr(sinks), _stream())
         return out
 
     # ------------------------------------------------------------------ the Mamba-2 recurrence

@@ -14,9 +14,9 @@ cache entry; the batched product into the latent space; attention; the batched p
 projection. A run that reads another run's cache makes no latent and writes nothing; its window may differ from the
 owner's (the cache is kept for the widest). With ``rope_dim`` 0 keys and queries have no rotated part: nothing is rotated and the
 cache entry is the latent alone. With ``head_gate`` one more small projection gives a number a token and head, and a kernel
-multiplies every head's output by its sigmoid before the output projection. bfloat16 steps of prompt portions of such a run (no
-rotated part, no window) carry the rows' cached latents out to keys and values a head (a gather and two products) and attend there
-on the tensor cores: a prompt needs a quarter of the products that way when the latent is four times as wide as a head.
+multiplies every head's output by its sigmoid before the output projection. bfloat16 steps of prompt portions carry the rows' cached latents
+out to keys and values a head (a gather and two products) and attend there on the tensor cores, the rotated part that the heads share beside
+the keys: a prompt needs a third to a quarter of the products that way when the latent is four times as wide as a head.
 
 With ``q_rank`` the queries go through a latent of their own: one projection gives [query latent | key/value latent and shared key part |
 output gate's argument], the kernel that makes the cache entry also norms the query latent, a second product makes the queries from it and
@@ -70,12 +70,15 @@ class LatentAttention(Mixer):
         require_plain_amplitude(self.position, "latent_attention")
         self.interleaved = getattr(self.position, "pairing", None) == "interleaved"
         self.head_gate = Linear(runtime, s.num_heads, s.hidden) if s.head_gate else None
-        # Prompt portions of a run without a rotated part and without a window may leave the latent space: the rows' cached latents
-        # are carried out to keys and values a head by two products, and the attention runs over those, a quarter of the products
-        # the latent space costs when the latent is four times as wide as a head. Decode steps stay in the latent space, where the
-        # cache is read once for all heads.
-        self.carried = (s.rope_dim == 0 and not s.learned_sink and s.window is None and s.own_latent and not runtime.full_precision and runtime.kernels is not None
-                        and getattr(runtime.kernels, "carried_attention_supported", lambda d, v: False)(s.nope_dim, s.v_dim))
+        # Prompt portions may leave the latent space: the rows' cached latents are carried out to keys and values a head by two products,
+        # and the attention runs over those (with the rotated part that all heads share beside the keys), a third to a quarter of the products
+        # the latent space costs when the latent is four times as wide as a head, and on tcgen05 where the sizes allow. Decode steps stay in
+        # the latent space, where the cache is read once for all heads.
+        serves = lambda name, *sizes: (not runtime.full_precision and runtime.kernels is not None
+                                       and getattr(runtime.kernels, name, lambda *_: False)(*sizes))
+        self.carried_tc = (serves("carried_attention_tc_supported", s.nope_dim, s.rope_dim, s.v_dim) and s.kv_rank % 8 == 0 and s.rope_dim % 8 == 0)
+        self.carried = self.carried_tc or (s.rope_dim == 0 and not s.learned_sink and s.window is None and s.own_latent
+                                           and serves("carried_attention_supported", s.nope_dim, s.v_dim))
         self.key_full = Linear(runtime, s.num_heads * s.nope_dim, s.kv_rank) if self.carried else None
         self.value_full = Linear(runtime, s.num_heads * s.v_dim, s.kv_rank) if self.carried else None
         self.carried_min_tokens = 128        # tokens of a step from which its prompt portions are worth the two products
@@ -158,12 +161,20 @@ class LatentAttention(Mixer):
             k.latent_prepare(q, down, cache.k_pool, self.latent_weight, inv_freq, rotary_dim, batch.positions,
                              tables.slot_mapping if s.own_latent else None, *sizes, **more)
             gate, gate_col = (self.gate(x), 0) if s.output_gate else (None, 0)
-        if (self.carried and not batch.all_single and T >= self.carried_min_tokens and batch.kv_cap
-                and batch.num_rows * batch.kv_cap <= self.carried_max_entries):
+        # Under a window the latent space costs no more for keys that the window has passed, but carrying them out does: measured with a
+        # window of 1,024 the two cross at about 16 entries a token of the step.
+        entries = batch.num_rows * batch.kv_cap
+        if (self.carried and not batch.all_single and T >= self.carried_min_tokens and 0 < entries <= self.carried_max_entries
+                and (s.window is None or entries <= 16 * T)):
             # a function of the step's sizes and kind only, so a captured step keeps its way
             latents = k.latent_gather(cache.k_pool, batch.kv_lens, tables.kv_indptr, tables.kv_indices, batch.num_rows, batch.kv_cap)
-            o = k.carried_attention(q, self.key_full(latents), self.value_full(latents), batch.positions, batch.q_indptr, H, s.nope_dim, s.v_dim,
-                                    batch.kv_cap, s.scale)
+            if self.carried_tc:
+                c = latents[:, : s.kv_rank]
+                o = k.carried_attention_tc(q, self.key_full(c), self.value_full(c), latents[:, s.kv_rank :] if s.rope_dim else None, batch.q_indptr,
+                                           batch.kv_lens, H, s.nope_dim, s.rope_dim, s.v_dim, batch.kv_cap, s.scale, s.window, self.sinks)
+            else:
+                o = k.carried_attention(q, self.key_full(latents), self.value_full(latents), batch.positions, batch.q_indptr, H, s.nope_dim, s.v_dim,
+                                        batch.kv_cap, s.scale)
             if s.head_gate:
                 k.head_gate_mul_(o, self.head_gate(x), 0, H)
             if gate is not None:

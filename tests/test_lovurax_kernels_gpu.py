@@ -247,3 +247,48 @@ def test_prompt_portions_over_keys_and_values_carried_out_of_a_latent_cache(kern
                 ref[t, h] = w @ V[: p + 1, h]
             t += 1
     close(got.cpu(), ref.reshape(T, -1), torch.bfloat16, "attention over carried keys and values")
+
+
+@pytest.mark.parametrize("heads,nope,rope,vdim", [(3, 64, 0, 64), (2, 64, 32, 64), (2, 64, 64, 128), (1, 128, 0, 64), (3, 128, 16, 128), (2, 128, 64, 128)])
+@pytest.mark.parametrize("window,sink", [(None, False), (1, True), (150, False)])
+def test_carried_attention_on_tcgen05(kernels, heads, nope, rope, vdim, window, sink):
+    """Every size of head, the shared part of a key, rows beside the key tiles' edges that start inside their keys, a row of one token and a
+    padding row; what lies beyond a row's keys or behind its window may be anything. Against 64 bits."""
+    g = torch.Generator().manual_seed(nope + rope + vdim)
+    stride, scale = 512, 2.0 / math.sqrt(nope + rope)
+    lens, counts = [129, 384, 257], [129, 255, 1]
+    T = sum(counts)
+    q = torch.randn(T + 2, heads * (nope + rope) + 8, generator=g).to(torch.bfloat16)       # a padding row's tokens at the end
+    own = torch.randn(4 * stride, heads * nope, generator=g).to(torch.bfloat16)
+    shared = torch.randn(4 * stride, 16 + rope, generator=g).to(torch.bfloat16)
+    values = torch.randn(4 * stride, heads * vdim, generator=g).to(torch.bfloat16)
+    for r, (n, m) in enumerate(zip(lens, counts)):
+        values[r * stride + n : (r + 1) * stride] = float("inf")
+        if window and n - m - window + 1 > 0:
+            values[r * stride : r * stride + n - m - window + 1] = float("nan")
+    sinks = torch.linspace(-3.0, 3.0, heads) if sink else None
+    got = kernels.carried_attention_tc(q.cuda(), own.cuda(), values.cuda(), shared.cuda()[:, 16:] if rope else None, i32([0, 129, 384, T, T + 2]),
+                                       i32(lens + [0]), heads, nope, rope, vdim, stride, scale, window, sinks.cuda() if sink else None)
+    want, t = torch.zeros(T, heads, vdim, dtype=torch.float64), 0
+    for r, (n, m) in enumerate(zip(lens, counts)):
+        at = slice(r * stride, r * stride + n)
+        for h in range(heads):
+            k = torch.cat([own[at, h * nope : (h + 1) * nope], shared[at, 16:]], -1).double() if rope else own[at, h * nope : (h + 1) * nope].double()
+            s = q[t : t + m, h * (nope + rope) : (h + 1) * (nope + rope)].double() @ k.T * scale
+            i, j = torch.arange(n - m, n)[:, None], torch.arange(n)[None]
+            e = torch.exp(s.masked_fill((j > i) | (j <= i - window if window else j < 0), -math.inf))
+            v = values[at, h * vdim : (h + 1) * vdim].double().nan_to_num(nan=0.0, posinf=0.0)
+            want[t : t + m, h] = (e @ v) / (e.sum(-1, keepdim=True) + (math.exp(float(sinks[h])) if sink else 0.0))
+        t += m
+    off = float((got[:T].double().cpu() - want.reshape(T, -1)).norm() / want.norm())
+    print(f"MEASURED carried attention on tcgen05: {off:.3e}")
+    assert off < 2.0 ** -8        # the output's rounding to bfloat16; the weights count to 16 bits
+
+
+def test_the_gather_of_cached_vectors_leaves_out_pages_that_were_given_back(kernels):
+    for width in (24, 20):
+        pool = torch.randn(6, 1, 4, width).to(torch.bfloat16).cuda()
+        got = kernels.latent_gather(pool, i32([10]), i32([0, 3]), i32([-1, 5, 2]), 1, 16)
+        want = torch.zeros(16, width, dtype=torch.bfloat16, device="cuda")
+        want[4:8], want[8:10] = pool[5, 0], pool[2, 0, :2]
+        assert torch.equal(got, want)

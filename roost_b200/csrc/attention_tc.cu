@@ -30,6 +30,10 @@
 // key/value head a query head, keys wider than values by a part that all heads share (a tensor of its own, as the queries' last numbers are):
 // what prompt portions of a latent attention carry out of their cache (rows of 2,048 and 1,000 tokens, 16 heads of 128 + 64 over a latent of 512:
 // 69 us, with the gather and the two products before it 98; 1,204 in the latent space on mma.sync). The work items follow from q_indptr, the last tiles of a row first.
+// Sigmoid weights (SIGMOID): a key's weight is the sigmoid of its score, less a slope a head times its distance, plus a bias a head; nothing divides
+// by the weights' sum, so there is no running maximum and the accumulator is never rescaled; the output is multiplied by the sigmoid of a gate
+// where there is one. The special-function unit bounds it (an exponential and a reciprocal a weight). Work items as for FLAT. Rows of 2,048 and
+// 777 tokens, 16 heads of 64 over 4: 67 us, 125 + 48 on mma.sync with a second kernel that adds the sums of a long row's chunks.
 // Value rows at positions the request does not hold yet (the rest of its last page) or before the CTA's first visible key
 // are zeroed in shared memory before the second product, so that whatever the pool holds there cannot reach a result;
 // their scores are masked by position. Every wait is bounded (see tma.cuh): a wait given up raises the CTA's abort flag
@@ -74,16 +78,30 @@ struct TcFlat {
   int stride, rows, own_blocks, k_steps;
 };
 
+// What a SIGMOID launch has beside it: a slope and a bias a query head, the gate's rows (null: none), ld apart.
+struct TcSigmoid {
+  const float *slopes, *bias;
+  const __nv_bfloat16* gate;
+  int64_t ld_gate;
+};
+
+// 1 / (1 + 2^x)
+__device__ __forceinline__ float sigmoid_of_ex2(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(1.0f + ex2(x)));
+  return y;
+}
+
 // work[i] = (batch row, first packed row of the item's NG x 128 rows); an item is run once for every key/value head.
 // The grid is persistent: CTA c takes the (item, head) pairs c, c + gridDim.x, ... of the list, which the host has sorted
 // longest first. Tensor memory and the barriers are set up once; the rings of keys and values, the score columns and the
 // barriers' phases run on from one pair to the next, so the copies of the next pair start while the last tiles of this
 // one are still being computed.
-template <int DK, int DV, int RPC, int NG, bool WIDE, bool FLAT>
+template <int DK, int DV, int RPC, int NG, bool WIDE, bool FLAT, bool SIGMOID>
 __global__ void __launch_bounds__(64 + NG * 128, 1)
     attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_q2,
-                                const __grid_constant__ CUtensorMap map_k2, TcFlat flat, __nv_bfloat16* __restrict__ out, const int32_t* __restrict__ q_indptr,
+                                const __grid_constant__ CUtensorMap map_k2, TcFlat flat, TcSigmoid sg, __nv_bfloat16* __restrict__ out, const int32_t* __restrict__ q_indptr,
                                 const int32_t* __restrict__ kv_lens, const int32_t* __restrict__ kv_indptr,
                                 const int32_t* __restrict__ kv_indices, const int2* __restrict__ work, int items, int q_heads, int kv_heads,
                                 int page_size, float scale_log2, int window, const float* __restrict__ sinks) {
@@ -177,18 +195,18 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
   auto load_pair = [&](int wi, Pair& p) -> bool {
     int n;
     p.kvh = wi % kv_heads;
-    if (FLAT) {
+    if (FLAT || SIGMOID) {
       int item = wi / kv_heads, tiles = 0;
       for (p.b = 0; p.b < flat.rows; ++p.b) {
         p.q_start = q_indptr[p.b];
         n = q_indptr[p.b + 1] - p.q_start;
         p.kv_len = kv_lens[p.b];
-        tiles = p.kv_len >= n ? (n + BM - 1) / BM : 0;      // a padding row holds no keys
+        tiles = p.kv_len >= n ? (n * group + NG * BM - 1) / (NG * BM) : 0;      // a padding row holds no keys
         if (item < tiles) break;
         item -= tiles;
       }
       if (p.b == flat.rows) return false;
-      p.row0 = (tiles - 1 - item) * BM;
+      p.row0 = (tiles - 1 - item) * NG * BM;
     } else {
       const int2 w = work[wi / kv_heads];
       p.b = w.x;
@@ -400,6 +418,8 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
       const int qpos = valid ? p.pos0 + pr / group : -1;
       const int qlo = valid && window > 0 ? max(0, qpos - window + 1) : 0;
       const int my_tiles = p.g_last[g] - p.g_first[g] + 1;  // at most 0 for a group without rows
+      const int head = p.kvh * group + (valid ? pr % group : 0);
+      const float slope = SIGMOID ? sg.slopes[head] * kLog2eTc : 0.f, bias = SIGMOID ? sg.bias[head] * kLog2eTc : 0.f;
       float m = -INFINITY, l = 0.f;
       for (int j = 0; j < my_tiles && ok; ++j) {
         const int i = p.g_first[g] + j - p.t0;       // the pair's tile
@@ -426,27 +446,37 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
             s[e] = (key <= qpos && key >= qlo) ? s[e] : -INFINITY;
           }
         }
-        // the maximum of the raw scores (the scale is positive); four chains, so that it is not one long dependency
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        float corr = 1.0f, msafe = 0.f;
+        if (!SIGMOID) {
+          // the maximum of the raw scores (the scale is positive); four chains, so that it is not one long dependency
+          float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int e = 0; e < TK; e += 4) {
+          for (int e = 0; e < TK; e += 4) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(mx4[u], s[e + u]);
+            for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(mx4[u], s[e + u]);
+          }
+          const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+          // the reference maximum moves only when it must: the weights of this tile are then at most 2^kTcLazyRescale
+          if (mx > m + kTcLazyRescale || (m == -INFINITY && mx > -INFINITY)) {
+            corr = ex2(m - mx);   // 0 when m is -inf
+            m = mx;
+          }
+          msafe = m == -INFINITY ? 0.f : m;  // a row that has seen no key yet: every weight below is 0
         }
-        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
-        // the reference maximum moves only when it must: the weights of this tile are then at most 2^kTcLazyRescale
-        float corr = 1.0f;
-        if (mx > m + kTcLazyRescale || (m == -INFINITY && mx > -INFINITY)) {
-          corr = ex2(m - mx);   // 0 when m is -inf
-          m = mx;
-        }
-        const float msafe = m == -INFINITY ? 0.f : m;  // a row that has seen no key yet: every weight below is 0
+        const float at0 = SIGMOID ? fmaf(slope, (float)(j0 - qpos), bias) : 0.f;      // bias - slope (position - first key), in log2 units
         float sum4[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t packed[TK / 2], rest[WIDE ? TK / 2 : 1];
 #pragma unroll
         for (int e = 0; e < TK; e += 2) {
-          const float p0 = ex2(fmaf(s[e], scale_log2, -msafe)), p1 = ex2(fmaf(s[e + 1], scale_log2, -msafe));
-          sum4[(e / 2) & 3] += p0 + p1;
+          float p0, p1;
+          if (SIGMOID) {
+            p0 = sigmoid_of_ex2(-fmaf(s[e], scale_log2, fmaf(slope, (float)e, at0)));
+            p1 = sigmoid_of_ex2(-fmaf(s[e + 1], scale_log2, fmaf(slope, (float)(e + 1), at0)));
+          } else {
+            p0 = ex2(fmaf(s[e], scale_log2, -msafe));
+            p1 = ex2(fmaf(s[e + 1], scale_log2, -msafe));
+            sum4[(e / 2) & 3] += p0 + p1;
+          }
           __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
           packed[e / 2] = *reinterpret_cast<uint32_t*>(&pb);
           if (WIDE) {
@@ -454,11 +484,11 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
             rest[e / 2] = *reinterpret_cast<uint32_t*>(&rb);
           }
         }
-        l = l * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
+        if (!SIGMOID) l = l * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
         // The accumulator holds the pair's tiles 0 .. j - 1 once the second product of tile j - 1 is done. With one set
         // of score columns the scores of tile j were computed after it (the issuer's order). With two sets they were
         // issued before it: the group then waits for that product where it hands the values back.
-        if (j >= 1 && __any_sync(0xffffffffu, corr != 1.0f)) {
+        if (!SIGMOID && j >= 1 && __any_sync(0xffffffffu, corr != 1.0f)) {
           if (SB == 2) {
             if (!(ok = mbar_wait_limited(v_empty((kt - 1) % VS), (uint32_t)((kt - 1) / VS) & 1u, abortp, 10, &g_attention_tc_error))) break;
             tcgen05_fence_after();
@@ -505,8 +535,9 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
       if (ok && my_tiles > 0) ok = mbar_wait_limited(o_done(g), (uint32_t)outs & 1u, abortp, 8, &g_attention_tc_error);
       if (ok && my_tiles > 0) {
         tcgen05_fence_after();
-        if (sink != 0.f) l += ex2((sinks != nullptr && valid ? sinks[p.kvh * group + pr % group] * kLog2eTc : 0.f) - (m == -INFINITY ? 0.f : m));
-        const float inv = l > 0.f ? 1.0f / l : 0.f;
+        if (!SIGMOID && sink != 0.f) l += ex2((sinks != nullptr && valid ? sinks[p.kvh * group + pr % group] * kLog2eTc : 0.f) - (m == -INFINITY ? 0.f : m));
+        const float inv = SIGMOID ? 1.0f : (l > 0.f ? 1.0f / l : 0.f);
+        const __nv_bfloat16* gate = SIGMOID && valid && sg.gate != nullptr ? sg.gate + (size_t)(p.q_start + pr / group) * sg.ld_gate + (size_t)head * DV : nullptr;
         __nv_bfloat16* dst = valid ? out + ((size_t)(p.q_start + pr / group) * q_heads + p.kvh * group + pr % group) * DV : nullptr;
 #pragma unroll 1
         for (int c = 0; c < DV / 32; ++c) {
@@ -516,6 +547,12 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
 #pragma unroll
             for (int e = 0; e < 32; e += 8) {
               uint32_t o[4];
+              if (SIGMOID && gate != nullptr) {
+                float gv[8];
+                Vec<__nv_bfloat16>::load(gate + c * 32 + e, gv);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[e + u] = __float_as_uint(__uint_as_float(v[e + u]) * sigmoid_f(gv[u]));
+              }
 #pragma unroll
               for (int u = 0; u < 4; ++u) {
                 __nv_bfloat162 ob = __floats2bfloat162_rn(__uint_as_float(v[e + 2 * u]) * inv, __uint_as_float(v[e + 2 * u + 1]) * inv);
@@ -565,12 +602,12 @@ bool prefill_tc_serves(int head_dim, int q_heads, int kv_heads, int page_size, l
   return (uintptr_t)k_pool % 128 == 0 && (q == nullptr || (uintptr_t)q % 16 == 0) && encode_tiled() != nullptr;
 }
 
-template <int DK, int DV, int RPC, int NG, bool WIDE, bool FLAT>
-static int launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mq2, const CUtensorMap& mk2, TcFlat flat, void* out,
+template <int DK, int DV, int RPC, int NG, bool WIDE, bool FLAT, bool SIGMOID = false>
+static int launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mq2, const CUtensorMap& mk2, TcFlat flat, TcSigmoid sg, void* out,
                      const int32_t* q_indptr, const int32_t* kv_lens, const int32_t* kv_indptr, const int32_t* kv_indices, const int32_t* work, int items,
                      int q_heads, int kv_heads, int page_size, float scale, int window, const float* sinks, cudaStream_t s) {
   constexpr size_t smem = TcCfg<DK, DV, NG>::kSmem;
-  auto kernel = attention_prefill_tc_kernel<DK, DV, RPC, NG, WIDE, FLAT>;
+  auto kernel = attention_prefill_tc_kernel<DK, DV, RPC, NG, WIDE, FLAT, SIGMOID>;
   static int sms[64] = {};   // per device: its SM count, and that the kernel's shared-memory size has been set there
   int dev = 0;
   cudaGetDevice(&dev);
@@ -585,18 +622,16 @@ static int launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   // list better than the fixed walk (8 x 8192 tokens: 1017 against 885 TFLOP/s).
   const long long pairs = (long long)items * kv_heads;
   const int grid = (int)(pairs <= 8LL * sms[dev] ? (pairs < sms[dev] ? pairs : sms[dev]) : pairs);
-  launch_kernel(kernel, dim3(grid), dim3(64 + NG * 128), smem, s, mq, mk, mv, mq2, mk2, flat, (__nv_bfloat16*)out, q_indptr, kv_lens, kv_indptr, kv_indices,
+  launch_kernel(kernel, dim3(grid), dim3(64 + NG * 128), smem, s, mq, mk, mv, mq2, mk2, flat, sg, (__nv_bfloat16*)out, q_indptr, kv_lens, kv_indptr, kv_indices,
                 (const int2*)work, items, q_heads, kv_heads, page_size, scale * kLog2eTc, window, sinks);
   return check_launch("attention_prefill_tc");
 }
 
-int launch_prefill_tc(const void* q, long long tokens, void* out, const void* k_pool, const void* v_pool, const int32_t* q_indptr,
-                      const int32_t* kv_lens, const int32_t* kv_indptr, const int32_t* kv_indices, const int32_t* work, int items, int tile_rows,
-                      int q_heads, int kv_heads, int head_dim, int page_size, long long pool_pages, float scale, int window, const float* sinks, cudaStream_t s) {
-  if (tile_rows != 128 && tile_rows != 256) return fail(ROOST_ERR_INVALID, "attention_prefill: the tcgen05 kernel takes work items of 128 or 256 packed rows");
-  const int groups = tile_rows / kTcRows;
-  const int group = q_heads / kv_heads;
-  CUtensorMap mq;
+static int paged_box_rows(int page_size) { return page_size < 32 ? page_size : 32; }
+
+static int paged_maps(const void* q, long long tokens, const void* k_pool, const void* v_pool, int q_heads, int kv_heads, int head_dim, int page_size,
+                      long long pool_pages, CUtensorMap& mq, CUtensorMap& mk, CUtensorMap& mv) {
+  const int group = q_heads / kv_heads, box_rows = paged_box_rows(page_size);
   {
     // q [tokens][kv_heads][group][D] as 64 columns x group x kv heads x tokens x column blocks; a box is 128 packed rows
     // of one key/value head: [column block][token][head of the group][64]
@@ -609,9 +644,7 @@ int launch_prefill_tc(const void* q, long long tokens, void* out, const void* k_
                                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ROOST_ERR_CUDA, "attention_prefill: cuTensorMapEncodeTiled (q) failed with code " + std::to_string((int)r));
   }
-  const int box_rows = page_size < 32 ? page_size : 32;
   const cuuint64_t pool_rows = (cuuint64_t)(pool_pages * kv_heads * page_size);
-  CUtensorMap mk, mv;
   {
     const cuuint64_t dims[2] = {(cuuint64_t)head_dim, pool_rows};
     const cuuint64_t strides[1] = {(cuuint64_t)head_dim * 2};
@@ -632,13 +665,25 @@ int launch_prefill_tc(const void* q, long long tokens, void* out, const void* k_
                                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ROOST_ERR_CUDA, "attention_prefill: cuTensorMapEncodeTiled (values) failed with code " + std::to_string((int)r));
   }
+  return ROOST_OK;
+}
+
+int launch_prefill_tc(const void* q, long long tokens, void* out, const void* k_pool, const void* v_pool, const int32_t* q_indptr,
+                      const int32_t* kv_lens, const int32_t* kv_indptr, const int32_t* kv_indices, const int32_t* work, int items, int tile_rows,
+                      int q_heads, int kv_heads, int head_dim, int page_size, long long pool_pages, float scale, int window, const float* sinks, cudaStream_t s) {
+  if (tile_rows != 128 && tile_rows != 256) return fail(ROOST_ERR_INVALID, "attention_prefill: the tcgen05 kernel takes work items of 128 or 256 packed rows");
+  const int groups = tile_rows / kTcRows;
+  const int box_rows = paged_box_rows(page_size);
+  CUtensorMap mq, mk, mv;
+  const int rc = paged_maps(q, tokens, k_pool, v_pool, q_heads, kv_heads, head_dim, page_size, pool_pages, mq, mk, mv);
+  if (rc != ROOST_OK) return rc;
   const bool wide = (window & ROOST_ATTENTION_WIDE_WEIGHTS) != 0;
 #define ROOST_TC_CASE(DD, RR, GG)                                                                                                              \
   if (head_dim == DD && box_rows == RR && groups == GG) {                                                                                      \
     if (wide)                                                                                                                                  \
-      return launch_tc<DD, DD, RR, GG, true, false>(mq, mk, mv, mq, mk, TcFlat{}, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items,  \
+      return launch_tc<DD, DD, RR, GG, true, false>(mq, mk, mv, mq, mk, TcFlat{}, TcSigmoid{}, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items,  \
                                                     q_heads, kv_heads, page_size, scale, window, sinks, s);                                    \
-    return launch_tc<DD, DD, RR, GG, false, false>(mq, mk, mv, mq, mk, TcFlat{}, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items,   \
+    return launch_tc<DD, DD, RR, GG, false, false>(mq, mk, mv, mq, mk, TcFlat{}, TcSigmoid{}, out, q_indptr, kv_lens, kv_indptr, kv_indices, work, items,   \
                                                    q_heads, kv_heads, page_size, scale, window, sinks, s);                                     \
   }
   ROOST_TC_CASE(128, 16, 1)
@@ -724,7 +769,7 @@ extern "C" int roost_carried_attention_tc(const void* q, int64_t ld_q, void* out
   const int dk = nope + (rope ? 64 : 0);
 #define ROOST_TC_FLAT(KK, VV)                                                                                                                \
   if (dk == KK && vdim == VV)                                                                                                                \
-    return launch_tc<KK, VV, 128, 1, true, true>(mq, mk, mv, mq2, mk2, flat, out, q_indptr, kv_lens, nullptr, nullptr, nullptr, (int)items,  \
+    return launch_tc<KK, VV, 128, 1, true, true>(mq, mk, mv, mq2, mk2, flat, TcSigmoid{}, out, q_indptr, kv_lens, nullptr, nullptr, nullptr, (int)items,  \
                                                  heads, heads, 1, scale, w, sinks, (cudaStream_t)stream);
   ROOST_TC_FLAT(64, 64)
   ROOST_TC_FLAT(64, 128)
@@ -734,6 +779,51 @@ extern "C" int roost_carried_attention_tc(const void* q, int64_t ld_q, void* out
   ROOST_TC_FLAT(192, 128)
 #undef ROOST_TC_FLAT
   return fail(ROOST_ERR_UNSUPPORTED, "carried_attention: no tcgen05 kernel for these sizes");
+}
+
+// Sigmoid weights over the paged cache (two planes of one size), prompt portions and single tokens mixed: as roost_sigmoid_attention_mma. 0 where
+// these sizes, pools or addresses are not served.
+extern "C" int roost_sigmoid_attention_tc_supported(int dim, int vdim, int heads, int kv_heads, int page_size, long long pool_pages, const void* k_pool,
+                                                    const void* v_pool, const void* q, const void* out, const void* gate, int64_t ld_gate) {
+  return dim == vdim && prefill_tc_serves(dim, heads, kv_heads, page_size, pool_pages, k_pool, v_pool, q) && (uintptr_t)out % 16 == 0 &&
+         (gate == nullptr || ((uintptr_t)gate % 16 == 0 && ld_gate % 8 == 0));
+}
+
+extern "C" int roost_sigmoid_attention_tc(const void* q, void* out, const void* k_pool, const void* v_pool, long long pool_pages, const void* gate, int64_t ld_gate,
+                                          const float* slopes, const float* head_bias, const int32_t* q_indptr, const int32_t* kv_lens, const int32_t* kv_indptr,
+                                          const int32_t* kv_indices, int tokens, int rows, int heads, int kv_heads, int dim, int page_size, float scale,
+                                          roost_stream_t stream) {
+  ROOST_REQUIRE(tokens >= 0 && rows >= 0 && heads > 0 && kv_heads > 0 && page_size > 0 && heads % kv_heads == 0 && scale > 0.f, "sigmoid_attention_tc: sizes and the scale must be positive");
+  ROOST_REQUIRE(q && out && k_pool && v_pool && slopes && head_bias && q_indptr && kv_lens && kv_indptr && kv_indices, "sigmoid_attention_tc: a pointer is null");
+  ROOST_REQUIRE(gate == nullptr || ld_gate >= (int64_t)heads * dim, "sigmoid_attention_tc: a gate's row is too narrow");
+  if (!roost_sigmoid_attention_tc_supported(dim, dim, heads, kv_heads, page_size, pool_pages, k_pool, v_pool, q, out, gate, ld_gate))
+    return fail(ROOST_ERR_UNSUPPORTED, "sigmoid_attention_tc: sizes or addresses the tcgen05 form does not serve");
+  if (tokens == 0 || rows == 0) return ROOST_OK;
+  CUtensorMap mq, mk, mv;
+  const int rc = paged_maps(q, tokens, k_pool, v_pool, heads, kv_heads, dim, page_size, pool_pages, mq, mk, mv);
+  if (rc != ROOST_OK) return rc;
+  const int group = heads / kv_heads;
+  // two row groups a CTA where every processor gets a pair of them; with less work the smaller items spread over more processors
+  const int groups = (long long)tokens * heads >= 2LL * 148 * kTcRows ? 2 : 1;
+  const long long items = (long long)tokens * group / (groups * kTcRows) + rows;
+  if (items * kv_heads >= (1LL << 30)) return fail(ROOST_ERR_UNSUPPORTED, "sigmoid_attention_tc: too many tokens or heads");
+  const TcFlat flat = {0, rows, 0, 0};
+  const TcSigmoid sg = {slopes, head_bias, (const __nv_bfloat16*)gate, ld_gate};
+  const int box_rows = paged_box_rows(page_size);
+#define ROOST_TC_SIGMOID(DD, RR, GG)                                                                                                            \
+  if (dim == DD && box_rows == RR && groups == GG)                                                                                             \
+    return launch_tc<DD, DD, RR, GG, true, false, true>(mq, mk, mv, mq, mk, flat, sg, out, q_indptr, kv_lens, kv_indptr, kv_indices, nullptr,  \
+                                                        (int)items, heads, kv_heads, page_size, scale, 0, nullptr, (cudaStream_t)stream);
+  ROOST_TC_SIGMOID(64, 16, 1)
+  ROOST_TC_SIGMOID(64, 32, 1)
+  ROOST_TC_SIGMOID(64, 16, 2)
+  ROOST_TC_SIGMOID(64, 32, 2)
+  ROOST_TC_SIGMOID(128, 16, 1)
+  ROOST_TC_SIGMOID(128, 32, 1)
+  ROOST_TC_SIGMOID(128, 16, 2)
+  ROOST_TC_SIGMOID(128, 32, 2)
+#undef ROOST_TC_SIGMOID
+  return fail(ROOST_ERR_UNSUPPORTED, "sigmoid_attention_tc: no kernel for these sizes");
 }
 
 ROOST_TRACE_TU(attention_tc)

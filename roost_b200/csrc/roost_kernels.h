@@ -549,6 +549,12 @@ int roost_sigmoid_attention(const void* q, void* out, float* part, const void* k
 
 /* The same on the tensor cores (bfloat16; dim and vdim multiples of 16 up to 128, entry a multiple of 8), a block per (row, 64 query
  * tokens, query head): for steps that bring prompt portions. q_indptr: the rows' token ranges (rows + 1 entries). */
+int roost_sigmoid_attention_tc_supported(int dim, int vdim, int heads, int kv_heads, int page_size, long long pool_pages, const void* k_pool, const void* v_pool,
+                                         const void* q, const void* out, const void* gate, int64_t ld_gate);
+int roost_sigmoid_attention_tc(const void* q, void* out, const void* k_pool, const void* v_pool, long long pool_pages, const void* gate, int64_t ld_gate,
+                               const float* slopes, const float* head_bias, const int32_t* q_indptr, const int32_t* kv_lens, const int32_t* kv_indptr,
+                               const int32_t* kv_indices, int tokens, int rows, int heads, int kv_heads, int dim, int page_size, float scale,
+                               roost_stream_t stream);
 int roost_sigmoid_attention_mma_supported(int dim, int vdim, int entry);
 int roost_sigmoid_attention_mma(const void* q, void* out, const void* k_base, const void* v_base, int entry, const void* gate, int64_t ld_gate,
                                 const float* slopes, const float* head_bias, const int32_t* positions, const int32_t* q_indptr,

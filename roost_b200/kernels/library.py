@@ -183,6 +183,9 @@ _SIGNATURES = {
                                         c_int, c_int, c_float, c_float, c_int, c_int, c_int, c_void_p],
     "roost_sigmoid_attention": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p],
+    "roost_sigmoid_attention_tc_supported": [c_int, c_int, c_int, c_int, c_int, ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64],
+    "roost_sigmoid_attention_tc": [c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_longlong, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
     "roost_sigmoid_attention_mma_supported": [c_int, c_int, c_int],
     "roost_sigmoid_attention_mma": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_int, c_void_p],
@@ -1459,10 +1462,10 @@ class KernelLibrary:
         return bool(self._lib.roost_sigmoid_attention_mma_supported(int(dim), int(vdim), int(dim if two_planes else dim + vdim)))
 
     def sigmoid_attention(self, q, k_pool, v_pool, gate_rows, gate_col, slopes, head_bias, positions, token_row, kv_indptr, kv_indices, kv_heads, vdim,
-                          scale, kv_cap: int = 0, q_indptr: torch.Tensor | None = None) -> torch.Tensor:
+                          scale, kv_cap: int = 0, q_indptr: torch.Tensor | None = None, kv_lens: torch.Tensor | None = None) -> torch.Tensor:
         """out[t, h] = sum over visible keys j of sigmoid((q . k_j) scale - slopes[h] (p - j) + head_bias[h]) v_j, times
         sigmoid(gate_rows[t, gate_col + h * vdim : ...]) when ``gate_col`` is not None: [T, heads * vdim]. With ``q_indptr`` (the rows'
-        token ranges) a bfloat16 step runs on the tensor cores where the sizes allow; without, the 32-bit form, a token's keys dealt to
+        token ranges) a bfloat16 step runs on the tensor cores where the sizes allow (with ``kv_lens`` on tcgen05); without, the 32-bit form, a token's keys dealt to
         several blocks when the step alone would not fill the device."""
         _need(q, "q"); _need(k_pool, "k_pool", q.dtype); _need(slopes, "slopes", torch.float32); _need(head_bias, "head_bias", torch.float32)
         for n, t in (("positions", positions), ("token_row", token_row), ("kv_indptr", kv_indptr), ("kv_indices", kv_indices)):
@@ -1478,6 +1481,16 @@ class KernelLibrary:
             gate_ptr, ld_gate = gate_rows.data_ptr() + gate_col * gate_rows.element_size(), gate_rows.stride(0)
         kb, vb, entry = self._sink_cache(k_pool, v_pool, dim, vdim)
         out = torch.empty((T, heads * vdim), dtype=q.dtype, device=q.device)
+        if (q_indptr is not None and kv_lens is not None and v_pool is not None and q.dtype == torch.bfloat16
+                and self._lib.roost_sigmoid_attention_tc_supported(dim, vdim, heads, kv_heads, k_pool.shape[2], k_pool.shape[0], kb, vb, _ptr(q), _ptr(out),
+                                                                   gate_ptr, ld_gate)):
+            _need(q_indptr, "q_indptr", torch.int32); _need(kv_lens, "kv_lens", torch.int32)
+            rows = q_indptr.numel() - 1
+            if kv_lens.numel() < rows:
+                raise KernelError("sigmoid_attention: one length a row")
+            self._call("roost_sigmoid_attention_tc", _ptr(q), _ptr(out), kb, vb, k_pool.shape[0], gate_ptr, ld_gate, _ptr(slopes), _ptr(head_bias),
+                       _ptr(q_indptr), _ptr(kv_lens), _ptr(kv_indptr), _ptr(kv_indices), T, rows, heads, kv_heads, dim, k_pool.shape[2], float(scale), _stream())
+            return out
         if q_indptr is not None and q.dtype == torch.bfloat16 and self.sigmoid_attention_mma_supported(dim, vdim, v_pool is not None):
             _need(q_indptr, "q_indptr", torch.int32)
             # rows of more than SIGMOID_MMA_CHUNK_TILES tiles of 64 keys have the keys of their later queries dealt to several blocks;

@@ -86,7 +86,7 @@ class SigmoidAttention(Mixer):
         portions = not batch.all_single and batch.num_tokens >= getattr(k, "SIGMOID_MMA_MIN_TOKENS", 1 << 30)
         o = k.sigmoid_attention(q, cache.k_pool, cache.v_pool, qkv, gate_col, self.slopes, self.head_bias, batch.positions, batch.token_row,
                                 tables.kv_indptr, tables.kv_indices, s.num_kv_heads, s.v_dim, s.scale, kv_cap=batch.kv_cap,
-                                **({"q_indptr": batch.q_indptr} if portions else {}))
+                                **({"q_indptr": batch.q_indptr, "kv_lens": batch.kv_lens} if portions else {}))
         return self.out(o)
 
 

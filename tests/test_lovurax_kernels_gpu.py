@@ -292,3 +292,46 @@ def test_the_gather_of_cached_vectors_leaves_out_pages_that_were_given_back(kern
         want = torch.zeros(16, width, dtype=torch.bfloat16, device="cuda")
         want[4:8], want[8:10] = pool[5, 0], pool[2, 0, :2]
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,page,gated", [(4, 2, 64, 16, True), (16, 1, 128, 16, True), (8, 8, 128, 32, False), (32, 4, 64, 32, True)])
+def test_sigmoid_weights_on_tcgen05(kernels, heads, kv_heads, dim, page, gated):
+    """Prompt portions beside the key tiles' edges that start inside their keys, a row of one token and a padding row, one and two row groups a
+    CTA (by the step's size); unseen slots hold what no result may show. Against 64 bits, and no further from it than the mma.sync form."""
+    g = torch.Generator().manual_seed(heads + dim)
+    lens, counts = ([129, 640, 300], [129, 387, 1]) if heads < 32 else ([1500, 129, 300], [1500, 65, 1])
+    T, group, scale = sum(counts), heads // kv_heads, 1.5 / math.sqrt(dim)
+    need = [-(-n // page) for n in lens]
+    order = torch.randperm(sum(need) + 3, generator=g)[: sum(need)]
+    pool = torch.full((2, sum(need) + 3, kv_heads, page, dim), float("nan"), dtype=torch.bfloat16)
+    kv, at = [torch.randn(2, n, kv_heads, dim, generator=g).to(torch.bfloat16) for n in lens], 0
+    for x, n in zip(kv, need):
+        for p in range(n):
+            part = x[:, p * page : (p + 1) * page].transpose(1, 2)
+            pool[:, order[at + p], :, : part.shape[2]] = part
+        at += n
+    pool = pool.cuda()
+    q = torch.randn(T + 3, heads, dim, generator=g).to(torch.bfloat16)
+    rows = torch.randn(T + 3, heads * dim + 16, generator=g).to(torch.bfloat16)
+    slopes, bias = torch.tensor(P.head_slopes(heads), dtype=torch.float32), torch.randn(heads, generator=g) - 1.0
+    positions = torch.cat([torch.arange(n - m, n) for n, m in zip(lens, counts)] + [torch.full((3,), -1)]).to(torch.int32)
+    token_row = torch.tensor([r for r, m in enumerate(counts) for _ in range(m)] + [3] * 3, dtype=torch.int32)
+    want, t = torch.zeros(T, heads, dim, dtype=torch.float64), 0
+    for (k, v), n, m in zip(kv, lens, counts):
+        i, j = torch.arange(n - m, n, dtype=torch.float64)[:, None], torch.arange(n, dtype=torch.float64)[None]
+        for h in range(heads):
+            s = q[t : t + m, h].double() @ k[:, h // group].double().T * scale - float(slopes[h]) * (i - j) + float(bias[h])
+            want[t : t + m, h] = (P.sigmoid(s) * (j <= i)) @ v[:, h // group].double()
+        t += m
+    want = want.reshape(T, -1)
+    if gated:
+        want = want * P.sigmoid(rows[:T, 16:].double())
+    indptr = [0] + torch.tensor(need).cumsum(0).tolist()
+    off = {}
+    for form, kv_lens in (("mma.sync", None), ("tcgen05", i32(lens + [0]))):
+        got = kernels.sigmoid_attention(q.cuda(), pool[0], pool[1], rows.cuda(), 16 if gated else None, slopes.cuda(), bias.cuda(), positions.cuda(), token_row.cuda(),
+                                        i32(indptr + indptr[-1:]), i32(order.tolist()), kv_heads, dim, scale, kv_cap=2048,
+                                        q_indptr=i32([0] + torch.tensor(counts + [3]).cumsum(0).tolist()), kv_lens=kv_lens)
+        off[form] = float((got[:T].double().cpu() - want).norm() / want.norm())
+    print(f"MEASURED sigmoid weights: {off}")
+    assert off["tcgen05"] < 1.1 * off["mma.sync"] and off["tcgen05"] < 2.0 ** -8       # the output's rounding to bfloat16

@@ -15,7 +15,7 @@
 //              element by element by sigmoid(gate) where a gate is given (columns of the same projection row). A token's tiles
 //              may be dealt to several blocks in ranges; the partial sums are then added in split order by a second kernel. A
 //              padding token (position -1) is skipped.
-#include "common.cuh"
+#include "head_prepare.cuh"
 
 namespace roost {
 
@@ -224,6 +224,11 @@ extern "C" int roost_sigmoid_attention_prepare(const void* qkv, int64_t ld, void
                 "sigmoid_attention_prepare: a row or a cache entry is too narrow");
   if (dim > kSgMaxDim) return fail(ROOST_ERR_UNSUPPORTED, "sigmoid_attention_prepare: heads beyond 512 numbers");
   if (tokens == 0) return ROOST_OK;
+  const HeadPrepare a = {ld, entry, tokens, heads, kv_heads, vdim, page_size, nullptr, 0, 0, 1.f, eps, q_w, k_w, temp_coef, temp_every, positions, slot_mapping};
+  if (head_prepare_serves(qkv, q_out, k_base, v_base, dim, a, dtype)) {
+    ROOST_DISPATCH_DTYPE(dtype, T, launch_head_prepare<T>(const_cast<void*>(qkv), q_out, k_base, v_base, dim, a, (cudaStream_t)stream));
+    return check_launch("sigmoid_attention_prepare");
+  }
   ROOST_DISPATCH_DTYPE(dtype, T, launch_kernel(sigmoid_prepare_kernel<T>, dim3(tokens), dim3(128), 0, (cudaStream_t)stream, (const T*)qkv, ld, (T*)q_out,
                                                (T*)k_base, (T*)v_base, entry, q_w, k_w, positions, slot_mapping, heads, kv_heads, dim, vdim, eps,
                                                temp_coef, temp_every, page_size));

@@ -23,7 +23,7 @@
 //   prepare_normed: the other preparation: all query heads of a token side by side are divided by one root mean square and multiplied
 //              by a weight as wide as they are, the key heads side by side likewise; nothing is rotated. Queries go to q_out (rows
 //              ld_q apart: the projection's own rows, or a dense tensor), keys and values to the token's cache slot.
-#include "common.cuh"
+#include "head_prepare.cuh"
 
 namespace roost {
 
@@ -345,6 +345,11 @@ extern "C" int roost_sink_attention_prepare(void* qkv, int64_t ld, void* q_out, 
                 "sink_attention_prepare: a row or a cache entry is too narrow");
   if (dim > kSaMaxDim) return fail(ROOST_ERR_UNSUPPORTED, "sink_attention_prepare: heads beyond 512 numbers");
   if (tokens == 0) return ROOST_OK;
+  const HeadPrepare a = {ld, entry, tokens, heads, kv_heads, vdim, page_size, inv_freq, rot_dims, halves, amplitude, eps, nullptr, nullptr, 0.f, 1, positions, slot_mapping};
+  if (head_prepare_serves(qkv, q_out, k_base, v_base, dim, a, dtype)) {
+    ROOST_DISPATCH_DTYPE(dtype, T, launch_head_prepare<T>(qkv, q_out, k_base, v_base, dim, a, (cudaStream_t)stream));
+    return check_launch("sink_attention_prepare");
+  }
   const size_t smem = ((size_t)rot_dims + 2) * sizeof(float);
   // four warps a token: measured faster than a warp a head (sixteen warps: 30.7 against 19.6 us at 2,048 tokens of 16 + 4 heads of 64)
   ROOST_DISPATCH_DTYPE(dtype, T, launch_kernel(sink_prepare_kernel<T>, dim3(tokens), dim3(128), smem, (cudaStream_t)stream, (T*)qkv, ld, (T*)q_out, (T*)k_base,

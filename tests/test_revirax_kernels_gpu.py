@@ -318,3 +318,32 @@ def test_wide_weights_on_tcgen05(kernels, heads, kv_heads, dim, page, window):
         here = off(run(tile_rows))
         print(f"MEASURED wide weights, items of {tile_rows}: {here:.3e} on tcgen05, {mma:.3e} on mma.sync")
         assert here < 1.1 * mma and here < 2.0 ** -8       # the output's own rounding to bfloat16 is all that shows
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens", [5, 701])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,rot,halves,eps", [(4, 2, 64, 64, 64, False, 1e-6), (5, 1, 128, 128, 128, True, 1e-6), (16, 4, 128, 64, 64, True, None),
+                                                                    (3, 3, 64, 40, 18, False, None), (8, 2, 64, 64, 32, True, 1e-6), (7, 7, 128, 128, 0, False, 1e-6)])
+def test_prepared_heads_a_piece_a_lane(kernels, dtype, tokens, heads, kv_heads, dim, vdim, rot, halves, eps):
+    """A row whose columns start off a whole piece takes the form of a number at a time: the two differ by the last bits of sums and products."""
+    g = torch.Generator().manual_seed(heads * dim + rot)
+    page, width = 16, (heads + kv_heads) * dim + kv_heads * vdim
+    rows = torch.randn(tokens, width, generator=g).to(dtype)
+    slots = torch.randperm(tokens + 40, generator=g)[:tokens].to(torch.int32)
+    slots[tokens // 2] = -1                                                    # a padding token
+    positions = torch.randint(0, 5000, (tokens,), generator=g, dtype=torch.int32)
+    freq = torch.rand(max(rot // 2, 1), generator=g, dtype=torch.float64).cuda()
+    out = []
+    for shift in (8, 9):
+        wide = torch.zeros(tokens, width + 16, dtype=dtype, device="cuda")
+        wide[:, shift : shift + width] = rows.cuda()
+        planes = 2 if dim == vdim else 1
+        pool = torch.zeros((planes, (tokens + 40) // page + 1, kv_heads, page, dim if planes == 2 else dim + vdim), dtype=dtype, device="cuda")
+        q = torch.zeros(tokens, heads, dim, dtype=dtype, device="cuda")
+        kernels.sink_attention_prepare(wide[:, shift : shift + width], pool[0], pool[1] if planes == 2 else None, freq if rot else None, rot, positions.cuda(),
+                                       slots.cuda(), heads, kv_heads, dim, vdim, eps, page, q_out=q, halves=halves, amplitude=1.25)
+        out.append((q, pool))
+    for what, a, b in zip(("queries", "cache"), *out):
+        off = float((a.double() - b.double()).abs().max() / b.double().abs().max())
+        print(f"MEASURED prepared {what} {dtype}: {off:.2e}")
+        assert off < (2.0 ** -21 if dtype == torch.float32 else 2.0 ** -7), what     # a few units of the sums' last place, then one rounding to the other side

@@ -409,3 +409,47 @@ def test_gated_group_norm_at_every_width(kernels, dtype, size, groups):
     v = y.double().cpu() * z * torch.sigmoid(z)
     want = P.unit_rms(v.reshape(5, groups, size), 1e-6).reshape(5, -1) * w.double().cpu()
     close(kernels.gated_group_norm(y, u, w, groups, 1e-6, dtype), want, dtype, "gated group norm")
+
+
+@pytest.mark.parametrize("T,E,top", [(1, 1, 1), (700, 3, 3), (2049, 700, 1), (900, 701, 5), (1500, 64, 6)])
+def test_pairs_sorted_by_one_block_and_by_a_cluster(kernels, T, E, top):
+    """Ranges, tiles of both widths and the sorted rows from the choices alone, twice (the counts are left at zero), experts that nobody chose."""
+    g = torch.Generator().manual_seed(E)
+    logits = torch.randn(T, E, generator=g)
+    logits[:, : E // 2] -= 3.0 * (E > 8)
+    for _ in range(2):
+        route = kernels.moe_route(logits.cuda(), top)
+    chosen = torch.topk(logits, top, dim=1).indices
+    counts = torch.bincount(chosen.flatten(), minlength=E)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+    assert torch.equal(route.offsets.cpu().long(), offsets)
+    inverse = route.inverse.cpu().long().reshape(T, top)
+    assert torch.equal(inverse.flatten().sort().values, torch.arange(T * top))
+    assert torch.equal(route.expert.cpu().long()[inverse].sort(1).values, chosen.sort(1).values)
+    assert torch.equal(route.token.cpu().long()[inverse], torch.arange(T)[:, None].expand(T, top))
+    want = torch.sigmoid(logits.double())[torch.arange(T)[:, None], route.expert.cpu().long()[inverse]]
+    assert float((route.weight.cpu().double()[inverse] - want).abs().max()) < 1e-6
+    for tiles, width in ((route.tiles, 64), (route.wide_tiles, 128)):
+        if tiles is None:
+            continue
+        rows = [(e, r, min(r + width, int(offsets[e + 1]))) for e in range(E) for r in range(int(offsets[e]), int(offsets[e + 1]), width)]
+        got = tiles.cpu().reshape(-1, 3)
+        assert [tuple(t) for t in got[: len(rows)].tolist()] == rows and (got[len(rows):, 0] == -1).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hidden", [4, 36, 264, 2048])
+def test_rows_gathered_and_combined_at_every_width(kernels, dtype, hidden):
+    g = torch.Generator().manual_seed(hidden)
+    T, E, top = 37, 5, 3
+    logits, x = torch.randn(T, E, generator=g), torch.randn(T, hidden, generator=g).to(dtype)
+    route = kernels.moe_route(logits.cuda(), top)
+    token, weight, inverse = route.token.cpu().long(), route.weight.cpu(), route.inverse.cpu().long().reshape(T, top)
+    assert torch.equal(kernels.moe_gather_scale(x.cuda(), route, scale=False).cpu(), x[token])
+    assert torch.equal(kernels.moe_gather_scale(x.cuda(), route).cpu(), (weight[:, None] * x[token].float()).to(dtype))
+    ys, shared = torch.randn(T * top, hidden, generator=g).to(dtype), torch.randn(T, hidden, generator=g).to(dtype)
+    total = torch.zeros(T, hidden)
+    for k in range(top):
+        total += ys[inverse[:, k]].float()
+    assert torch.equal(kernels.moe_combine(ys.cuda(), route, None).cpu(), total.to(dtype))
+    assert torch.equal(kernels.moe_combine(ys.cuda(), route, shared.cuda()).cpu(), (total + shared.float()).to(dtype))

@@ -106,3 +106,17 @@ def test_the_matrix_memory_walked_and_in_chunks(kernels, dtype, heads, dim, vdim
         close(got[:, :, -1], M, torch.float32, f"its m, call {call}")
     assert float(state[:, heads * per_head :].abs().max()) == 0.0
     assert float(state[7].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,vdim", [(2, 4), (3, 64), (16, 128), (2, 132), (5, 256), (2, 512), (2, 516), (3, 30)])
+@pytest.mark.parametrize("gate", ["silu", "sigmoid"])
+def test_head_norm_and_gate_at_every_width(kernels, dtype, heads, vdim, gate):
+    g = torch.Generator().manual_seed(vdim)
+    T, col = 11, 4
+    o, w = torch.randn(T, heads * vdim, generator=g) * 3, torch.randn(heads * vdim, generator=g)
+    u = torch.randn(T, col + heads * vdim + 4, generator=g).to(dtype)
+    z = u.double()[:, col : col + heads * vdim]
+    x = o.double().reshape(T, heads, vdim)
+    want = (x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6)).reshape(T, -1) * w.double() * torch.sigmoid(z) * (z if gate == "silu" else 1.0)
+    close(kernels.head_norm_gate(o.cuda(), u.cuda(), col, w.cuda(), heads, 1e-6, dtype, gate=gate).cpu(), want, dtype, "head norm and gate")

@@ -39,7 +39,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) gla_prepare_kernel(const T* u, int64_t ld, int a_col, const T* __restrict__ w,
                                                          const float* __restrict__ bias, float* __restrict__ alpha, int tokens, int channels, int rank,
                                                          float inv_tau) {
-  extern __shared__ float rows[];      // [kGlaPrepareTokens][rank]
+  extern __shared__ __align__(16) float rows[];      // [kGlaPrepareTokens][rank]
   pdl_launch_dependents();
   pdl_wait();
   const int t0 = blockIdx.x * kGlaPrepareTokens;
@@ -53,11 +53,26 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(const T* u, int64_t ld
 #pragma unroll
   for (int j = 0; j < kGlaPrepareTokens; ++j) z[j] = 0.f;
   const T* wc = w + (size_t)c * rank;
-  for (int r = 0; r < rank; ++r) {
-    const float x = to_float(wc[r]);
+  constexpr int V = Vec<T>::N;
+  if (rank % V == 0 && (uintptr_t)w % 16 == 0) {       // whole 16-byte pieces of the channel's row: the same sums in the same order
+    for (int r = 0; r < rank; r += V) {
+      float x[V];
+      Vec<T>::load(wc + r, x);
 #pragma unroll
-    for (int j = 0; j < kGlaPrepareTokens; ++j)
-      if (j < n) z[j] = fmaf(rows[j * rank + r], x, z[j]);
+      for (int j = 0; j < kGlaPrepareTokens; ++j)
+#pragma unroll
+        for (int e = 0; e < V; e += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(rows + j * rank + r + e);
+          z[j] = fmaf(a.w, x[e + 3], fmaf(a.z, x[e + 2], fmaf(a.y, x[e + 1], fmaf(a.x, x[e], z[j]))));
+        }
+    }
+  } else {
+    for (int r = 0; r < rank; ++r) {
+      const float x = to_float(wc[r]);
+#pragma unroll
+      for (int j = 0; j < kGlaPrepareTokens; ++j)
+        if (j < n) z[j] = fmaf(rows[j * rank + r], x, z[j]);
+    }
   }
 #pragma unroll
   for (int j = 0; j < kGlaPrepareTokens; ++j)

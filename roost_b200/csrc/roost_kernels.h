@@ -389,6 +389,11 @@ int roost_gla_prepare(const void* u, int64_t ld, int a_col, const void* w, const
  * scan makes the decays from the rows' a1 columns itself (steps of one token a row). ws: float[roost_gla_scan_chunks(tokens, rows) * heads *
  * dim * vdim] and ws_keep: float[chunks * heads * dim], or both null; with them rows are cut into chunks of 64 tokens that run side by side
  * (three launches). */
+/* Prompt portions in chunks of 16 tokens on the tensor cores (gla_chunks.cu): the parts a step's rows are cut into (0: whole rows, no workspace), -1 for
+ * sizes it does not serve; ws float[parts * heads * dim * vdim], ws_keep float[parts * heads * dim], or null for whole rows. */
+int roost_gla_chunks_parts(int rows, int tokens, int heads, int dim, int vdim, int dtype);
+int roost_gla_chunks(const void* u, int64_t ld, float q_scale, const float* alpha, float* out, float* state, int64_t state_stride, const int32_t* q_indptr,
+                     const int32_t* slots, int rows, int tokens, int heads, float* ws, float* ws_keep, roost_stream_t stream);
 int roost_gla_scan_chunks(int tokens, int rows);
 int roost_gla_scan(const void* u, int64_t ld, float q_scale, const float* alpha, int a_col, const void* w, const float* bias, int rank, float tau,
                    float* out, float* state, int64_t state_stride, const int32_t* q_indptr, const int32_t* slots, int rows, int tokens, int heads,

@@ -130,6 +130,8 @@ _SIGNATURES = {
     "roost_latent_attention_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                   c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
     "roost_gla_prepare": [c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p],
+    "roost_gla_chunks_parts": [c_int, c_int, c_int, c_int, c_int, c_int],
+    "roost_gla_chunks": [c_void_p, c_int64, c_float, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
     "roost_gla_scan_chunks": [c_int, c_int],
     "roost_gla_scan": [c_void_p, c_int64, c_float, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
                        c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p],
@@ -1332,8 +1334,8 @@ class KernelLibrary:
                  single: bool = False, chunked: bool | None = None) -> torch.Tensor:
         """S <- diag(alpha) S + k v^T, o = S^T q a head over rows [q heads | k heads | v heads | ... a1 from ``a_col`` on] of ``u``, alpha =
         sigmoid(a1 gate_w^T + gate_bias)^(1 / tau): float32 [T, heads * vdim]; see csrc/gated_linear_attention.cu. ``single``: every row brings
-        one token, the scan makes the decays itself. ``chunked`` None: steps of ``SCAN_CHUNKED_MIN_TOKENS`` tokens or more cut their rows into
-        chunks."""
+        one token, the scan makes the decays itself. ``chunked`` None: prompt portions run on the tensor cores where the sizes allow, else steps
+        of ``SCAN_CHUNKED_MIN_TOKENS`` tokens or more cut their rows into chunks; True and False force the walk with and without chunks."""
         _need_rows(u, "u"); _need(gate_w, "gate_w", u.dtype); _need(gate_bias, "gate_bias", torch.float32); _need(state, "state", torch.float32)
         _need(q_indptr, "q_indptr", torch.int32); _need(slots, "slots", torch.int32)
         T, (channels, rank) = u.shape[0], gate_w.shape
@@ -1345,6 +1347,15 @@ class KernelLibrary:
             alpha = torch.empty((T, channels), dtype=torch.float32, device=u.device)
             self._call("roost_gla_prepare", _ptr(u), u.stride(0), a_col, _ptr(gate_w), _ptr(gate_bias), _ptr(alpha), T, channels, rank, float(tau),
                        dtype_code(u.dtype), _stream())
+            whole = u.data_ptr() % 16 == 0 and u.stride(0) % 8 == 0 and chunked is None
+            parts = self._lib.roost_gla_chunks_parts(slots.numel(), T, heads, dim, vdim, dtype_code(u.dtype)) if whole else -1
+            if parts >= 0:       # prompt portions on the tensor cores
+                if parts:
+                    ws = torch.empty((parts * heads * dim * vdim,), dtype=torch.float32, device=u.device)
+                    ws_keep = torch.empty((parts * channels,), dtype=torch.float32, device=u.device)
+                self._call("roost_gla_chunks", _ptr(u), u.stride(0), float(q_scale), _ptr(alpha), _ptr(out), _ptr(state), state.stride(0), _ptr(q_indptr),
+                           _ptr(slots), slots.numel(), T, heads, _ptr(ws), _ptr(ws_keep), _stream(), launches=3 if parts else 1)
+                return out
             if (T >= self.SCAN_CHUNKED_MIN_TOKENS) if chunked is None else chunked:
                 chunks = self._lib.roost_gla_scan_chunks(T, slots.numel())
                 ws = torch.empty((chunks * heads * dim * vdim,), dtype=torch.float32, device=u.device)

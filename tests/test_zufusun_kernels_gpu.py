@@ -259,3 +259,40 @@ def test_gated_linear_attention(kernels, dtype, heads, dim, vdim, rank, tau, for
                 want[t] = torch.einsum("hd,hdv->hv", q[t], S[slot])
         close(got.cpu(), want.reshape(T, V), torch.float32, f"outputs of call {call}", f32=1e-4)
         close(state[:, : QK * vdim].cpu(), S.reshape(8, -1), torch.float32, f"states after call {call}", f32=1e-4)
+
+
+@pytest.mark.parametrize("tau,odd", [(16.0, False), (16.0, True), (1.0, False), (0.02, False)])
+@pytest.mark.parametrize("lengths", [[1, 16, 17], [300, 31], [64, 1, 200, 8]])
+def test_gated_linear_attention_in_chunks_on_the_tensor_cores(kernels, lengths, tau, odd):
+    """Edges of chunks and segments, rows of one token, carried states, decays from hardly any to complete; against 64 bits, and no further from it
+    than the walk in 32 bits over the same numbers. A value that is not finite shows from its own token on and not before."""
+    heads, dim, vdim, rank, T = 3, 64, 128, 16, sum(lengths)
+    g = torch.Generator().manual_seed(T)
+    width = heads * (2 * dim + vdim)
+    u = torch.randn(T, width + rank, generator=g).to(torch.bfloat16)
+    w = (torch.randn(heads * dim, rank, generator=g) * 0.5).to(torch.bfloat16)
+    bias, state = torch.randn(heads * dim, generator=g), torch.randn(len(lengths), heads * dim * vdim, generator=g)
+    if odd:
+        u[T - 5, 2 * heads * dim + 130], u[T - 3, 70] = float("inf"), float("nan")
+    x = u.double()
+    q, k, v = x[:, : heads * dim].reshape(T, heads, dim) * dim ** -0.5, x[:, heads * dim : 2 * heads * dim].reshape(T, heads, dim), x[:, 2 * heads * dim : width].reshape(T, heads, vdim)
+    fade = torch.sigmoid(x[:, width:] @ w.double().T + bias.double()).pow(1.0 / tau).reshape(T, heads, dim)
+    S, want, at = state.double().reshape(-1, heads, dim, vdim).clone(), [], 0
+    for r, n in enumerate(lengths):
+        for t in range(at, at + n):
+            S[r] = fade[t][:, :, None] * S[r] + k[t][:, :, None] * v[t][:, None]
+            want.append(torch.einsum("hdv,hd->hv", S[r], q[t]))
+        at += n
+    want = torch.stack(want).reshape(T, -1)
+    indptr, slots = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32).cuda(), torch.arange(len(lengths), dtype=torch.int32).cuda()
+    got = {}
+    for dtype in (torch.float32, torch.bfloat16):
+        s = state.cuda()
+        o = kernels.gla_scan(u.to(dtype).cuda(), width, w.to(dtype).cuda(), bias.cuda(), tau, dim ** -0.5, s, indptr, slots, heads, dim, vdim)
+        got[dtype] = (o.double().cpu(), s.double().cpu().reshape(S.shape))
+    for what, exact, i in (("outputs", want, 0), ("states", S, 1)):
+        fine = torch.isfinite(exact)
+        assert torch.equal(torch.isfinite(got[torch.bfloat16][i]), fine), what
+        walk, here = (float((got[d][i] - exact)[fine].norm() / exact[fine].norm()) for d in (torch.float32, torch.bfloat16))
+        print(f"MEASURED gated linear attention in chunks, {what}: {here:.2e}, the walk {walk:.2e}")
+        assert here < max(2 * walk, 1e-6), what         # float32 sums of up to 64 and 16 terms: a few units of 2^-24, whichever the order

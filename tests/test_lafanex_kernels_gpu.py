@@ -461,3 +461,35 @@ def test_the_command_line_writes_a_lafanex_folder_and_generates_from_it(tmp_path
         top = logits[len(prompt) - 1 + j].topk(2)
         if float(top.values[0] - top.values[1]) > 1e-3:
             assert tok == int(top.indices[0]), (j, tok, int(top.indices[0]))
+
+
+@pytest.mark.parametrize("lengths,inner,slow", [([130, 1, 64, 17], 64, False), ([600, 300], 128, False), ([1500, 63], 64, True)])
+def test_chunked_scan_of_sixteen_state_numbers(kernels, lengths, inner, slow):
+    """The walk with two lanes a channel against 64 bits, and no further from it than the walk for any sizes over the same numbers (rows of the
+    projection that are no whole 16-byte pieces take that one): edges of stages and chunks, carried states, decays just below one."""
+    g = torch.Generator().manual_seed(inner + len(lengths))
+    r = lambda *shape: torch.randn(*shape, generator=g)
+    T, rank, N = sum(lengths), 8, 16
+    a = -torch.exp(-1 + torch.rand(inner, N, generator=g)) if slow else -torch.exp(-2 + 2 * torch.rand(inner, N, generator=g))
+    dt_bias, d = (torch.full((inner,), -6.0) if slow else -1 + 0.5 * r(inner)), 1 + 0.3 * r(inner)
+    xc, dbc, xz, dt_raw = r(T, inner).bfloat16(), r(T, rank + 2 * N).bfloat16(), r(T, 2 * inner).bfloat16(), (0.3 if slow else 1.0) * r(T, inner)
+    state = r(len(lengths), inner * N)
+    indptr = i32([0] + torch.tensor(lengths).cumsum(0).tolist())
+    got = []
+    for pad in (0, 1):
+        st = state.cuda()
+        y = kernels.mamba1_scan(xc.cuda(), dt_raw.cuda(), torch.nn.functional.pad(dbc, (0, pad)).cuda(), xz.cuda(), dt_bias.cuda(), a.cuda(), d.cuda(), st, indptr,
+                                i32(range(len(lengths))), inner, N, rank, chunked=True)
+        got.append((y.double().cpu(), st.double().cpu()))
+    want, S, at = [], [], 0
+    for b, n in enumerate(lengths):
+        rows = slice(at, at + n)
+        y, s = plain_scan(xc[rows].double(), dt_raw[rows].double(), dbc[rows].double(), xz[rows, inner:].double(), dt_bias.double(), a.double(), d.double(),
+                          state[b].double().reshape(inner, N), rank, N)
+        want.append(y)
+        S.append(s.flatten())
+        at += n
+    for what, exact, i in (("outputs", torch.cat(want), 0), ("states", torch.stack(S), 1)):
+        here, other = (float((x[i] - exact).norm() / exact.norm()) for x in got)
+        print(f"MEASURED chunked scan of 16, {what}: {here:.3e}, the walk for any sizes {other:.3e}")
+        assert here < 1.1 * other, what               # the same decays; products of the two walks may be contracted otherwise

@@ -20,6 +20,8 @@
 // chunk's own S' and P, one thread an entry then carries the row's state from chunk to chunk leaving every chunk's true starting state
 // in the place of S', and a second walk of every chunk from there writes the outputs and, from a row's last chunk, the slot.
 //
+// Prompt portions in bfloat16 with heads of 64 keys and 128 values take gla_chunks.cu instead of these walks.
+//
 // What an earlier kernel of the step writes comes through pointers without __restrict__: with it the compiler may load before pdl_wait().
 #include "common.cuh"
 

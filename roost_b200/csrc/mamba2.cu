@@ -11,6 +11,7 @@
 //               the slot. 32-bit throughout; x, B, C are read in the activation dtype, y is written in 32-bit.
 //   gated_group_norm: g = y * silu(z); each of `groups` equal parts of a token's g is divided by its root mean square (eps
 //               inside the root) and multiplied by the weight; the output has the activation dtype.
+// Prompt portions in bfloat16 of the sizes that mamba2_chunks.cu names run the scan there, as products on the tensor cores.
 // Rows are given by q_indptr (token range) and state_slots (slot per row); the padding rows of a captured step name a scratch
 // slot. Every sum's order depends on the sizes only, never on the batch.
 #include "common.cuh"

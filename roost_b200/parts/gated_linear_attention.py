@@ -5,7 +5,8 @@ Per step: one projection gives a token's [q | k | v | g | a1] (g: the output gat
 numbers); one kernel makes the decays alpha = sigmoid(W a1 + bias)^(1 / tau) in 32-bit; one walks every (row, head) through its tokens with
 the head's matrix in registers, S <- diag(alpha) S + k v^T, o = S^T q head_dim^(-1/2); one divides each head's o by its root mean square,
 multiplies by a weight that the heads share and by g sigmoid(g), and rounds once; then the output projection. In a decode step the walk
-makes the decays itself: one kernel fewer. Steps of many tokens cut their rows into chunks that run side by side.
+makes the decays itself: one kernel fewer. Steps of many tokens cut their rows into chunks that run side by side; in bfloat16,
+with heads of 64 keys and 128 values, a walk takes 16 tokens at a time on the tensor cores.
 
 A request's slot holds S [heads, head_dim, v_dim] as one float32 vector; the executor zeroes it when the request's first token arrives.
 The kernels read the step's device tables only, so steps are captured.

@@ -4,7 +4,8 @@ Per step: the input projection gives a token's [z | x | B | C | dt]; one kernel 
 over [x | B | C], reading the taps before a row's first token from the request's state; one kernel moves the row's last
 ``conv_taps`` - 1 inputs into the state; one kernel walks every (row, head) through its tokens,
 S <- exp(-exp(A_log) dt) S + dt B x^T, y = S^T C + D x with dt = softplus(dt + dt_bias), the state S (``state`` x
-``head_dim``, 32-bit) read from and written back to the request's slot; one kernel multiplies y by SiLU(z), divides each
+``head_dim``, 32-bit) read from and written back to the request's slot (bfloat16 steps of prompts take 64 tokens at a
+time as products on the tensor cores, in segments that run side by side); one kernel multiplies y by SiLU(z), divides each
 of ``norm_groups`` equal parts by its root mean square and applies the weight; then the output projection. Everything
 that enters the recurrence besides the projection and the convolution's output is 32-bit.
 

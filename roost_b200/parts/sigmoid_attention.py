@@ -6,8 +6,8 @@ position, 1 + c ln(floor((p + 1) / every) + 1), writes them to a tensor of their
 page slots; attention of the step's queries over the pages, key j of query i weighing sigmoid((q_i . k_j) scale - slope_h (i - j)
 + b_h), the weighted sum of the values multiplied by sigmoid(gate) in the same kernel; the output projection. Scores, weights and
 sums are 32-bit. A step of few rows deals a token's keys to several blocks whose partial sums a second kernel adds in order; a
-bfloat16 step that brings prompt portions runs the same sums on the tensor cores (mma.sync), the 32-bit weights entering P V as two
-bfloat16 operands.
+bfloat16 step that brings prompt portions runs the same sums on the tensor cores (tcgen05 where the sizes and the cache's alignment
+allow, else mma.sync), the 32-bit weights entering P V as two bfloat16 operands.
 
 The cache is a paged group: two planes (keys, values) when keys and values have one size, else one plane whose entries are
 [key | value] of one key/value head.

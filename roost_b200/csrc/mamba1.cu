@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kM1Threads) mamba1_scan_kernel(const T* __rest
 // The chunked walks for a state of 16 numbers a channel in bfloat16, channels in blocks of 64 and whole 16-byte pieces. Two lanes share a channel; of
 // every two tokens each lane makes one token's step size and one token's output. The next 16 tokens' inputs arrive by cp.async; B and C are
 // widened once for the block's 64 channels. Bound by the special-function unit and issue slots: 2,348 tokens of 2,048 channels, first and second
-// walk 70 + 171 us in the form above (its staging made the step sizes between two barriers); the layer 295 us, 204 so. The exponential is the accurate
+// walk 70 + 171 us in the form above (its staging made the step sizes between two barriers); the layer 295 us, 204 so (187 with the carry below as it is now). The exponential is the accurate
 // one: with ex2.approx on a prescaled argument the layer took 177 us, but the states were 1.7 times as far from 64 bits.
 __device__ __forceinline__ void m1_copy16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
@@ -267,13 +267,15 @@ __global__ void __launch_bounds__(128) mamba1_scan16_kernel(const __nv_bfloat16*
 
 // One thread a (row, channel, state index): the row's state through its chunks in order. ws_state[chunk] holds the chunk's own
 // state on entry (all but a row's last chunk) and the state the chunk starts from on exit. The slot is read, not written: the
-// second walk of the row's last chunk leaves the row's final state there.
+// second walk of the row's last chunk leaves the row's final state there. What bounds it is the latency of its loads, which do not
+// depend on S: eight chunks' own states and step sums are asked for before the first is used (a chunk at a time every load waited for
+// the store before it, whose place the compiler cannot tell
+// apart): rows of 2,048 and 300 tokens, 2,048 channels, the layer 204.7 us before and 187.5 so, the same bits.
 template <typename T>
-__global__ void mamba1_carry_kernel(float* state, int64_t state_stride, float* __restrict__ ws_state, const float* __restrict__ ws_dt,
-                                    const float* __restrict__ a_neg, const int32_t* __restrict__ q_indptr, const int32_t* __restrict__ slots,
-                                    int inner, int N) {
+__global__ void mamba1_carry_kernel(const float* state, int64_t state_stride, float* ws_state, const float* ws_dt, const float* __restrict__ a_neg,
+                                    const int32_t* __restrict__ q_indptr, const int32_t* __restrict__ slots, int inner, int N) {
+  constexpr int kAhead = 8;
   pdl_launch_dependents();
-  pdl_wait();
   const int r = blockIdx.x;
   const int idx = blockIdx.y * blockDim.x + threadIdx.x;
   if (idx >= inner * N) return;
@@ -281,15 +283,25 @@ __global__ void mamba1_carry_kernel(float* state, int64_t state_stride, float* _
   int first = 0;
   for (int rr = 0; rr < r; ++rr) first += (q_indptr[rr + 1] - q_indptr[rr] + kM1ChunkTokens - 1) / kM1ChunkTokens;
   const int chunks = (q_indptr[r + 1] - q_indptr[r] + kM1ChunkTokens - 1) / kM1ChunkTokens;
-  if (chunks == 0) return;
   const float a = a_neg[idx];
-  float S = state[(size_t)slots[r] * state_stride + idx];
-#pragma unroll 4      // the chunks' own states and step sums do not depend on S: several loads in flight
-  for (int k = 0; k < chunks; ++k) {
-    float* w = ws_state + ((size_t)(first + k) * inner) * N + idx;
-    const float own = k < chunks - 1 ? *w : 0.f;
-    *w = S;                                                                  // what chunk k starts from
-    if (k < chunks - 1) S = fmaf(decay_exp<T>(a * ws_dt[(size_t)(first + k) * inner + c]), S, own);
+  const float* slot = state + (size_t)slots[r] * state_stride + idx;
+  pdl_wait();
+  if (chunks == 0) return;
+  float S = *slot;
+  for (int k0 = 0; k0 < chunks; k0 += kAhead) {
+    float own[kAhead], fade[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j)
+      if (k0 + j < chunks - 1) {
+        own[j] = ws_state[(size_t)(first + k0 + j) * inner * N + idx];
+        fade[j] = ws_dt[(size_t)(first + k0 + j) * inner + c];
+      }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j)
+      if (k0 + j < chunks) {
+        ws_state[(size_t)(first + k0 + j) * inner * N + idx] = S;              // what chunk k0 + j starts from
+        if (k0 + j < chunks - 1) S = fmaf(decay_exp<T>(a * fade[j]), S, own[j]);
+      }
   }
 }
 

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(const P* pool, P* ou
   const int r = blockIdx.y;
   const long long at = (long long)blockIdx.x * 256 + threadIdx.x;
   const int j = (int)(at / pieces), i = (int)(at % pieces);
-  if (j >= stride) return;
+  if (j >= stride) { pdl_wait(); return; }
   const int page = j < kv_lens[r] ? kv_indices[kv_indptr[r] + j / page_size] : -1;
   pdl_wait();
   P v = {};
@@ -74,13 +74,13 @@ __global__ void __launch_bounds__(128) carried_attention_kernel(const __nv_bfloa
   __nv_bfloat16* Vb = Kb + 2 * kCaTile * ldq;                        // two buffers of [64][vdim + 8]
   pdl_launch_dependents();
   int r, tile;
-  if (!ca_tile_of_block(q_indptr, rows, (int)gridDim.x - 1 - (int)blockIdx.x, r, tile)) return;
+  if (!ca_tile_of_block(q_indptr, rows, (int)gridDim.x - 1 - (int)blockIdx.x, r, tile)) { pdl_wait(); return; }
   const int h = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t0 = q_indptr[r] + tile * kCaTile;
   const int n_valid = min(kCaTile, q_indptr[r + 1] - t0);
   const int p0 = positions[t0];
-  if (p0 < 0) return;                                          // a padding row
+  if (p0 < 0) { pdl_wait(); return; }                                          // a padding row
   const int p_last = p0 + n_valid - 1;
   const __nv_bfloat16* krow = keys + ((size_t)r * stride) * heads * dim + (size_t)h * dim;
   const __nv_bfloat16* vrow = values + ((size_t)r * stride) * heads * vdim + (size_t)h * vdim;

@@ -18,6 +18,8 @@ void set_error(const std::string& msg);
 // weights, which no kernel writes) overlaps that kernel's tail; pdl_wait() returns once the earlier kernel has finished
 // and its writes are visible. pdl_launch_dependents() lets the next kernel start its own preamble. Both are no-ops for a
 // kernel launched without the attribute. The switch is process-wide (roost_set_pdl).
+// A block that has nothing to do waits all the same before it returns: a grid none of whose blocks waited may be over before the
+// kernels ahead of it are, and the wait of the kernel behind it, which covers that grid alone, would order nothing.
 extern bool g_pdl_enabled;
 
 // `cluster_x` > 1 launches the grid as thread-block clusters of that many CTAs along x (the grid's x is a multiple of it).

@@ -120,8 +120,8 @@ __global__ void __launch_bounds__(32 * W) gla_tile_kernel(const T* u, int64_t ld
   int r = blockIdx.x, k = 0, chunks_of_row = 1;
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dg = lane & 3, cg = lane >> 2;
-  if (MODE != 0 && !gla_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) return;
-  if (MODE == 1 && k == chunks_of_row - 1) return;       // nobody starts from the state a row's last chunk ends with
+  if (MODE != 0 && !gla_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) { pdl_wait(); return; }
+  if (MODE == 1 && k == chunks_of_row - 1) { pdl_wait(); return; }       // nobody starts from the state a row's last chunk ends with
   int start = q_indptr[r], end = q_indptr[r + 1];
   if (MODE != 0) {
     start += k * kGlaChunkTokens;
@@ -280,8 +280,8 @@ __global__ void __launch_bounds__(32) gla_scan_kernel(const T* u, int64_t ld, fl
   const int lane = threadIdx.x;
   const int col = slice * 32 + lane;
   const bool live = col < vdim;
-  if (MODE != 0 && !gla_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) return;
-  if (MODE == 1 && k == chunks_of_row - 1) return;       // nobody starts from the state a row's last chunk ends with
+  if (MODE != 0 && !gla_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) { pdl_wait(); return; }
+  if (MODE == 1 && k == chunks_of_row - 1) { pdl_wait(); return; }       // nobody starts from the state a row's last chunk ends with
   int start = q_indptr[r], end = q_indptr[r + 1];
   if (MODE != 0) {
     start += k * kGlaChunkTokens;

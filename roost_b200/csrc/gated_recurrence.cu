@@ -46,9 +46,9 @@ __global__ void __launch_bounds__(128) gated_recurrence_scan_kernel(const T* __r
   pdl_launch_dependents();
   int r = blockIdx.x, k = 0, chunks_of_row = 1;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
-  if (c >= width) return;
-  if (MODE != 0 && !recurrence_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) return;
-  if (MODE == 1 && k == chunks_of_row - 1) return;       // nobody starts from the state a row's last chunk ends with
+  if (c >= width) { pdl_wait(); return; }
+  if (MODE != 0 && !recurrence_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) { pdl_wait(); return; }
+  if (MODE == 1 && k == chunks_of_row - 1) { pdl_wait(); return; }       // nobody starts from the state a row's last chunk ends with
   const int b = c / block_width, j = c % block_width;
   const float bias_r = gate_bias[(size_t)b * 2 * block_width + j], bias_i = gate_bias[(size_t)b * 2 * block_width + block_width + j];
   const float rate = decay[c];

@@ -46,9 +46,9 @@ __global__ void __launch_bounds__(256, 2) gla_chunks_kernel(const __nv_bfloat16*
       if (k < count) break;
       k -= count;
     }
-    if (r == rows) return;
+    if (r == rows) { pdl_wait(); return; }
     last = k == count - 1;
-    if (MODE == 1 && last) return;
+    if (MODE == 1 && last) { pdl_wait(); return; }
     start = q_indptr[r] + k * segment;
     end = min(start + segment, q_indptr[r + 1]);
   }

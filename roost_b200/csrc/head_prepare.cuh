@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(128) head_prepare_kernel(T* qkv, T* q_out, T* 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane % LPH;
   const int t = blockIdx.x * (4 / WPT) + warp / WPT, share = warp % WPT;
-  if (t >= a.tokens) return;                                       // no barrier of the block below
+  if (t >= a.tokens) { pdl_wait(); return; }                                       // no barrier of the block below
   const int pos = a.positions[t], slot = a.slot_mapping[t];
   const int half = a.rot_dims / 2;
   float* cs = angles[warp];

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(128 * RC) latent_attention_tc_kernel(
   }
   __syncthreads();
   const int b = item[0], r0 = item[1];
-  if (b < 0) return;
+  if (b < 0) { pdl_wait(); return; }
   const int tok0 = q_indptr[b];
   const int n_rows = (q_indptr[b + 1] - tok0) * heads;
   const int32_t* pages = kv_indices + kv_indptr[b];

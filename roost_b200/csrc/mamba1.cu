@@ -72,8 +72,8 @@ __global__ void __launch_bounds__(kM1Threads) mamba1_scan_kernel(const T* __rest
   float* sy = sx + stage_tokens * CPB;           // [chunk][CPB]
   pdl_launch_dependents();
   int r = blockIdx.x, k = 0, chunks_of_row = 1;
-  if (MODE != 0 && !chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) return;
-  if (MODE == 1 && k == chunks_of_row - 1) return;       // nobody starts from the state a row's last chunk ends with
+  if (MODE != 0 && !chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) { pdl_wait(); return; }
+  if (MODE == 1 && k == chunks_of_row - 1) { pdl_wait(); return; }       // nobody starts from the state a row's last chunk ends with
   const int c0 = blockIdx.y * CPB;
   const int cl = threadIdx.x / L, j = threadIdx.x % L;
   const int c = c0 + cl;
@@ -178,8 +178,8 @@ __global__ void __launch_bounds__(128) mamba1_scan16_kernel(const __nv_bfloat16*
   __shared__ __align__(16) float bc[kM16Tokens][32];       // B, then C
   pdl_launch_dependents();
   int r, k, chunks_of_row;
-  if (!chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) return;
-  if (MODE == 1 && k == chunks_of_row - 1) return;
+  if (!chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) { pdl_wait(); return; }
+  if (MODE == 1 && k == chunks_of_row - 1) { pdl_wait(); return; }
   const int tid = threadIdx.x, cl = tid >> 1, j = tid & 1, c0 = blockIdx.y * kM16Channels, c = c0 + cl, n0 = j * 8;
   const int start = q_indptr[r] + k * kM1ChunkTokens, end = min(start + kM1ChunkTokens, q_indptr[r + 1]);
   float a[8], S[8];
@@ -278,7 +278,7 @@ __global__ void mamba1_carry_kernel(const float* state, int64_t state_stride, fl
   pdl_launch_dependents();
   const int r = blockIdx.x;
   const int idx = blockIdx.y * blockDim.x + threadIdx.x;
-  if (idx >= inner * N) return;
+  if (idx >= inner * N) { pdl_wait(); return; }
   const int c = idx / N;
   int first = 0;
   for (int rr = 0; rr < r; ++rr) first += (q_indptr[rr + 1] - q_indptr[rr] + kM1ChunkTokens - 1) / kM1ChunkTokens;

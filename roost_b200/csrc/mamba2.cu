@@ -26,7 +26,7 @@ __global__ void mamba2_conv_kernel(const T* __restrict__ u, int64_t ld, int col,
   pdl_launch_dependents();
   const int t = blockIdx.x;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
-  if (c >= channels) return;
+  if (c >= channels) { pdl_wait(); return; }
   const int r = token_row[t];
   const int start = q_indptr[r];
   const float* st = state + (size_t)slots[r] * state_stride + conv_off;
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(128) mamba2_conv_vec_kernel(const T* u, int64_
   constexpr int V = Vec<T>::N;
   pdl_launch_dependents();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
-  if (c >= channels) return;
+  if (c >= channels) { pdl_wait(); return; }
   const int t0 = blockIdx.x * TT;
   float4 wt[V];
   float b[V], x[3][V];       // the inputs of tokens t - 3, t - 2, t - 1
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(64) mamba2_scan_vec_kernel(const T* __restrict
     }
     __syncthreads();
     r = item[0];
-    if (r < 0) return;
+    if (r < 0) { pdl_wait(); return; }
     start = q_indptr[r] + item[1] * kScanChunkTokens;
     end = min(start + kScanChunkTokens, q_indptr[r + 1]);
   }

@@ -64,9 +64,9 @@ __global__ void __launch_bounds__(256, 2) mamba2_chunks_kernel(const __nv_bfloat
       if (k < count) break;
       k -= count;
     }
-    if (r == rows) return;
+    if (r == rows) { pdl_wait(); return; }
     last = k == count - 1;
-    if (MODE == 1 && last) return;       // nobody starts from the state a row's last segment ends with
+    if (MODE == 1 && last) { pdl_wait(); return; }       // nobody starts from the state a row's last segment ends with
     start = q_indptr[r] + k * segment;
     end = min(start + segment, q_indptr[r + 1]);
   }
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(256) mamba2_segment_carry_kernel(float* ws_sta
                                                                   int segment) {
   pdl_launch_dependents();
   const int r = blockIdx.x, h = blockIdx.y, e = (blockIdx.z * 256 + threadIdx.x) * 4;
-  if (e >= per) return;
+  if (e >= per) { pdl_wait(); return; }
   int first = 0;
   for (int i = 0; i < r; ++i) first += (q_indptr[i + 1] - q_indptr[i] + segment - 1) / segment;
   const int count = (q_indptr[r + 1] - q_indptr[r] + segment - 1) / segment;

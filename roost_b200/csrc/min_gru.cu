@@ -42,9 +42,9 @@ __global__ void __launch_bounds__(128) min_gru_scan_kernel(const T* __restrict__
   pdl_launch_dependents();
   int r = blockIdx.x, k = 0, chunks_of_row = 1;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
-  if (c >= width) return;
-  if (MODE != 0 && !min_gru_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) return;
-  if (MODE == 1 && k == chunks_of_row - 1) return;       // nobody starts from the state a row's last chunk ends with
+  if (c >= width) { pdl_wait(); return; }
+  if (MODE != 0 && !min_gru_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) { pdl_wait(); return; }
+  if (MODE == 1 && k == chunks_of_row - 1) { pdl_wait(); return; }       // nobody starts from the state a row's last chunk ends with
   const float bz = z_bias[c], bx = x_bias[c];
   int start = q_indptr[r], end = q_indptr[r + 1];
   if (MODE != 0) {

@@ -92,8 +92,8 @@ __global__ void __launch_bounds__(32) retention_scan_kernel(const void* __restri
   const int lane = threadIdx.x;
   const int col = slice * 32 + lane;
   const bool live = col < vdim;
-  if (MODE != 0 && !retention_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) return;
-  if (MODE == 1 && k == chunks_of_row - 1) return;       // nobody starts from the state a row's last chunk ends with
+  if (MODE != 0 && !retention_chunk_of_block(q_indptr, rows, blockIdx.x, r, k, chunks_of_row)) { pdl_wait(); return; }
+  if (MODE == 1 && k == chunks_of_row - 1) { pdl_wait(); return; }       // nobody starts from the state a row's last chunk ends with
   int start = q_indptr[r], end = q_indptr[r + 1];
   if (MODE != 0) {
     start += k * kRtChunkTokens;

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kSgWarps * 32) sigmoid_attention_kernel(const 
   const bool active = hg < group;
   const int h = g * group + hg;
   const int pos = positions[t];
-  if (pos < 0) return;                                     // a padding token
+  if (pos < 0) { pdl_wait(); return; }                                     // a padding token
   const int r = token_row[t];
   const int32_t* pages = kv_indices + kv_indptr[r];
   const float slope = active ? slopes[h] : 0.f, bias = active ? head_bias[h] : 0.f;
@@ -371,15 +371,15 @@ __global__ void __launch_bounds__(128) sigmoid_attention_mma_kernel(const __nv_b
   pdl_launch_dependents();
   int r, tile;
   // the blocks with the most keys ahead of them (a row's last tiles) start first
-  if (!sigmoid_tile_of_block(q_indptr, rows, (int)gridDim.x - 1 - (int)blockIdx.x, r, tile)) return;
+  if (!sigmoid_tile_of_block(q_indptr, rows, (int)gridDim.x - 1 - (int)blockIdx.x, r, tile)) { pdl_wait(); return; }
   const int h = blockIdx.y, g = h / (heads / kv_heads);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t0 = q_indptr[r] + tile * kSmTile;
   const int n_valid = min(kSmTile, q_indptr[r + 1] - t0);
   const int p0 = positions[t0];
-  if (p0 < 0) return;                                          // a padding row
+  if (p0 < 0) { pdl_wait(); return; }                                          // a padding row
   const int p_last = p0 + n_valid - 1;
-  if ((int)blockIdx.z * tiles_a_chunk > p_last / kSmTile) return;      // the tile's keys end before this block's chunk
+  if ((int)blockIdx.z * tiles_a_chunk > p_last / kSmTile) { pdl_wait(); return; }      // the tile's keys end before this block's chunk
   const int32_t* pages = kv_indices + kv_indptr[r];
   const float slope = slopes[h], bias = head_bias[h];
   pdl_wait();

@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kSaWarps * 32) sink_attention_kernel(const T* 
   const bool active = hg < group;
   const int h = g * group + hg;
   const int pos = positions[t];
-  if (pos < 0) return;                                     // a padding token
+  if (pos < 0) { pdl_wait(); return; }                                     // a padding token
   const int r = token_row[t];
   const int32_t* pages = kv_indices + kv_indptr[r];
   pdl_wait();

@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kTaThreads) talking_attention_kernel(
   pdl_launch_dependents();
   const int t = blockIdx.x, z = blockIdx.z, tid = threadIdx.x;
   const int pos = positions[t];
-  if (pos < 0) return;                                                       // a padding token
+  if (pos < 0) { pdl_wait(); return; }                                                       // a padding token
   const int group = heads / kv_heads;
   const int32_t* pages = kv_indices + kv_indptr[token_row[t]];
   const int lo = window > 0 ? max(0, pos - window + 1) : 0;

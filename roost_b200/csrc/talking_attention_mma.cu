@@ -97,17 +97,17 @@ __global__ void __launch_bounds__(kTmThreads, 1) talking_attention_mma_kernel(
   pdl_launch_dependents();
   int r, tile;
   // the blocks with the most keys ahead of them (a row's last tiles) start first
-  if (!tm_tile_of_block(q_indptr, rows, (int)gridDim.x - 1 - (int)blockIdx.x, r, tile)) return;
+  if (!tm_tile_of_block(q_indptr, rows, (int)gridDim.x - 1 - (int)blockIdx.x, r, tile)) { pdl_wait(); return; }
   const int t0 = q_indptr[r] + tile * kTmQueries;
   const int n_valid = min(kTmQueries, q_indptr[r + 1] - t0);
   const int p0 = positions[t0];
-  if (p0 < 0) return;                                                        // a padding row
+  if (p0 < 0) { pdl_wait(); return; }                                                        // a padding row
   const int p_last = p0 + n_valid - 1;
   const int lo = window > 0 ? max(0, p0 - window + 1) : 0;                   // the first key any of the queries sees
   const int tile0 = lo / kTmKeys, all = p_last / kTmKeys - tile0 + 1;
   const int chunks = min((all + tiles_a_chunk - 1) / tiles_a_chunk, max_chunks);
   const int z = blockIdx.z;
-  if (z >= chunks) return;
+  if (z >= chunks) { pdl_wait(); return; }
   const int first = tile0 + z * tiles_a_chunk, last = z == chunks - 1 ? tile0 + all - 1 : first + tiles_a_chunk - 1;
   const int group = heads / kv_heads;
   const int h0 = blockIdx.y * 16 * OH, hn = min(16 * OH, heads - h0);

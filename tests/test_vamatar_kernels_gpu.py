@@ -348,22 +348,25 @@ def _recurrence_in_64_bits(xbc, dt, dt_bias, a_log, d, state, lengths, heads, N,
     return torch.stack(ys).reshape(at, -1), S
 
 
-@pytest.mark.parametrize("odd", [False, True])
-@pytest.mark.parametrize("N,groups,lengths", [(64, 1, [64, 65]), (128, 2, [1, 300, 17]), (128, 4, [63, 128]), (64, 2, [8, 9, 1, 200])])
-def test_recurrence_in_chunks_on_the_tensor_cores(kernels, N, groups, lengths, odd):
-    """Edges of chunks, rows of one token, carried states, decays from none to complete; against 64 bits, and no further from it than the
-    walk in 32 bits over the same numbers. A value that is not finite shows from its own token on and not before."""
-    H, T = 4, sum(lengths)
+@pytest.mark.parametrize("odd", [None, "late", "early"])
+@pytest.mark.parametrize("H,N,groups,lengths", [(4, 64, 1, [64, 65]), (4, 128, 2, [1, 300, 17]), (4, 128, 4, [63, 128]), (4, 64, 2, [8, 9, 1, 200]),
+                                                (4, 128, 1, [1300, 70]), (4, 64, 4, [2100]), (64, 128, 8, [1700, 1320])])
+def test_recurrence_in_chunks_on_the_tensor_cores(kernels, H, N, groups, lengths, odd):
+    """Edges of chunks, rows of one token, rows of six and nine segments (the carry takes four at a time), a step whose segments are longer than
+    the shortest, carried states, decays from none to complete; against 64 bits, and no further from it than the walk in 32 bits over the same
+    numbers. A value that is not finite, in a row's last segment or in its first, shows from its own token on and not before."""
+    T = sum(lengths)
     g = torch.Generator().manual_seed(N + len(lengths))
     xbc = torch.randn(T, H * 64 + 2 * groups * N, generator=g).to(torch.bfloat16)
     u = torch.zeros(T, 8 + H)
     u[:, 8:] = torch.randn(T, H, generator=g)
     u = u.to(torch.bfloat16)
     dt_bias, d = torch.randn(H, generator=g), torch.randn(H, generator=g)
-    a_log = torch.tensor([-3.0, -1.0, 1.0, 4.0])
+    a_log = torch.tensor([-3.0, -1.0, 1.0, 4.0]).repeat(H // 4)
     state = torch.randn(len(lengths), H * 64 * N, generator=g)
     if odd:
-        xbc[T - 6, 70], u[T - 6, 9] = float("inf"), float("inf")
+        t = T - 6 if odd == "late" else min(100, T - 6)
+        xbc[t, 70], u[t, 9] = float("inf"), float("inf")
     want, S = _recurrence_in_64_bits(xbc, u[:, 8:].float(), dt_bias, a_log, d, state.reshape(len(lengths), H, 64, N), lengths, H, N, groups)
     q_indptr = torch.tensor([0] + list(np.cumsum(lengths)), dtype=torch.int32).cuda()
     slots = torch.arange(len(lengths), dtype=torch.int32).cuda()
@@ -382,7 +385,7 @@ def test_recurrence_in_chunks_on_the_tensor_cores(kernels, N, groups, lengths, o
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("lengths,channels", [([1, 2, 3, 4, 37], 24), ([3000, 1, 2000], 1032)])
+@pytest.mark.parametrize("lengths,channels", [([1, 2, 3, 4, 37], 24), ([300, 1, 2, 3, 214], 1032), ([3000, 1, 2000], 1032)])
 def test_convolution_forms_agree_bit_for_bit(kernels, dtype, lengths, channels):
     """Sixteen tokens a thread, one, and a number at a time (columns that start off a whole piece): the same sums."""
     T = sum(lengths)

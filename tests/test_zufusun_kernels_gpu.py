@@ -261,19 +261,21 @@ def test_gated_linear_attention(kernels, dtype, heads, dim, vdim, rank, tau, for
         close(state[:, : QK * vdim].cpu(), S.reshape(8, -1), torch.float32, f"states after call {call}", f32=1e-4)
 
 
-@pytest.mark.parametrize("tau,odd", [(16.0, False), (16.0, True), (1.0, False), (0.02, False)])
-@pytest.mark.parametrize("lengths", [[1, 16, 17], [300, 31], [64, 1, 200, 8]])
-def test_gated_linear_attention_in_chunks_on_the_tensor_cores(kernels, lengths, tau, odd):
-    """Edges of chunks and segments, rows of one token, carried states, decays from hardly any to complete; against 64 bits, and no further from it
-    than the walk in 32 bits over the same numbers. A value that is not finite shows from its own token on and not before."""
-    heads, dim, vdim, rank, T = 3, 64, 128, 16, sum(lengths)
+@pytest.mark.parametrize("tau,odd", [(16.0, None), (16.0, "late"), (16.0, "early"), (1.0, None), (0.02, None)])
+@pytest.mark.parametrize("heads,lengths", [(3, [1, 16, 17]), (3, [300, 31]), (3, [64, 1, 200, 8]), (24, [1500, 1480])])
+def test_gated_linear_attention_in_chunks_on_the_tensor_cores(kernels, heads, lengths, tau, odd):
+    """Edges of chunks and segments, rows of one token, a step whose segments are longer than the shortest, carried states, decays from hardly any
+    to complete; against 64 bits, and no further from it than the walk in 32 bits over the same numbers. A value that is not finite, in a row's last
+    segment or in its first, shows from its own token on and not before."""
+    dim, vdim, rank, T = 64, 128, 16, sum(lengths)
     g = torch.Generator().manual_seed(T)
     width = heads * (2 * dim + vdim)
     u = torch.randn(T, width + rank, generator=g).to(torch.bfloat16)
     w = (torch.randn(heads * dim, rank, generator=g) * 0.5).to(torch.bfloat16)
     bias, state = torch.randn(heads * dim, generator=g), torch.randn(len(lengths), heads * dim * vdim, generator=g)
     if odd:
-        u[T - 5, 2 * heads * dim + 130], u[T - 3, 70] = float("inf"), float("nan")
+        t = T if odd == "late" else 12
+        u[t - 5, 2 * heads * dim + 130], u[t - 3, 70] = float("inf"), float("nan")
     x = u.double()
     q, k, v = x[:, : heads * dim].reshape(T, heads, dim) * dim ** -0.5, x[:, heads * dim : 2 * heads * dim].reshape(T, heads, dim), x[:, 2 * heads * dim : width].reshape(T, heads, vdim)
     fade = torch.sigmoid(x[:, width:] @ w.double().T + bias.double()).pow(1.0 / tau).reshape(T, heads, dim)

@@ -120,7 +120,7 @@ class LatentAttention(Mixer):
             self.head_gate.load(params["head_gate"])
         if self.carried:
             self.key_full.load(params["uk"])
-            self.value_full.load(params["uv"])
+            self.value_full.load(self.value_up.view(s.num_heads * s.v_dim, s.kv_rank))      # the same memory
         if s.learned_sink:
             self.sinks = params["sink"].float().contiguous()
         if s.q_rank:

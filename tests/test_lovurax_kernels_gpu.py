@@ -285,6 +285,17 @@ def test_carried_attention_on_tcgen05(kernels, heads, nope, rope, vdim, window, 
     assert off < 2.0 ** -8        # the output's rounding to bfloat16; the weights count to 16 bits
 
 
+def test_the_values_up_projection_is_kept_once(kernels):
+    """The latent space's form and the products that carry latents out read one tensor, also where the checkpoint's type is not the run's."""
+    from roost_b200.config.spec import LatentAttentionSpec
+    from roost_b200.parts import Runtime
+    from roost_b200.parts.base import MIXERS
+    spec = LatentAttentionSpec(hidden=64, num_heads=2, nope_dim=64, rope_dim=0, v_dim=64, kv_rank=128, scale=0.125, latent_eps=1e-6, position=None)
+    part = MIXERS.build(spec, Runtime(torch.bfloat16, "cuda", kernels))
+    part.load({k: torch.randn(d.shape, device="cuda") for k, d in MIXERS.get(spec.kind).parameters(spec).items()})
+    assert part.carried and part.value_full.weight.data_ptr() == part.value_up.data_ptr()
+
+
 def test_the_gather_of_cached_vectors_leaves_out_pages_that_were_given_back(kernels):
     for width in (24, 20):
         pool = torch.randn(6, 1, 4, width).to(torch.bfloat16).cuda()

@@ -162,10 +162,14 @@ class LatentAttention(Mixer):
                              tables.slot_mapping if s.own_latent else None, *sizes, **more)
             gate, gate_col = (self.gate(x), 0) if s.output_gate else (None, 0)
         # Under a window the latent space costs no more for keys that the window has passed, but carrying them out does: measured with a
-        # window of 1,024 the two cross at about 16 entries a token of the step.
+        # window of 1,024 the two cross at about 16 entries a token of the step. Without one the latent space takes as long as the longest row is
+        # (width 2,048: 242 us at 900 keys, 903 at 3,900), the carried form as long as there are entries (52 us at 1,024, 77 at 8,192, 115 at
+        # 16,384), which are made for the bound on the lengths, 1,024 at least: rows below the smallest bound may all be short (15 rows of 20
+        # tokens 56 and 112 us, 8 of 40 63 and 78; 4 of 40 no slower), so more than four of them have to bring 128 tokens each.
         entries = batch.num_rows * batch.kv_cap
+        rows_pay = batch.num_rows <= 4 or batch.kv_cap > 1024 or T >= 128 * batch.num_rows
         if (self.carried and not batch.all_single and T >= self.carried_min_tokens and 0 < entries <= self.carried_max_entries
-                and (s.window is None or entries <= 16 * T)):
+                and (rows_pay if s.window is None else entries <= 16 * T)):
             # a function of the step's sizes and kind only, so a captured step keeps its way
             latents = k.latent_gather(cache.k_pool, batch.kv_lens, tables.kv_indptr, tables.kv_indices, batch.num_rows, batch.kv_cap)
             if self.carried_tc:

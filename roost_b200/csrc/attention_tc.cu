@@ -32,8 +32,9 @@
 // 69 us, with the gather and the two products before it 98; 1,204 in the latent space on mma.sync). The work items follow from q_indptr, the last tiles of a row first.
 // Sigmoid weights (SIGMOID): a key's weight is the sigmoid of its score, less a slope a head times its distance, plus a bias a head; nothing divides
 // by the weights' sum, so there is no running maximum and the accumulator is never rescaled; the output is multiplied by the sigmoid of a gate
-// where there is one. The special-function unit bounds it (an exponential and a reciprocal a weight). Work items as for FLAT. Rows of 2,048 and
-// 777 tokens, 16 heads of 64 over 4: 67 us, 125 + 48 on mma.sync with a second kernel that adds the sums of a long row's chunks.
+// where there is one. Work items as for FLAT. A tile's chain bounds it (product, weights, product; an exponential and a reciprocal for each of 41 M
+// weights would be 18 us of special-function time). Rows of 2,048 and 777 tokens, 16 heads of 64 over 4: 67 us, 125 + 48 on mma.sync with a second kernel that adds
+// the sums of a long row's chunks.
 // Value rows at positions the request does not hold yet (the rest of its last page) or before the CTA's first visible key
 // are zeroed in shared memory before the second product, so that whatever the pool holds there cannot reach a result;
 // their scores are masked by position. Every wait is bounded (see tma.cuh): a wait given up raises the CTA's abort flag
@@ -78,12 +79,65 @@ struct TcFlat {
   int stride, rows, own_blocks, k_steps;
 };
 
-// What a SIGMOID launch has beside it: a slope and a bias a query head, the gate's rows (null: none), ld apart.
+// What a SIGMOID launch has beside it: a slope and a bias a query head, the gate's rows (null: none), ld apart; the key tiles of a chunk, how many
+// chunks a row of keys has at most (the last one takes what is left) and, with more than one, the chunks' sums [token][head][chunk][DV].
 struct TcSigmoid {
   const float *slopes, *bias;
   const __nv_bfloat16* gate;
   int64_t ld_gate;
+  int chunk_tiles, chunks;
+  float* sums;
 };
+
+// The pairs of a launch that has no work list, found from the rows' lengths: rows in order, of a row chunk after chunk, of a chunk the items that
+// see any of its keys, the last first, of an item the key/value heads. Pair `wi` as (batch row, first packed row, key/value head, chunk), row -1 beyond
+// the last pair, and its row as (first token, tokens, position of the first). By a whole warp, a lane a row: with the walk over all rows in every
+// thread the search grew with the square of a step's rows.
+struct TcPair {
+  int4 at;
+  int q_start, n, pos0;
+};
+__device__ __forceinline__ TcPair tc_find_pair(int wi, const int32_t* q_indptr, const int32_t* kv_lens, int rows, int group, int kv_heads, int item_rows, int chunk_keys,
+                                               int chunks) {
+  const int lane = threadIdx.x & 31, item_tokens = item_rows / group;
+  int item = wi / kv_heads;
+  auto items_of = [&](int n, int pos0, int z) {       // a row's items whose last token sees keys of chunk z: the last ones
+    const int tiles = (n + item_tokens - 1) / item_tokens, before = z * chunk_keys - pos0;
+    return before <= 0 ? tiles : (before >= n ? 0 : tiles - before / item_tokens);
+  };
+  for (int r0 = 0; r0 < rows; r0 += 32) {
+    const int r = r0 + lane;
+    int n = 0, pos0 = 0, mine = 0, start = 0;
+    if (r < rows) {
+      start = q_indptr[r];
+      n = q_indptr[r + 1] - start;
+      pos0 = kv_lens[r] - n;
+      if (pos0 >= 0)                                  // a padding row holds no keys
+        for (int z = 0; z < chunks; ++z) mine += items_of(n, pos0, z);
+    }
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int left = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += left;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, upto > item);
+    if (past == 0) {
+      item -= __shfl_sync(0xffffffffu, upto, 31);
+      continue;
+    }
+    const int src = __ffs(past) - 1;
+    item -= __shfl_sync(0xffffffffu, upto - mine, src);
+    n = __shfl_sync(0xffffffffu, n, src);
+    pos0 = __shfl_sync(0xffffffffu, pos0, src);
+    start = __shfl_sync(0xffffffffu, start, src);
+    int z = 0;
+    for (int count = items_of(n, pos0, 0); item >= count; count = items_of(n, pos0, ++z)) item -= count;
+    return {make_int4(r0 + src, ((n + item_tokens - 1) / item_tokens - 1 - item) * item_rows, wi % kv_heads, z), start, n, pos0};
+  }
+  return {make_int4(-1, 0, 0, 0), 0, 0, 0};
+}
+constexpr int kTcRounds = 32;      // pairs that a CTA of such a launch walks at most
 
 // 1 / (1 + 2^x)
 __device__ __forceinline__ float sigmoid_of_ex2(float x) {
@@ -94,7 +148,7 @@ __device__ __forceinline__ float sigmoid_of_ex2(float x) {
 
 // work[i] = (batch row, first packed row of the item's NG x 128 rows); an item is run once for every key/value head.
 // The grid is persistent: CTA c takes the (item, head) pairs c, c + gridDim.x, ... of the list, which the host has sorted
-// longest first. Tensor memory and the barriers are set up once; the rings of keys and values, the score columns and the
+// longest first (FLAT and SIGMOID: the pairs of tc_find_pair, in its order). Tensor memory and the barriers are set up once; the rings of keys and values, the score columns and the
 // barriers' phases run on from one pair to the next, so the copies of the next pair start while the last tiles of this
 // one are still being computed.
 template <int DK, int DV, int RPC, int NG, bool WIDE, bool FLAT, bool SIGMOID>
@@ -128,6 +182,8 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
   __shared__ __align__(8) uint64_t bars[2 + 2 * KS + 2 * VS + NG * kGroupBars];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
+  constexpr bool FOUND = FLAT || SIGMOID;
+  __shared__ TcPair found[FOUND ? kTcRounds : 1];
   const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
   const uint32_t q_full = bar0, q_empty = bar0 + 8u;
   auto k_full = [&](int s) { return bar0 + 8u * (2 + s); };
@@ -163,6 +219,19 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
+  const int group = q_heads / kv_heads;
+  const int total = items * kv_heads;
+  // The pairs are sorted longest first (a work list's). CTA c takes, in round r, pair r G + c when r is even and r G + (G - 1 - c) when it
+  // is odd: the CTA that got the longest pair of one round gets the shortest of the next, so every CTA walks about the
+  // same number of tiles. (The last round may leave a CTA without a pair while a later one of the same round has one:
+  // the walk then ends for it a round early, which costs it nothing.)
+  auto pair_of = [&](int round) { return round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x); };
+  if (FOUND) {      // the step's tables were there before its first kernel
+    for (int round = warp; round < kTcRounds && pair_of(round) < total; round += 2 + 4 * NG) {
+      const TcPair p = tc_find_pair(pair_of(round), q_indptr, kv_lens, flat.rows, group, kv_heads, NG * BM, sg.chunk_tiles * TK, sg.chunks);
+      if (lane == 0) found[round] = p;
+    }
+  }
   pdl_launch_dependents();
   pdl_wait();
   if (warp == 1) {
@@ -178,39 +247,30 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
   auto tmem_s = [&](int g, int sb) { return tmem_base + (uint32_t)g * kGroupCols + (uint32_t)sb * TK; };   // the scores; the weights go over them
   auto tmem_o = [&](int g) { return tmem_base + (uint32_t)g * kGroupCols + SB * TK; };
   volatile int* abortp = &abort_flag;
-  const int group = q_heads / kv_heads;
-  const int total = items * kv_heads;
-  // The pairs are sorted longest first. CTA c takes, in round r, pair r G + c when r is even and r G + (G - 1 - c) when it
-  // is odd: the CTA that got the longest pair of one round gets the shortest of the next, so every CTA walks about the
-  // same number of tiles. (The last round may leave a CTA without a pair while a later one of the same round has one:
-  // the walk then ends for it a round early, which costs it nothing.)
-  auto pair_of = [&](int round) { return round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x); };
-
   // What every thread derives of an (item, head) pair.
   struct Pair {
-    int b, row0, kvh, q_start, kv_len, pos0, rows_total;
+    int b, row0, kvh, z, q_start, kv_len, pos0, rows_total;
     int g_first[NG], g_last[NG];  // first and last key tile of each row group (last < first: none)
     int t0, ntiles, lo, hi;
   };
-  auto load_pair = [&](int wi, Pair& p) -> bool {
+  auto load_pair = [&](int round, int wi, Pair& p) -> bool {
     int n;
-    p.kvh = wi % kv_heads;
-    if (FLAT || SIGMOID) {
-      int item = wi / kv_heads, tiles = 0;
-      for (p.b = 0; p.b < flat.rows; ++p.b) {
-        p.q_start = q_indptr[p.b];
-        n = q_indptr[p.b + 1] - p.q_start;
-        p.kv_len = kv_lens[p.b];
-        tiles = p.kv_len >= n ? (n * group + NG * BM - 1) / (NG * BM) : 0;      // a padding row holds no keys
-        if (item < tiles) break;
-        item -= tiles;
-      }
-      if (p.b == flat.rows) return false;
-      p.row0 = (tiles - 1 - item) * NG * BM;
+    if (FOUND) {
+      const TcPair f = found[round];
+      p.b = f.at.x;
+      p.row0 = f.at.y;
+      p.kvh = f.at.z;
+      p.z = f.at.w;
+      p.q_start = f.q_start;
+      n = f.n;
+      p.kv_len = f.pos0 + n;
+      if (p.b < 0) return false;
     } else {
       const int2 w = work[wi / kv_heads];
       p.b = w.x;
       p.row0 = w.y;
+      p.kvh = wi % kv_heads;
+      p.z = 0;
       if (p.b < 0) return false;  // padding of a fixed-size work list
       p.q_start = q_indptr[p.b];
       n = q_indptr[p.b + 1] - p.q_start;
@@ -231,8 +291,16 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
         p.g_first[g] = 1;
         p.g_last[g] = 0;
       }
+      if (SIGMOID && sg.chunks > 1 && p.g_last[g] >= p.g_first[g]) {       // the chunk's tiles of them; of two groups the first may see none
+        p.g_first[g] = p.z * sg.chunk_tiles;
+        if (p.z < sg.chunks - 1) p.g_last[g] = min(p.g_last[g], p.g_first[g] + sg.chunk_tiles - 1);
+        if (p.g_last[g] < p.g_first[g]) {
+          p.g_first[g] = 1;
+          p.g_last[g] = 0;
+        }
+      }
     }
-    p.t0 = p.g_first[0];
+    p.t0 = SIGMOID ? p.z * sg.chunk_tiles : p.g_first[0];
     int t1 = p.g_last[0];
 #pragma unroll
     for (int g = 1; g < NG; ++g) {
@@ -252,7 +320,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
     bool ok = true;
     Pair p;
     for (int round = 0, wi = pair_of(0); wi < total && ok; wi = pair_of(++round)) {
-      if (!load_pair(wi, p)) continue;
+      if (!load_pair(round, wi, p)) continue;
       const int32_t* pages = FLAT ? nullptr : kv_indices + kv_indptr[p.b];
       const int p_first = (p.t0 * TK) >> page_shift, p_last = FLAT ? -1 : p.hi >> page_shift;
       const int fallback = FLAT ? 0 : pages[p_last];
@@ -327,7 +395,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
       bool ok = true;
       Pair p;
       for (int round = 0, wi = pair_of(0); wi < total && ok; wi = pair_of(++round)) {
-        if (!load_pair(wi, p)) continue;
+        if (!load_pair(round, wi, p)) continue;
         if (!(ok = mbar_wait_limited(q_full, (uint32_t)pairs & 1u, abortp, 2, &g_attention_tc_error))) break;
         ++pairs;
         tcgen05_fence_after();
@@ -412,7 +480,7 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
     bool ok = true;
     Pair p;
     for (int round = 0, wi = pair_of(0); wi < total && ok; wi = pair_of(++round)) {
-      if (!load_pair(wi, p)) continue;
+      if (!load_pair(round, wi, p)) continue;
       const int pr = p.row0 + g * BM + row;
       const bool valid = pr < p.rows_total;
       const int qpos = valid ? p.pos0 + pr / group : -1;
@@ -539,11 +607,21 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
         const float inv = SIGMOID ? 1.0f : (l > 0.f ? 1.0f / l : 0.f);
         const __nv_bfloat16* gate = SIGMOID && valid && sg.gate != nullptr ? sg.gate + (size_t)(p.q_start + pr / group) * sg.ld_gate + (size_t)head * DV : nullptr;
         __nv_bfloat16* dst = valid ? out + ((size_t)(p.q_start + pr / group) * q_heads + p.kvh * group + pr % group) * DV : nullptr;
+        // a row that sees keys of several chunks leaves this one's sums for the kernel that adds them; one that sees none of the chunk, nothing
+        float* sums = nullptr;
+        bool writes = valid;
+        if (SIGMOID && sg.chunks > 1 && valid) {
+          writes = qpos >= p.z * sg.chunk_tiles * TK;
+          if (qpos >= sg.chunk_tiles * TK) sums = sg.sums + (((size_t)(p.q_start + pr / group) * q_heads + head) * sg.chunks + p.z) * DV;
+        }
 #pragma unroll 1
         for (int c = 0; c < DV / 32; ++c) {
           uint32_t v[32];
           tcgen05_ld_32x32b_x32(tmem_o(g) + lane_addr + c * 32, v);
-          if (valid) {
+          if (SIGMOID && sums != nullptr && writes) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) *reinterpret_cast<uint4*>(sums + c * 32 + e) = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+          } else if (writes) {
 #pragma unroll
             for (int e = 0; e < 32; e += 8) {
               uint32_t o[4];
@@ -586,6 +664,31 @@ __global__ void __launch_bounds__(64 + NG * 128, 1)
   }
 }
 
+// The sums of a token's chunks, added in their order, then the output gate and the one rounding: a block a token, a thread four numbers. A token that
+// sees one chunk has its output already.
+__global__ void __launch_bounds__(256) sigmoid_tc_merge_kernel(const float* sums, __nv_bfloat16* out, const __nv_bfloat16* gate, int64_t ld_gate,
+                                                              const int32_t* __restrict__ positions, int width, int dim, int chunk_keys, int chunks) {
+  pdl_launch_dependents();
+  const int t = blockIdx.x, own = min(positions[t] / chunk_keys + 1, chunks);
+  pdl_wait();
+  if (own <= 1) return;
+  for (int i = threadIdx.x * 4; i < width; i += 1024) {
+    const float* from = sums + ((size_t)t * (width / dim) + i / dim) * chunks * dim + i % dim;
+    float4 a = *reinterpret_cast<const float4*>(from);
+    for (int z = 1; z < own; ++z) {
+      const float4 b = *reinterpret_cast<const float4*>(from + (size_t)z * dim);
+      a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+    }
+    if (gate != nullptr) {
+      const uint2 g = *reinterpret_cast<const uint2*>(gate + (size_t)t * ld_gate + i);
+      a.x *= sigmoid_f(__uint_as_float(g.x << 16)); a.y *= sigmoid_f(__uint_as_float(g.x & 0xffff0000u));
+      a.z *= sigmoid_f(__uint_as_float(g.y << 16)); a.w *= sigmoid_f(__uint_as_float(g.y & 0xffff0000u));
+    }
+    __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+    *reinterpret_cast<uint2*>(out + (size_t)t * width + i) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ host side
 static bool g_prefill_tc = true;
 
@@ -620,8 +723,11 @@ static int launch_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   // each walking its share of the sorted list (measured at 1 x 2048 tokens of 32/8 heads: 50 against 72 us); with many
   // pairs an SM every pair is a CTA of its own and the hardware hands them out as SMs fall free, which balances a long
   // list better than the fixed walk (8 x 8192 tokens: 1017 against 885 TFLOP/s).
+  // Where keys are dealt in chunks most of the pairs that are counted here do not exist and those that do are of a length, so the walk goes on to
+  // kTcRounds pairs.
   const long long pairs = (long long)items * kv_heads;
-  const int grid = (int)(pairs <= 8LL * sms[dev] ? (pairs < sms[dev] ? pairs : sms[dev]) : pairs);
+  const int rounds = SIGMOID && sg.chunks > 1 ? kTcRounds : 8;
+  const int grid = (int)(pairs <= (long long)rounds * sms[dev] ? (pairs < sms[dev] ? pairs : sms[dev]) : pairs);
   launch_kernel(kernel, dim3(grid), dim3(64 + NG * 128), smem, s, mq, mk, mv, mq2, mk2, flat, sg, (__nv_bfloat16*)out, q_indptr, kv_lens, kv_indptr, kv_indices,
                 (const int2*)work, items, q_heads, kv_heads, page_size, scale * kLog2eTc, window, sinks);
   return check_launch("attention_prefill_tc");
@@ -765,11 +871,13 @@ extern "C" int roost_carried_attention_tc(const void* q, int64_t ld_q, void* out
   }
   if (rc != ROOST_OK) return rc;
   const TcFlat flat = {stride, rows, nope / 64, (nope + rope) / 16};
+  TcSigmoid whole = {};       // a row's keys in one chunk
+  whole.chunk_tiles = whole.chunks = 1;
   const int w = window | (sinks != nullptr ? ROOST_ATTENTION_SINK : 0);
   const int dk = nope + (rope ? 64 : 0);
 #define ROOST_TC_FLAT(KK, VV)                                                                                                                \
   if (dk == KK && vdim == VV)                                                                                                                \
-    return launch_tc<KK, VV, 128, 1, true, true>(mq, mk, mv, mq2, mk2, flat, TcSigmoid{}, out, q_indptr, kv_lens, nullptr, nullptr, nullptr, (int)items,  \
+    return launch_tc<KK, VV, 128, 1, true, true>(mq, mk, mv, mq2, mk2, flat, whole, out, q_indptr, kv_lens, nullptr, nullptr, nullptr, (int)items,  \
                                                  heads, heads, 1, scale, w, sinks, (cudaStream_t)stream);
   ROOST_TC_FLAT(64, 64)
   ROOST_TC_FLAT(64, 128)
@@ -789,11 +897,15 @@ extern "C" int roost_sigmoid_attention_tc_supported(int dim, int vdim, int heads
          (gate == nullptr || ((uintptr_t)gate % 16 == 0 && ld_gate % 8 == 0));
 }
 
-extern "C" int roost_sigmoid_attention_tc(const void* q, void* out, const void* k_pool, const void* v_pool, long long pool_pages, const void* gate, int64_t ld_gate,
-                                          const float* slopes, const float* head_bias, const int32_t* q_indptr, const int32_t* kv_lens, const int32_t* kv_indptr,
-                                          const int32_t* kv_indices, int tokens, int rows, int heads, int kv_heads, int dim, int page_size, float scale,
-                                          roost_stream_t stream) {
+// `chunk_tiles`: the key tiles of 128 that a block takes of a row's keys; `chunks`: how many such chunks a row has at most, the last one takes what is
+// left. With more than one: positions, and sums float[tokens * heads * chunks * dim], which a second kernel adds.
+extern "C" int roost_sigmoid_attention_tc_chunks(const void* q, void* out, const void* k_pool, const void* v_pool, long long pool_pages, const void* gate, int64_t ld_gate,
+                                                  const float* slopes, const float* head_bias, const int32_t* q_indptr, const int32_t* kv_lens, const int32_t* kv_indptr,
+                                                  const int32_t* kv_indices, int tokens, int rows, int heads, int kv_heads, int dim, int page_size, float scale,
+                                                  const int32_t* positions, float* sums, int chunk_tiles, int chunks, roost_stream_t stream) {
   ROOST_REQUIRE(tokens >= 0 && rows >= 0 && heads > 0 && kv_heads > 0 && page_size > 0 && heads % kv_heads == 0 && scale > 0.f, "sigmoid_attention_tc: sizes and the scale must be positive");
+  ROOST_REQUIRE(chunk_tiles >= 1 && chunks >= 1 && chunk_tiles <= (1 << 20) && (chunks == 1 || (sums != nullptr && positions != nullptr && (uintptr_t)sums % 16 == 0)),
+                "sigmoid_attention_tc: chunks of keys need a workspace for their sums");
   ROOST_REQUIRE(q && out && k_pool && v_pool && slopes && head_bias && q_indptr && kv_lens && kv_indptr && kv_indices, "sigmoid_attention_tc: a pointer is null");
   ROOST_REQUIRE(gate == nullptr || ld_gate >= (int64_t)heads * dim, "sigmoid_attention_tc: a gate's row is too narrow");
   if (!roost_sigmoid_attention_tc_supported(dim, dim, heads, kv_heads, page_size, pool_pages, k_pool, v_pool, q, out, gate, ld_gate))
@@ -805,15 +917,17 @@ extern "C" int roost_sigmoid_attention_tc(const void* q, void* out, const void* 
   const int group = heads / kv_heads;
   // two row groups a CTA where every processor gets a pair of them; with less work the smaller items spread over more processors
   const int groups = (long long)tokens * heads >= 2LL * 148 * kTcRows ? 2 : 1;
-  const long long items = (long long)tokens * group / (groups * kTcRows) + rows;
-  if (items * kv_heads >= (1LL << 30)) return fail(ROOST_ERR_UNSUPPORTED, "sigmoid_attention_tc: too many tokens or heads");
+  const long long items = ((long long)tokens * group / (groups * kTcRows) + rows) * chunks;
+  if (items * kv_heads >= (1LL << 30)) return fail(ROOST_ERR_UNSUPPORTED, "sigmoid_attention_tc: too many tokens, heads or chunks");
   const TcFlat flat = {0, rows, 0, 0};
-  const TcSigmoid sg = {slopes, head_bias, (const __nv_bfloat16*)gate, ld_gate};
+  const TcSigmoid sg = {slopes, head_bias, (const __nv_bfloat16*)gate, ld_gate, chunk_tiles, chunks, sums};
   const int box_rows = paged_box_rows(page_size);
+  int launched = ROOST_ERR_UNSUPPORTED;
 #define ROOST_TC_SIGMOID(DD, RR, GG)                                                                                                            \
   if (dim == DD && box_rows == RR && groups == GG)                                                                                             \
-    return launch_tc<DD, DD, RR, GG, true, false, true>(mq, mk, mv, mq, mk, flat, sg, out, q_indptr, kv_lens, kv_indptr, kv_indices, nullptr,  \
-                                                        (int)items, heads, kv_heads, page_size, scale, 0, nullptr, (cudaStream_t)stream);
+    launched = launch_tc<DD, DD, RR, GG, true, false, true>(mq, mk, mv, mq, mk, flat, sg, out, q_indptr, kv_lens, kv_indptr, kv_indices,       \
+                                                            nullptr, (int)items, heads, kv_heads, page_size, scale, 0, nullptr,                \
+                                                            (cudaStream_t)stream);
   ROOST_TC_SIGMOID(64, 16, 1)
   ROOST_TC_SIGMOID(64, 32, 1)
   ROOST_TC_SIGMOID(64, 16, 2)
@@ -823,7 +937,21 @@ extern "C" int roost_sigmoid_attention_tc(const void* q, void* out, const void* 
   ROOST_TC_SIGMOID(128, 16, 2)
   ROOST_TC_SIGMOID(128, 32, 2)
 #undef ROOST_TC_SIGMOID
-  return fail(ROOST_ERR_UNSUPPORTED, "sigmoid_attention_tc: no kernel for these sizes");
+  if (launched == ROOST_ERR_UNSUPPORTED) return fail(ROOST_ERR_UNSUPPORTED, "sigmoid_attention_tc: no kernel for these sizes");
+  if (launched == ROOST_OK && chunks > 1) {
+    launch_kernel(sigmoid_tc_merge_kernel, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, (const float*)sums, (__nv_bfloat16*)out, (const __nv_bfloat16*)gate, ld_gate,
+                  positions, heads * dim, dim, chunk_tiles * kTcKeys, chunks);
+    return check_launch("sigmoid_attention_tc");
+  }
+  return launched;
+}
+
+extern "C" int roost_sigmoid_attention_tc(const void* q, void* out, const void* k_pool, const void* v_pool, long long pool_pages, const void* gate, int64_t ld_gate,
+                                          const float* slopes, const float* head_bias, const int32_t* q_indptr, const int32_t* kv_lens, const int32_t* kv_indptr,
+                                          const int32_t* kv_indices, int tokens, int rows, int heads, int kv_heads, int dim, int page_size, float scale,
+                                          roost_stream_t stream) {
+  return roost_sigmoid_attention_tc_chunks(q, out, k_pool, v_pool, pool_pages, gate, ld_gate, slopes, head_bias, q_indptr, kv_lens, kv_indptr, kv_indices, tokens,
+                                           rows, heads, kv_heads, dim, page_size, scale, nullptr, nullptr, 1, 1, stream);
 }
 
 ROOST_TRACE_TU(attention_tc)

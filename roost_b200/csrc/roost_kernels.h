@@ -560,6 +560,12 @@ int roost_sigmoid_attention_tc(const void* q, void* out, const void* k_pool, con
                                const float* slopes, const float* head_bias, const int32_t* q_indptr, const int32_t* kv_lens, const int32_t* kv_indptr,
                                const int32_t* kv_indices, int tokens, int rows, int heads, int kv_heads, int dim, int page_size, float scale,
                                roost_stream_t stream);
+/* The same with a row's keys in chunks of `chunk_tiles` tiles of 128, `chunks` at most (the last one takes what is left), a block a chunk: sums
+ * float[tokens * heads * chunks * dim] and positions with more than one (two launches). */
+int roost_sigmoid_attention_tc_chunks(const void* q, void* out, const void* k_pool, const void* v_pool, long long pool_pages, const void* gate, int64_t ld_gate,
+                                      const float* slopes, const float* head_bias, const int32_t* q_indptr, const int32_t* kv_lens, const int32_t* kv_indptr,
+                                      const int32_t* kv_indices, int tokens, int rows, int heads, int kv_heads, int dim, int page_size, float scale,
+                                      const int32_t* positions, float* sums, int chunk_tiles, int chunks, roost_stream_t stream);
 int roost_sigmoid_attention_mma_supported(int dim, int vdim, int entry);
 int roost_sigmoid_attention_mma(const void* q, void* out, const void* k_base, const void* v_base, int entry, const void* gate, int64_t ld_gate,
                                 const float* slopes, const float* head_bias, const int32_t* positions, const int32_t* q_indptr,

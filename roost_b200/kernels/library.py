@@ -186,8 +186,8 @@ _SIGNATURES = {
     "roost_sigmoid_attention": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p],
     "roost_sigmoid_attention_tc_supported": [c_int, c_int, c_int, c_int, c_int, ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64],
-    "roost_sigmoid_attention_tc": [c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_longlong, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p],
+    "roost_sigmoid_attention_tc_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_longlong, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
+                                          c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "roost_sigmoid_attention_mma_supported": [c_int, c_int, c_int],
     "roost_sigmoid_attention_mma": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_int, c_void_p],
@@ -1468,6 +1468,7 @@ class KernelLibrary:
 
     SIGMOID_MMA_MIN_TOKENS = 32     # tokens from which a bfloat16 step that brings prompt portions runs the tensor-core form
     SIGMOID_MMA_CHUNK_TILES = 8     # tiles of 64 keys a block of the tensor-core form takes of a long row
+    SIGMOID_TC_CHUNK_TILES = 16     # tiles of 128 keys a block of the tcgen05 form takes of a long row
 
     def sigmoid_attention_mma_supported(self, dim: int, vdim: int, two_planes: bool) -> bool:
         return bool(self._lib.roost_sigmoid_attention_mma_supported(int(dim), int(vdim), int(dim if two_planes else dim + vdim)))
@@ -1499,8 +1500,14 @@ class KernelLibrary:
             rows = q_indptr.numel() - 1
             if kv_lens.numel() < rows:
                 raise KernelError("sigmoid_attention: one length a row")
-            self._call("roost_sigmoid_attention_tc", _ptr(q), _ptr(out), kb, vb, k_pool.shape[0], gate_ptr, ld_gate, _ptr(slopes), _ptr(head_bias),
-                       _ptr(q_indptr), _ptr(kv_lens), _ptr(kv_indptr), _ptr(kv_indices), T, rows, heads, kv_heads, dim, k_pool.shape[2], float(scale), _stream())
+            # keys in chunks at fixed positions, so that a long row's do not wait in one block for one another; the bound on the requests' lengths
+            # says how many there can be (every replay of a captured step agrees)
+            per = self.SIGMOID_TC_CHUNK_TILES
+            chunks = -(-kv_cap // (128 * per)) if kv_cap else 1
+            sums = torch.empty((T * heads * chunks * dim,), dtype=torch.float32, device=q.device) if chunks > 1 else None
+            self._call("roost_sigmoid_attention_tc_chunks", _ptr(q), _ptr(out), kb, vb, k_pool.shape[0], gate_ptr, ld_gate, _ptr(slopes), _ptr(head_bias),
+                       _ptr(q_indptr), _ptr(kv_lens), _ptr(kv_indptr), _ptr(kv_indices), T, rows, heads, kv_heads, dim, k_pool.shape[2], float(scale),
+                       _ptr(positions), _ptr(sums), per, chunks, _stream(), launches=2 if chunks > 1 else 1)
             return out
         if q_indptr is not None and q.dtype == torch.bfloat16 and self.sigmoid_attention_mma_supported(dim, vdim, v_pool is not None):
             _need(q_indptr, "q_indptr", torch.int32)

@@ -346,3 +346,87 @@ def test_sigmoid_weights_on_tcgen05(kernels, heads, kv_heads, dim, page, gated):
         off[form] = float((got[:T].double().cpu() - want).norm() / want.norm())
     print(f"MEASURED sigmoid weights: {off}")
     assert off["tcgen05"] < 1.1 * off["mma.sync"] and off["tcgen05"] < 2.0 ** -8       # the output's rounding to bfloat16
+
+
+def _sigmoid_step(lens, counts, heads, kv_heads, dim, page, g):
+    """(pools, tables) of a step whose row r brings its last ``counts[r]`` tokens of ``lens[r]``, a padding row of three tokens behind them; what a pool
+    holds beyond a row's keys is NaN."""
+    need = [-(-n // page) for n in lens]
+    order = torch.randperm(sum(need) + 3, generator=g)[: sum(need)]
+    pool = torch.full((2, sum(need) + 3, kv_heads, page, dim), float("nan"), dtype=torch.bfloat16)
+    kv, at = [torch.randn(2, n, kv_heads, dim, generator=g).to(torch.bfloat16) for n in lens], 0
+    for x, n in zip(kv, need):
+        for p in range(n):
+            part = x[:, p * page : (p + 1) * page].transpose(1, 2)
+            pool[:, order[at + p], :, : part.shape[2]] = part
+        at += n
+    indptr = [0] + torch.tensor(need).cumsum(0).tolist()
+    positions = torch.cat([torch.arange(n - m, n) for n, m in zip(lens, counts)] + [torch.full((3,), -1)]).to(torch.int32)
+    token_row = torch.tensor([r for r, m in enumerate(counts) for _ in range(m)] + [len(lens)] * 3, dtype=torch.int32)
+    tables = dict(positions=positions.cuda(), token_row=token_row.cuda(), kv_indptr=i32(indptr + indptr[-1:]), kv_indices=i32(order.tolist()),
+                  q_indptr=i32([0] + torch.tensor(counts + [3]).cumsum(0).tolist()), kv_lens=i32(lens + [0]))
+    return kv, pool.cuda(), tables
+
+
+@pytest.mark.parametrize("per,kv_cap", [(1, 1024), (1, 512), (2, 1024), (3, 4096)])
+@pytest.mark.parametrize("heads,kv_heads,dim,counts", [(4, 2, 64, [129, 387, 1, 1, 2]), (32, 4, 128, [700, 387, 1, 128, 2])])
+def test_sigmoid_weights_over_keys_in_chunks(kernels, monkeypatch, heads, kv_heads, dim, counts, per, kv_cap):
+    """Chunks of one, two and three key tiles, rows that end beside a chunk's edge, a bound on the lengths that a row exceeds (the last chunk takes what is
+    left), one and two row groups a CTA, more rows than a warp has lanes: against 64 bits, and where a token sees one chunk the same bits as without."""
+    g = torch.Generator().manual_seed(heads + per)
+    lens = [700 if counts[0] == 700 else 129, 640, 257, 128, 386] + [200 + 7 * i for i in range(33)]
+    counts = counts + [1] * 33
+    kv, pool, tables = _sigmoid_step(lens, counts, heads, kv_heads, dim, 16, g)
+    T, group, scale = sum(counts), heads // kv_heads, 1.5 / math.sqrt(dim)
+    q = torch.randn(T + 3, heads, dim, generator=g).to(torch.bfloat16)
+    rows = torch.randn(T + 3, heads * dim + 16, generator=g).to(torch.bfloat16)
+    slopes, bias = torch.tensor(P.head_slopes(heads), dtype=torch.float32), torch.randn(heads, generator=g) - 1.0
+    want, t = torch.zeros(T, heads, dim, dtype=torch.float64), 0
+    for (k, v), n, m in zip(kv, lens, counts):
+        i, j = torch.arange(n - m, n, dtype=torch.float64)[:, None], torch.arange(n, dtype=torch.float64)[None]
+        for h in range(heads):
+            s = q[t : t + m, h].double() @ k[:, h // group].double().T * scale - float(slopes[h]) * (i - j) + float(bias[h])
+            want[t : t + m, h] = (P.sigmoid(s) * (j <= i)) @ v[:, h // group].double()
+        t += m
+    want = want.reshape(T, -1) * P.sigmoid(rows[:T, 16:].double())
+    monkeypatch.setattr(kernels, "SIGMOID_TC_CHUNK_TILES", per, raising=False)
+    run = lambda cap: kernels.sigmoid_attention(q.cuda(), pool[0], pool[1], rows.cuda(), 16, slopes.cuda(), bias.cuda(), tables["positions"], tables["token_row"],   # noqa: E731
+                                                tables["kv_indptr"], tables["kv_indices"], kv_heads, dim, scale, kv_cap=cap, q_indptr=tables["q_indptr"],
+                                                kv_lens=tables["kv_lens"])[:T].cpu()
+    got, whole = run(kv_cap), run(0)
+    off = {n: float((x.double() - want).norm() / want.norm()) for n, x in (("chunks", got), ("whole", whole))}
+    print(f"MEASURED sigmoid weights in chunks of {per}: {off}")
+    assert off["chunks"] < 1.1 * off["whole"] and off["chunks"] < 2.0 ** -8       # the output's rounding to bfloat16
+    early = tables["positions"][:T].cpu() < 128 * per
+    assert torch.equal(got[early], whole[early]) and early.any() and not early.all()
+
+
+@pytest.mark.parametrize("counts,lens", [([64], [16000]), ([1, 1, 1, 480], [16000, 16000, 16000, 480])])
+def test_a_long_row_of_keys_does_not_wait_in_one_block(kernels, counts, lens):
+    """A short portion, or decode rows beside a prompt, at 16,000 keys: 85 and 163 us on mma.sync, whose blocks take 512 keys each; 233 and 359 with all of a
+    row's keys in one block of the tcgen05 form."""
+    heads, kv_heads, dim = 16, 4, 64
+    kv, pool, tables = _sigmoid_step(lens, counts, heads, kv_heads, dim, 16, torch.Generator().manual_seed(1))
+    T = sum(counts) + 3
+    q = torch.randn(T, heads, dim).to(torch.bfloat16).cuda()
+    slopes, bias = torch.tensor(P.head_slopes(heads), dtype=torch.float32).cuda(), torch.zeros(heads).cuda()
+
+    def us(**more):
+        call = lambda: kernels.sigmoid_attention(q, pool[0], pool[1], None, None, slopes, bias, tables["positions"], tables["token_row"], tables["kv_indptr"],   # noqa: E731
+                                                 tables["kv_indices"], kv_heads, dim, 0.125, kv_cap=16384, q_indptr=tables["q_indptr"], **more)
+        for _ in range(3):
+            call()
+        times = []
+        for _ in range(5):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(20):
+                call()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end) * 50.0)
+        return min(times)
+
+    mma, tc = us(), us(kv_lens=tables["kv_lens"])
+    print(f"MEASURED sigmoid weights at 16,000 keys, rows of {counts}: tcgen05 {tc:.0f} us, mma.sync {mma:.0f} us")
+    assert tc < 1.25 * mma

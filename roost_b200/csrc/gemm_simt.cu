@@ -4,7 +4,7 @@
 // row falls in. Definition: src/Starlings.Roost.Ops/CpuOps.cs:395-437 (TransposeB, Alpha 1, no bias).
 //
 // Two forms, bit for bit alike; the operands of both arrive by cp.async several stages of 32 k ahead, [row][k] as they lie in
-// memory, and are read four k (16 bytes) at a time:
+// memory (bfloat16 operands and rows that are no whole 16-byte pieces: through registers, a stage ahead), and are read four k (16 bytes) at a time:
 //   tiles: a thread makes TM x TN outputs of a block's BM x BN. Bound by issue slots and shared-memory reads together (78 %
 //     and 68 % busy, the FMA pipe 64 %, at 2,048 x 4,096 x 4,096): 45 TFLOP/s there, 22.5 with the form before (one buffer,
 //     scalar loads and reads); 512 x 6,144 x 1,024 170 us (337 before). Two outputs an instruction (fma.rn.f32x2) were
@@ -24,23 +24,37 @@ __device__ __forceinline__ void simt_copy16(float* smem, const float* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
 }
 
-// `ROWS` rows of one stage, [row][k], zeros beyond the matrix. ASYNC: whole 16-byte pieces of floats by cp.async; else an element at a time.
-template <typename T, int ROWS, int NT, bool ASYNC>
-__device__ __forceinline__ void simt_stage(float* dst, const T* p, int64_t ld, int row0, int rows, int k0, int K) {
-  if constexpr (ASYNC) {
+// `ROWS` rows of one stage, [row][k], zeros beyond the matrix, in whole 16-byte pieces of floats by cp.async.
+template <int ROWS, int NT>
+__device__ __forceinline__ void simt_stage(float* dst, const float* p, int64_t ld, int row0, int rows, int k0, int K) {
 #pragma unroll
-    for (int i = 0; i < (ROWS * (kSimtK / 4) + NT - 1) / NT; ++i) {
-      const int idx = threadIdx.x + i * NT, r = idx / (kSimtK / 4), kk = idx % (kSimtK / 4) * 4;
-      if (ROWS * (kSimtK / 4) % NT != 0 && r >= ROWS) break;
-      float* d = dst + r * kSimtLd + kk;
-      if (row0 + r < rows && k0 + kk < K) simt_copy16(d, (const float*)p + (int64_t)(row0 + r) * ld + k0 + kk);
-      else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  } else {
-    for (int idx = threadIdx.x; idx < ROWS * kSimtK; idx += NT) {
-      const int r = idx / kSimtK, kk = idx % kSimtK;
-      dst[r * kSimtLd + kk] = row0 + r < rows && k0 + kk < K ? to_float(p[(int64_t)(row0 + r) * ld + k0 + kk]) : 0.f;
-    }
+  for (int i = 0; i < (ROWS * (kSimtK / 4) + NT - 1) / NT; ++i) {
+    const int idx = threadIdx.x + i * NT, r = idx / (kSimtK / 4), kk = idx % (kSimtK / 4) * 4;
+    if (ROWS * (kSimtK / 4) % NT != 0 && r >= ROWS) break;
+    float* d = dst + r * kSimtLd + kk;
+    if (row0 + r < rows && k0 + kk < K) simt_copy16(d, p + (int64_t)(row0 + r) * ld + k0 + kk);
+    else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
+// The same an element at a time, through registers, so that a stage is on its way while the one before is multiplied.
+// (Elements beyond the matrix are read at its end and replaced by zeros: with a condition around a load of 16 bits every load waited for the one
+// before: 300 x 1,024 x 1,024 in bfloat16 106 us, 77 with the form before, whose tiles were 64 x 64.)
+template <typename T, int ROWS, int NT>
+__device__ __forceinline__ void simt_fetch(T (&held)[ROWS * kSimtK / NT], const T* p, int64_t ld, int row0, int rows, int k0, int K) {
+  static_assert(ROWS * kSimtK % NT == 0, "whole passes");
+#pragma unroll
+  for (int i = 0; i < ROWS * kSimtK / NT; ++i) {
+    const int idx = threadIdx.x + i * NT, r = min(row0 + idx / kSimtK, rows - 1), k = min(k0 + idx % kSimtK, K - 1);
+    held[i] = p[(int64_t)r * ld + k];
+  }
+}
+template <typename T, int ROWS, int NT>
+__device__ __forceinline__ void simt_put(float* dst, const T (&held)[ROWS * kSimtK / NT], int row0, int rows, int k0, int K) {
+#pragma unroll
+  for (int i = 0; i < ROWS * kSimtK / NT; ++i) {
+    const int idx = threadIdx.x + i * NT, r = idx / kSimtK, k = idx % kSimtK;
+    dst[r * kSimtLd + k] = row0 + r < rows && k0 + k < K ? to_float(held[i]) : 0.f;
   }
 }
 
@@ -63,22 +77,41 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
   auto issue = [&](int step) {
     if (step < steps) {
       const int buf = step % STAGES;
-      simt_stage<TIn, BM, NT, ASYNC>(ast + buf * BM * kSimtLd, a, lda, m0, M, step * kSimtK, K);
-      simt_stage<TIn, BN, NT, ASYNC>(wst + buf * BN * kSimtLd, w, ldw, n0, N, step * kSimtK, K);
+      simt_stage<BM, NT>(ast + buf * BM * kSimtLd, (const float*)a, lda, m0, M, step * kSimtK, K);
+      simt_stage<BN, NT>(wst + buf * BN * kSimtLd, (const float*)w, ldw, n0, N, step * kSimtK, K);
     }
     asm volatile("cp.async.commit_group;\n" ::);
+  };
+  TIn ra[ASYNC ? 1 : BM * kSimtK / NT], rw[ASYNC ? 1 : BN * kSimtK / NT];
+  auto fetch = [&](int step) {
+    if constexpr (!ASYNC) {
+      simt_fetch<TIn, BM, NT>(ra, a, lda, m0, M, step * kSimtK, K);
+      simt_fetch<TIn, BN, NT>(rw, w, ldw, n0, N, step * kSimtK, K);
+    }
+  };
+  auto put = [&](int step) {
+    if constexpr (!ASYNC) {
+      simt_put<TIn, BM, NT>(ast + step % STAGES * BM * kSimtLd, ra, m0, M, step * kSimtK, K);
+      simt_put<TIn, BN, NT>(wst + step % STAGES * BN * kSimtLd, rw, n0, N, step * kSimtK, K);
+    }
   };
   float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+  if constexpr (ASYNC) {
 #pragma unroll
-  for (int s = 0; s < STAGES - 1; ++s) issue(s);
+    for (int s = 0; s < STAGES - 1; ++s) issue(s);
+  } else {
+    fetch(0);
+    put(0);
+  }
   for (int step = 0; step < steps; ++step) {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+    if constexpr (ASYNC) asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
     __syncthreads();       // the stage has arrived for everyone, and the one before it has been read by everyone
-    issue(step + STAGES - 1);
+    if constexpr (ASYNC) issue(step + STAGES - 1);
+    else if (step + 1 < steps) fetch(step + 1);
     const float* as = ast + (step % STAGES) * BM * kSimtLd + ty * kSimtLd;      // a thread's rows and columns: every NY-th and every NX-th
     const float* ws = wst + (step % STAGES) * BN * kSimtLd + tx * kSimtLd;
     // the operands of the next four k are read while these are multiplied
@@ -111,6 +144,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(x[b][i].w, y[b][j].w, acc[i][j]);
     }
+    if (!ASYNC && step + 1 < steps) put(step + 1);       // its buffer was read two steps ago
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -242,7 +276,7 @@ static int launch_simt(const SimtArgs& g) {
                      (uintptr_t)g.a % 16 == 0 && (uintptr_t)g.w % 16 == 0;
   if constexpr (sizeof(TIn) == 4 && sizeof(TOut) == 4) {
     if (whole && g.m <= 8) {
-      // a block takes 128 or 256 columns where two of them a processor remain, else 32 or 64 (a tile's weights are then read by fewer
+      // a block takes 128 columns where two of them a processor remain, else 32 or 64 (a tile's weights are then read by fewer
       // threads, but by more processors: 3 x 1,024 x 3,072 39 us, 230 with 64 x 64 tiles)
       const bool wide = (long long)((g.n + 127) / 128) * g.batch >= 2 * 148;
       if (g.m <= 2) return wide ? launch_simt_few<1, 2, 1>(g) : launch_simt_few<2, 1, 1>(g);

@@ -372,11 +372,12 @@ __global__ void __launch_bounds__(128) paged_attention_rows_kernel(const T* q, T
 
 using namespace roost;
 
-extern "C" int roost_paged_attention_generic(const void* q, void* out, const void* k_pool, const void* v_pool,
+// `rows`: the requests that the step's tokens belong to (0: not known), which only chooses between the two forms.
+extern "C" int roost_paged_attention_generic_rows(const void* q, void* out, const void* k_pool, const void* v_pool,
                                              const int32_t* positions, const int32_t* token_row,
                                              const int32_t* kv_indptr, const int32_t* kv_indices, int tokens,
                                              int q_heads, int kv_heads, int head_dim, int page_size, float scale,
-                                             int window, int dtype, roost_stream_t stream) {
+                                             int window, int dtype, int rows, roost_stream_t stream) {
   ROOST_REQUIRE(tokens >= 0 && q_heads > 0 && kv_heads > 0 && head_dim > 0 && page_size > 0,
                 "paged_attention: sizes must be positive");
   ROOST_REQUIRE(q_heads % kv_heads == 0, "paged_attention: q_heads must be a multiple of kv_heads");
@@ -385,7 +386,13 @@ extern "C" int roost_paged_attention_generic(const void* q, void* out, const voi
   if (tokens == 0) return ROOST_OK;
   const int group = q_heads / kv_heads;
   const uintptr_t piece = dtype == ROOST_F32 ? 16 : 8;      // four numbers
-  if (head_dim % 4 == 0 && head_dim <= 128 && group <= kRows && ((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) % piece == 0) {
+  // Where a block of many rows is the slower one: a prompt of a few tokens, whose one or two tiles are over before the larger block has begun (17 and 33
+  // tokens, 16 heads of 128 over 8: 11.0 and 13.4 us, 7.4 and 12.5 in the other form; 15.8 and 15.4 at 64, 24 and 28 at 100), and steps that decode more tokens
+  // than two blocks a processor, which is what its shared memory leaves (64 and 96 rows of 300 keys: 109 and 173 us, 100 and 111; 32 rows of 1,000: 167, 284).
+  // A single token over fewer than thirty keys stays here although it is up to 2.5 us slower: the lengths are not known on the host.
+  const bool single = rows > 0 && rows >= tokens;
+  const bool many_rows = single ? (long long)tokens * kv_heads <= 2 * 148 : tokens > 64;
+  if (many_rows && head_dim % 4 == 0 && head_dim <= 128 && group <= kRows && ((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) % piece == 0) {
     const int span = kRows / group;
     dim3 tiles((tokens + span - 1) / span, kv_heads, min(span, tokens));
     const size_t bytes = ((size_t)4 * kTile * kRowsLd + (size_t)kRows * kRowsLd + (size_t)kRows * (kTile + 4) + kRows) * sizeof(float);
@@ -407,4 +414,11 @@ extern "C" int roost_paged_attention_generic(const void* q, void* out, const voi
                                                               head_dim, page_size, scale, window);
   });
   return check_launch("paged_attention_generic");
+}
+
+extern "C" int roost_paged_attention_generic(const void* q, void* out, const void* k_pool, const void* v_pool, const int32_t* positions, const int32_t* token_row,
+                                             const int32_t* kv_indptr, const int32_t* kv_indices, int tokens, int q_heads, int kv_heads, int head_dim, int page_size,
+                                             float scale, int window, int dtype, roost_stream_t stream) {
+  return roost_paged_attention_generic_rows(q, out, k_pool, v_pool, positions, token_row, kv_indptr, kv_indices, tokens, q_heads, kv_heads, head_dim, page_size, scale,
+                                            window, dtype, 0, stream);
 }

@@ -108,6 +108,10 @@ int roost_paged_attention_generic(const void* q, void* out, const void* k_pool, 
                                   const int32_t* positions, const int32_t* token_row, const int32_t* kv_indptr,
                                   const int32_t* kv_indices, int tokens, int q_heads, int kv_heads, int head_dim,
                                   int page_size, float scale, int window, int dtype, roost_stream_t stream);
+/* The same; rows: the requests that the tokens belong to (0: not known), which chooses between two forms of the same bits. */
+int roost_paged_attention_generic_rows(const void* q, void* out, const void* k_pool, const void* v_pool, const int32_t* positions, const int32_t* token_row,
+                                       const int32_t* kv_indptr, const int32_t* kv_indices, int tokens, int q_heads, int kv_heads, int head_dim, int page_size,
+                                       float scale, int window, int dtype, int rows, roost_stream_t stream);
 
 /* Tensor-core attention for bfloat16 (attention_mma.cu). head_dim must be one roost_attention_mma_supported accepts.
  * q_indptr[b] .. q_indptr[b+1] are row b's tokens, kv_lens[b] its keys after this step.

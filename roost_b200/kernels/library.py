@@ -77,8 +77,8 @@ _SIGNATURES = {
                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int64, c_int, c_int, c_int,
                                  c_void_p],
     "roost_rope_table": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p],
-    "roost_paged_attention_generic": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                                      c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
+    "roost_paged_attention_generic_rows": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                                           c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p],
     "roost_attention_mma_supported": [c_int],
     "roost_attention_prefill_tile_rows": [c_int, c_int, c_int, c_int, ctypes.c_longlong, c_void_p, c_void_p, ctypes.c_longlong],
     "roost_attention_set_prefill_tc": [c_int],
@@ -427,9 +427,9 @@ class KernelLibrary:
         if d2 != d:
             raise KernelError("paged_attention: head_dim of q and of the pool differ")
         out = torch.empty((T, nq * d), dtype=q.dtype, device=q.device)
-        self._call("roost_paged_attention_generic", _ptr(q), _ptr(out), _ptr(k_pool), _ptr(v_pool), _ptr(positions),
+        self._call("roost_paged_attention_generic_rows", _ptr(q), _ptr(out), _ptr(k_pool), _ptr(v_pool), _ptr(positions),
                    _ptr(token_row), _ptr(kv_indptr), _ptr(kv_indices), T, nq, nkv, d, page, scale,
-                   int(window) if window else 0, dtype_code(q.dtype), _stream())
+                   int(window) if window else 0, dtype_code(q.dtype), kv_indptr.numel() - 1, _stream())
         return out
 
     def attention_mma_supported(self, head_dim: int) -> bool:

@@ -315,6 +315,42 @@ def test_paged_attention_forms_agree_bit_for_bit(kernels, dtype, window, nq, nkv
     assert torch.isfinite(want).float().mean() > 0.5 and not torch.isfinite(want).all()
 
 
+@pytest.mark.parametrize("counts,lens", [([17], [17]), ([1] * 64, [300] * 64), ([1] * 8, [300] * 8), ([100], [100])])
+def test_the_form_of_many_rows_runs_where_it_is_no_slower(kernels, counts, lens):
+    """Ahead of the rule 17 tokens took 11 us instead of 7 and 64 rows of 300 keys 109 instead of 100. Queries off a whole piece of four numbers go to the
+    form for any sizes."""
+    nq, nkv, d, page = 16, 8, 128, 16
+    need = [-(-n // page) for n in lens]
+    kp, vp = (torch.randn(sum(need), nkv, page, d, device="cuda") for _ in range(2))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()   # noqa: E731
+    T = sum(counts)
+    tables = (i32([i for n, m in zip(lens, counts) for i in range(n - m, n)]), i32([r for r, m in enumerate(counts) for _ in range(m)]),
+              i32([0] + torch.tensor(need).cumsum(0).tolist()), i32(list(range(sum(need)))))
+    flat = torch.randn(T * nq * d + 1, device="cuda")
+
+    def us(q):
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            kernels.paged_attention_generic(q, kp, vp, *tables, d ** -0.5, None)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                kernels.paged_attention_generic(q, kp, vp, *tables, d ** -0.5, None)
+        times = []
+        for _ in range(7):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            graph.replay()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end) * 50.0)
+        return min(times)
+
+    chosen, other = us(flat[:-1].view(T, nq, d)), us(flat[1:].view(T, nq, d))
+    print(f"MEASURED 32-bit attention, portions {counts[:3]} of {lens[:3]}: {chosen:.1f} us, the form for any sizes {other:.1f}")
+    assert chosen < 1.07 * other + 0.3
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("case", ["far key", "first key", "page edge", "window edge in", "window edge out"])
 def test_paged_attention_finds_the_one_key_that_matters(kernels, dtype, case):

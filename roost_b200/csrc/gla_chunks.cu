@@ -5,14 +5,15 @@
 //   S'  = diag(P_n) S + sum_s (Q_s k_s) v_s^T.
 // Products of decays only ever shrink, so nothing overflows whatever the decays are. Values are bfloat16 and enter the products as they are; what is
 // kept in 32 bits stays so: the state, the decayed queries and keys and A enter as three bfloat16 operands each, whose sum is the 24 bits of the
-// float (six products where both sides are split, as many as count), sums are float32.
+// float (six products where both sides are split, as many as count), sums are float32: a few products from zero each, added to nearest (mma.cuh says why).
+// Outputs are no further from 64 bits than the walk's (1.1e-7 and 1.2e-7 of their norm; 6e-7 with all products of an output in one chain).
 //
 // A block takes a head of a row, eight warps 16 of its 128 values each with all 64 keys: a warp's part of S^T stays in registers as sums of a
 // product, which have the layout of a first operand. Per chunk all threads make the decayed queries and keys and A (a thread a key token and four
 // channels walks the queries after it) and leave them in shared memory; the next chunk's inputs arrive meanwhile. Rows are cut into segments as in
-// mamba2_chunks.cu: MODE 1 leaves a segment's own state and the products of its decays, the carry kernel every segment's true starting state, MODE
+// mamba2_chunks.cu (by the step's tokens): MODE 1 leaves a segment's own state and the products of its decays, the carry kernel every segment's true starting state, MODE
 // 2 makes the outputs; MODE 0 walks whole rows. A chunk whose outputs are not finite is taken again a token at a time (a product multiplies what a
-// token must not see by zero). What bounds it is the chain of a chunk's phases. Rows of 3,000 and 1,096 tokens, 16 heads: the layer 254 us, 447 with the
+// token must not see by zero). What bounds it is the chain of a chunk's phases. Rows of 3,000 and 1,096 tokens, 16 heads: the layer 260 us (256 with the chains), 447 with the
 // two walks on the FMA pipe (97 + 194 us of it) and a number a thread in the norm after it; 382 tokens 73 us, 293 before.
 #include "mma.cuh"
 
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(256, 2) gla_chunks_kernel(const __nv_bfloat16*
         if (MODE != 1) {
           const uint32_t qv = *reinterpret_cast<const uint32_t*>(qs + (t + i) * kGcD + d);
           const float fx = i ? pre.x : before.x * a0.x, fy = i ? pre.y : before.y * a0.y;
-          split3(__uint_as_float(qv << 16) * q_scale * fx, __uint_as_float(qv & 0xffff0000u) * q_scale * fy, p[0], p[1], p[2]);
+          split3_nearest(__uint_as_float(qv << 16) * q_scale * fx, __uint_as_float(qv & 0xffff0000u) * q_scale * fy, p[0], p[1], p[2]);
 #pragma unroll
           for (int pl = 0; pl < 3; ++pl) *reinterpret_cast<uint32_t*>(smem + kGcPq + pl * kGcTokens * kGcD * 2 + off) = p[pl];
         }
@@ -179,47 +180,56 @@ __global__ void __launch_bounds__(256, 2) gla_chunks_kernel(const __nv_bfloat16*
     uint32_t v[4];         // V^T: rows 16 values of the warp, k the chunk's tokens
     ldsm_x4_trans(v, tv + swizzled<kGcV * 2>((lane & 7) + ((lane >> 4) << 3), 2 * warp + ((lane >> 3) & 1)));
     if (MODE != 1) {
-      float Y[2][2][4];    // two sums of every tile, so that products of one do not wait for one another
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) Y[j][i][0] = Y[j][i][1] = Y[j][i][2] = Y[j][i][3] = 0.f;
+      // the products of leading parts are summed from zero and added in float32, rounded to nearest; the others, 2^-8 of them, in chains
+      float Y[2][4], low[2][4];
 #pragma unroll
       for (int pl = 2; pl >= 0; --pl) {
         uint32_t b[4];     // tokens t = 0 .. 7 at s 0 .. 7, 8 .. 15, then t = 8 .. 15
         ldsm_x4(b, sbase + kGcPa + pl * kGcTokens * kGcTokens * 2 + ((lane & 7) + ((lane >> 4) << 3)) * kGcTokens * 2 + ((lane >> 3) & 1) * 16);
-        mma_bf16(Y[0][0], v, b[0], b[1]);
-        mma_bf16(Y[1][0], v, b[2], b[3]);
+        if (pl == 1) {
+          mma_bf16(low[0], v, b[0], b[1]);
+          mma_bf16(low[1], v, b[2], b[3]);
+        } else {
+          mma_bf16_zero(pl == 2 ? low[0] : Y[0], v, b[0], b[1]);
+          mma_bf16_zero(pl == 2 ? low[1] : Y[1], v, b[2], b[3]);
+        }
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         uint32_t a[3][4], b[3][4];
-        split3(S[2 * k][0], S[2 * k][1], a[0][0], a[1][0], a[2][0]);
-        split3(S[2 * k][2], S[2 * k][3], a[0][1], a[1][1], a[2][1]);
-        split3(S[2 * k + 1][0], S[2 * k + 1][1], a[0][2], a[1][2], a[2][2]);
-        split3(S[2 * k + 1][2], S[2 * k + 1][3], a[0][3], a[1][3], a[2][3]);
+        split3_nearest(S[2 * k][0], S[2 * k][1], a[0][0], a[1][0], a[2][0]);
+        split3_nearest(S[2 * k][2], S[2 * k][3], a[0][1], a[1][1], a[2][1]);
+        split3_nearest(S[2 * k + 1][0], S[2 * k + 1][1], a[0][2], a[1][2], a[2][2]);
+        split3_nearest(S[2 * k + 1][2], S[2 * k + 1][3], a[0][3], a[1][3], a[2][3]);
 #pragma unroll
         for (int pl = 0; pl < 3; ++pl)
           ldsm_x4(b[pl], sbase + kGcPq + pl * kGcTokens * kGcD * 2 + swizzled<kGcD * 2>((lane & 7) + ((lane >> 4) << 3), 2 * k + ((lane >> 3) & 1)));
         // the parts' products down to 2^-16 of the largest, the least first; what is left out lies below the sums' last place
 #pragma unroll
-        for (int o = 2; o >= 0; --o)
+        for (int o = 2; o >= 1; --o)
 #pragma unroll
           for (int x = 0; x <= o; ++x) {
-            mma_bf16(Y[0][(o + x) & 1], a[x], b[o - x][0], b[o - x][1]);
-            mma_bf16(Y[1][(o + x) & 1], a[x], b[o - x][2], b[o - x][3]);
+            mma_bf16(low[0], a[x], b[o - x][0], b[o - x][1]);
+            mma_bf16(low[1], a[x], b[o - x][2], b[o - x][3]);
           }
+        float top[2][4];
+        mma_bf16_zero(top[0], a[0], b[0][0], b[0][1]);
+        mma_bf16_zero(top[1], a[0], b[0][2], b[0][3]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) Y[j][e] += top[j][e];
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) Y[j][0][e] += Y[j][1][e];
+        for (int e = 0; e < 4; ++e) Y[j][e] += low[j][e];
       if (n > 1) {
         bool odd = false;
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) odd |= 8 * j + 2 * c + (e & 1) < n && !isfinite(Y[j][0][e]);
+          for (int e = 0; e < 4; ++e) odd |= 8 * j + 2 * c + (e & 1) < n && !isfinite(Y[j][e]);
         if (__syncthreads_or(odd)) {       // again, a token at a time
           careful_until = t0 + n;
           copy_wait<0>();
@@ -233,28 +243,33 @@ __global__ void __launch_bounds__(256, 2) gla_chunks_kernel(const __nv_bfloat16*
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int t = 8 * j + 2 * c + (e & 1);
-          if (t < n) out[(size_t)(t0 + t) * heads * kGcV + (size_t)h * kGcV + warp * 16 + g + (e >> 1) * 8] = Y[j][0][e];
+          if (t < n) out[(size_t)(t0 + t) * heads * kGcV + (size_t)h * kGcV + warp * 16 + g + (e >> 1) * 8] = Y[j][e];
         }
     }
     // the state after the chunk
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float2 f = *reinterpret_cast<const float2*>(fade + 8 * j + 2 * c);
-      S[j][0] *= f.x;
-      S[j][1] *= f.y;
-      S[j][2] *= f.x;
-      S[j][3] *= f.y;
-    }
     if (MODE == 1 && tid < kGcD) keep *= fade[tid];
 #pragma unroll
-    for (int pl = 2; pl >= 0; --pl)
+    for (int j = 0; j < 8; j += 2) {
+      float low[2][4], top[2][4];
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
+      for (int pl = 2; pl >= 0; --pl) {
         uint32_t b[4];
         ldsm_x4_trans(b, sbase + kGcPk + pl * kGcTokens * kGcD * 2 + swizzled<kGcD * 2>(lane & 15, j + (lane >> 4)));
-        mma_bf16(S[j], v, b[0], b[1]);
-        mma_bf16(S[j + 1], v, b[2], b[3]);
+        if (pl == 1) {
+          mma_bf16(low[0], v, b[0], b[1]);
+          mma_bf16(low[1], v, b[2], b[3]);
+        } else {
+          mma_bf16_zero(pl == 2 ? low[0] : top[0], v, b[0], b[1]);
+          mma_bf16_zero(pl == 2 ? low[1] : top[1], v, b[2], b[3]);
+        }
       }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float2 f = *reinterpret_cast<const float2*>(fade + 8 * (j + i) + 2 * c);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[j + i][e] = fmaf(S[j + i][e], e & 1 ? f.y : f.x, top[i][e] + low[i][e]);
+      }
+    }
     t0 += n;
     if (careful) {
       if (t0 < end) {
@@ -317,6 +332,8 @@ static int gla_segment_tokens(int rows, int tokens, int heads) {
 
 using namespace roost;
 
+// Steps of few tokens a row stay with the walk, as in mamba2_chunks.cu: 16 heads, a prompt of 480 tokens beside 31 and 63 rows that decode 79 and 154 us a
+// layer here, 319 and 347 with the walk; fewer than eight tokens a row were not measured.
 extern "C" int roost_gla_chunks_parts(int rows, int tokens, int heads, int dim, int vdim, int dtype) {
   if (dtype != ROOST_BF16 || dim != kGcD || vdim != kGcV || rows <= 0 || rows > 65535 || heads > 65535 || tokens < 8LL * rows) return -1;
   const int segment = gla_segment_tokens(rows, tokens, heads);

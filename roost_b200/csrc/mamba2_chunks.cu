@@ -3,21 +3,22 @@
 //   y_t  = exp(e_t) S C_t + sum_{s <= t} [exp(e_t - e_s) dt_s (C_t . B_s)] x_s + D x_t,
 //   S'   = exp(e_n) S + sum_s [exp(e_n - e_s) dt_s x_s] B_s^T.
 // B, C and x are bfloat16 and enter the products as they are. What the walk keeps in 32 bits stays so: the state and the bracketed weights
-// enter as three bfloat16 operands each, whose sum is the 24 bits of the float; sums are float32; e_t is summed in double and kept as two floats.
+// enter as three bfloat16 operands each, whose sum is the 24 bits of the float; sums are float32, a few products from zero each, added to nearest (mma.cuh
+// says why: outputs 1.1e-7 from 64 bits, the walk's 1.6e-7, 2.1e-7 with all products in one chain); e_t is summed in double and kept as two floats.
 //
 // A block takes a head of a row and walks its chunks in order, the state in registers, so nothing of it goes through memory between chunks.
 // Eight warps: warp (pw, nh) keeps S for 16 of the head's 64 values and half of the state's N indices, as sums of a product, which have the
 // layout of a first operand: S C^T needs no shared memory for S. The two warps of a pw exchange their halves of it and then own half of the
 // chunk's tokens each. The weights of (t, s) are made once a block, from C B^T by all warps, and pass through shared memory.
 //
-// One long row would leave most processors idle, so steps of several chunks a processor cut their rows into segments of whole chunks (three
-// launches): MODE 1 walks every segment but a row's last from an empty state, making no outputs, and leaves its state and the product of its
+// One long row would leave most processors idle, so steps of more tokens than a segment cut their rows into segments of whole chunks, as long as the
+// step's tokens make them (a row's bits may then depend on what else is in its step; three launches): MODE 1 walks every segment but a row's last from an empty state, making no outputs, and leaves its state and the product of its
 // decays; a carry gives every segment the state it starts from; MODE 2 walks all segments from there. MODE 0 walks whole rows.
 //
 // A product multiplies what a token must not see by zero, so where a chunk's outputs are not finite the chunk is taken again a token at a time.
 //
 // What bounds it is the chain of a chunk's phases (about 5 us a chunk with two blocks a processor; mma.sync's 4 M multiply-adds a head and
-// chunk would take 2). Measured, bfloat16, 64 heads of 64 x 128, rows of 2,048, 1,037 and 1,011 tokens: the layer 476 us, 1,180 with the two
+// chunk would take 2). Measured, bfloat16, 64 heads of 64 x 128, rows of 2,048, 1,037 and 1,011 tokens: the layer 490 us (471 with the chains), 1,180 with the two
 // walks in 32-bit arithmetic (398 + 592 us of it); whole rows without segments 593. 32 heads, one row of 1,619: 120 us a layer, 351 before.
 #include "mma.cuh"
 
@@ -200,13 +201,23 @@ __global__ void __launch_bounds__(256, 2) mamba2_chunks_kernel(const __nv_bfloat
 #pragma unroll
         for (int j = 0; j < 2; ++j)
           ldsm_x4(b[j], tc + swizzled<KB>(32 * half + 16 * j + (lane & 7) + ((lane >> 4) << 3), nh * (NS / 16) + 2 * k + ((lane >> 3) & 1)));
+        float part[4][4];       // from zero, then added in float32 (see mma_bf16_zero)
 #pragma unroll
-        for (int q = 2; q >= 0; --q)
+        for (int j = 0; j < 2; ++j) {
+          mma_bf16_zero(part[2 * j], a[2], b[j][0], b[j][1]);
+          mma_bf16_zero(part[2 * j + 1], a[2], b[j][2], b[j][3]);
+        }
+#pragma unroll
+        for (int q = 1; q >= 0; --q)
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            mma_bf16(Y[4 * half + 2 * j], a[q], b[j][0], b[j][1]);
-            mma_bf16(Y[4 * half + 2 * j + 1], a[q], b[j][2], b[j][3]);
+            mma_bf16(part[2 * j], a[q], b[j][0], b[j][1]);
+            mma_bf16(part[2 * j + 1], a[q], b[j][2], b[j][3]);
           }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) Y[4 * half + j][e] += part[j][e];
       }
     }
     // the other half's owner gets its tokens' share
@@ -229,8 +240,11 @@ __global__ void __launch_bounds__(256, 2) mamba2_chunks_kernel(const __nv_bfloat
           if (i > pw) break;
           uint32_t b[4];
           ldsm_x4(b, tb + swizzled<KB>(8 * (nh * (pw + 1) + i) + (lane & 7), 2 * k + (lane >> 3)));
-          mma_bf16(G[i], a0, b[0], b[1]);
-          mma_bf16(G[i], a1, b[2], b[3]);
+          float part[4];
+          mma_bf16_zero(part, a0, b[0], b[1]);
+          mma_bf16(part, a1, b[2], b[3]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) G[i][e] += part[e];
         }
       }
     }
@@ -277,6 +291,7 @@ __global__ void __launch_bounds__(256, 2) mamba2_chunks_kernel(const __nv_bfloat
       if (k > 2 * nh + 1 || 32 * nh >= n) break;
       uint32_t a[4];
       ldsm_x4_trans(a, tx + swizzled<kM2P * 2>(16 * k + (lane & 7) + ((lane >> 4) << 3), 2 * pw + ((lane >> 3) & 1)));
+      float part[4][4];
 #pragma unroll
       for (int pl = 2; pl >= 0; --pl)
 #pragma unroll
@@ -285,9 +300,23 @@ __global__ void __launch_bounds__(256, 2) mamba2_chunks_kernel(const __nv_bfloat
           if (k > tt || 16 * tt >= n) continue;
           uint32_t b[4];
           ldsm_x4(b, sbase + M::kW + pl * kM2Tokens * kM2Tokens * 2 + swizzled<kM2Tokens * 2>(16 * tt + (lane & 7) + ((lane >> 4) << 3), 2 * k + ((lane >> 3) & 1)));
-          mma_bf16(Z[2 * q], a, b[0], b[1]);
-          mma_bf16(Z[2 * q + 1], a, b[2], b[3]);
+          if (pl == 2) {
+            mma_bf16_zero(part[2 * q], a, b[0], b[1]);
+            mma_bf16_zero(part[2 * q + 1], a, b[2], b[3]);
+          } else {
+            mma_bf16(part[2 * q], a, b[0], b[1]);
+            mma_bf16(part[2 * q + 1], a, b[2], b[3]);
+          }
         }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        if (k > 2 * nh + q || 16 * (2 * nh + q) >= n) continue;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          Z[2 * q][e] += part[2 * q][e];
+          Z[2 * q + 1][e] += part[2 * q + 1][e];
+        }
+      }
     }
     if (n > 1) {
       bool odd = false;
@@ -340,13 +369,23 @@ __global__ void __launch_bounds__(256, 2) mamba2_chunks_kernel(const __nv_bfloat
         uint32_t b[2][4];
 #pragma unroll
         for (int i = 0; i < 2; ++i) ldsm_x4_trans(b[i], tb + swizzled<KB>(16 * k + (lane & 15), nh * (NS / 16) + j + 2 * i + (lane >> 4)));
+        float part[4][4];
 #pragma unroll
-        for (int q = 2; q >= 0; --q)
+        for (int i = 0; i < 2; ++i) {
+          mma_bf16_zero(part[2 * i], a[2], b[i][0], b[i][1]);
+          mma_bf16_zero(part[2 * i + 1], a[2], b[i][2], b[i][3]);
+        }
+#pragma unroll
+        for (int q = 1; q >= 0; --q)
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
-            mma_bf16(S[j + 2 * i], a[q], b[i][0], b[i][1]);
-            mma_bf16(S[j + 2 * i + 1], a[q], b[i][2], b[i][3]);
+            mma_bf16(part[2 * i], a[q], b[i][0], b[i][1]);
+            mma_bf16(part[2 * i + 1], a[q], b[i][2], b[i][3]);
           }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) S[j + i][e] += part[i][e];
       }
     }
     t0 += n;
@@ -408,6 +447,8 @@ __global__ void __launch_bounds__(256) mamba2_segment_carry_kernel(float* ws_sta
   }
 }
 
+// A row of one token takes a block as long as a chunk does, so steps of few tokens a row stay with the walk. On this side of the line, 64 heads, a prompt of
+// 480 tokens beside 31 and 63 rows that decode: 250 and 543 us a layer, 509 and 1,186 with the walk; fewer than eight tokens a row were not measured.
 bool mamba2_chunks_serve(int rows, int tokens, int heads, int head_dim, int state_rows, int groups, int dtype) {
   return dtype == ROOST_BF16 && head_dim == kM2P && (state_rows == 64 || state_rows == 128) && rows <= 65535 && heads <= 65535 && tokens >= 8LL * rows;
 }

@@ -14,6 +14,14 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The same from zero. The tensor cores cut their sums off (towards zero), so a long chain of products onto one sum leans that way: 27 of them left
+// outputs five times as far from 64 bits as a chain of FMAs does. A few products from zero whose sum then joins a float32 sum by an addition that
+// rounds to nearest do not.
+__device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
@@ -49,6 +57,19 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
   mid = __byte_perm(xb1, yb1, 0x7632);
   const float x2 = x1 - __uint_as_float(xb1 & 0xffff0000u), y2 = y1 - __uint_as_float(yb1 & 0xffff0000u);
   lo = __byte_perm(__float_as_uint(x2), __float_as_uint(y2), 0x7632);
+}
+
+// The same parts rounded to nearest, for products of two such numbers: what is left out of them (the middle part of one times the last of the other)
+// is then a quarter as large and of either sign.
+__device__ __forceinline__ void split3_nearest(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  auto pack = [](float u, float v) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(u, v);
+    return *reinterpret_cast<const uint32_t*>(&p);
+  };
+  hi = pack(x, y);
+  const float x1 = x - __uint_as_float(hi << 16), y1 = y - __uint_as_float(hi & 0xffff0000u);
+  mid = pack(x1, y1);
+  lo = pack(x1 - __uint_as_float(mid << 16), y1 - __uint_as_float(mid & 0xffff0000u));
 }
 
 }  // namespace roost

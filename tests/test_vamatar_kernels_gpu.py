@@ -380,8 +380,8 @@ def test_recurrence_in_chunks_on_the_tensor_cores(kernels, H, N, groups, lengths
         assert torch.equal(torch.isfinite(got[torch.bfloat16][k]), fine) and torch.equal(torch.isfinite(got[torch.float32][k]), fine), name
         off = {t: float((got[t][k] - w)[fine].norm() / w[fine].norm()) for t in DTYPES}
         print(f"MEASURED recurrence in chunks {name}: tensor cores {off[torch.bfloat16]:.2e}, walk {off[torch.float32]:.2e}")
-        # float32 sums of up to N and 64 terms: a few units of 2^-24, whichever the order
-        assert off[torch.bfloat16] < max(2 * off[torch.float32], 1e-6), (name, off)
+        # no further off than the walk, whose sums of N and 64 terms leave it within a unit of 2^-23 or two
+        assert off[torch.bfloat16] < max(1.1 * off[torch.float32], 2.0 ** -23), (name, off)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

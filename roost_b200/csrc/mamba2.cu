@@ -13,7 +13,8 @@
 //               inside the root) and multiplied by the weight; the output has the activation dtype.
 // Prompt portions in bfloat16 of the sizes that mamba2_chunks.cu names run the scan there, as products on the tensor cores.
 // Rows are given by q_indptr (token range) and state_slots (slot per row); the padding rows of a captured step name a scratch
-// slot. Every sum's order depends on the sizes only, never on the batch.
+// slot. The convolution's sums have one order whatever the step holds, and in float32 the norm's. Which form of the scan runs, where a long row is
+// cut, and in bfloat16 the order of the norm's sum follow from the step's tokens and rows, so a row's bits may depend on what else is in its step.
 #include "common.cuh"
 
 namespace roost {
@@ -60,6 +61,9 @@ __global__ void __launch_bounds__(128) mamba2_conv_vec_kernel(const T* u, int64_
     wt[i] = *reinterpret_cast<const float4*>(w + (size_t)(c + i) * 4);
     b[i] = bias[c + i];
   }
+  // the first token's place in its row: the step's tables are looked up ahead of the wait (with a token a thread behind it they were most of the time)
+  const int r0 = token_row[t0], since0 = t0 - q_indptr[r0];
+  const float* st0 = state + (size_t)slots[r0] * state_stride + conv_off + c;
   pdl_wait();
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -78,9 +82,10 @@ __global__ void __launch_bounds__(128) mamba2_conv_vec_kernel(const T* u, int64_
     for (int j = 0; j < BATCH; ++j) {
       const int t = t0 + j0 + j;
       if (t >= tokens) return;
-      const int r = token_row[t], since = t - q_indptr[r];
+      const bool first = j0 + j == 0;
+      const int r = first ? r0 : token_row[t], since = first ? since0 : t - q_indptr[r];
       if (since < 3) {       // taps before the row's first token of the step are the slot's
-        const float* st = state + (size_t)slots[r] * state_stride + conv_off + c;
+        const float* st = first ? st0 : state + (size_t)slots[r] * state_stride + conv_off + c;
 #pragma unroll
         for (int k = 0; k < 3; ++k)
           if (since + k < 3) {
@@ -431,11 +436,11 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const T* __
   }
 }
 
-// The same with a row's values in registers, 16 bytes of y at a time: a warp a (token, group) of up to 1,024 values (WARP), else a block of 256
-// threads. Bound by memory: 4,096 tokens x 4,096 in groups of 512 took 184 us a number at a time, 27 us here (134 MB).
-template <typename T, int NV, bool WARP>
-__global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* y, const T* u, int64_t ld_u, const float* __restrict__ w, T* out, int tokens,
-                                                                  int inner, int groups, float eps) {
+// The same in bfloat16 with a row's values in registers, 16 bytes of y at a time: a warp a (token, group) of up to 1,024 values (WARP), else a block of 256
+// threads. Its squares are added in another order, so float32, whose bits do not depend on a step's size, stays with the form above. Bound by memory: 4,096 tokens x 4,096 in groups of 512 took 184 us a number at a time, 27 us here (134 MB).
+template <int NV, bool WARP>
+__global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* y, const __nv_bfloat16* u, int64_t ld_u, const float* __restrict__ w,
+                                                                  __nv_bfloat16* out, int tokens, int inner, int groups, float eps) {
   __shared__ float scratch[32];
   pdl_launch_dependents();
   const int gs = inner / groups, width = WARP ? 32 : 256;
@@ -452,14 +457,8 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
     v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0.f;
     if (j < gs) {
       const float4 a = *reinterpret_cast<const float4*>(y + (size_t)t * inner + c0 + j);
-      float z[4];
-      if constexpr (sizeof(T) == 4) {
-        Vec<float>::load(u + (size_t)t * ld_u + c0 + j, z);
-      } else {
-        const uint2 q = *reinterpret_cast<const uint2*>(u + (size_t)t * ld_u + c0 + j);
-        z[0] = __uint_as_float(q.x << 16); z[1] = __uint_as_float(q.x & 0xffff0000u);
-        z[2] = __uint_as_float(q.y << 16); z[3] = __uint_as_float(q.y & 0xffff0000u);
-      }
+      const uint2 q = *reinterpret_cast<const uint2*>(u + (size_t)t * ld_u + c0 + j);
+      const float z[4] = {__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xffff0000u), __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xffff0000u)};
       v[i][0] = a.x * silu_f(z[0]); v[i][1] = a.y * silu_f(z[1]); v[i][2] = a.z * silu_f(z[2]); v[i][3] = a.w * silu_f(z[3]);
     }
 #pragma unroll
@@ -472,16 +471,16 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
     const int j = (lane + i * width) * 4;
     if (j >= gs) continue;
     const float4 ww = *reinterpret_cast<const float4*>(w + c0 + j);
-    T* to = out + (size_t)t * inner + c0 + j;
     const float o[4] = {v[i][0] * inv * ww.x, v[i][1] * inv * ww.y, v[i][2] * inv * ww.z, v[i][3] * inv * ww.w};
-    if constexpr (sizeof(T) == 4) {
-      Vec<float>::store(to, o);
-    } else {
-      __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
-      *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-    }
+    __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+    *reinterpret_cast<uint2*>(out + (size_t)t * inner + c0 + j) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
   }
 }
+
+// Where the vector forms begin to win: numbers of a step's convolution (2,048 channels: 256 tokens 6.3 us, 5.8 a number a thread; 512 9.5 and 9.9; 1,000 13.8 and 17.3;
+// 6,144 channels: 192 tokens 8.7 and 10.8), and groups of a step's norm where a warp takes one (8 of 512 a token: 148 tokens 4.3 us, 3.9 with a block a group;
+// 192 4.5 and 4.7; 1,200 9.9 and 19.9).
+constexpr long long kConvVecMin = 1 << 20, kNormVecMin = 1536;
 
 }  // namespace roost
 
@@ -497,10 +496,11 @@ extern "C" int roost_mamba2_conv(const void* u, int64_t ld, int col, void* out, 
   {
     const int64_t vec = dtype == ROOST_F32 ? 4 : 8;
     const uintptr_t at = (uintptr_t)u | (uintptr_t)out | (uintptr_t)w | (uintptr_t)state;
-    if ((dtype == ROOST_F32 || dtype == ROOST_BF16) && taps == 4 && channels % vec == 0 && ld % vec == 0 && col % vec == 0 && at % 16 == 0 && state_stride % 4 == 0 &&
+    if ((long long)tokens * channels >= kConvVecMin && (dtype == ROOST_F32 || dtype == ROOST_BF16) && taps == 4 && channels % vec == 0 && ld % vec == 0 && col % vec == 0 && at % 16 == 0 && state_stride % 4 == 0 &&
         conv_off % 4 == 0) {
       const unsigned gy = (unsigned)((channels / vec + 127) / 128);
-      // sixteen tokens a thread where that leaves every processor several blocks, else one
+      // sixteen tokens a thread where that leaves every processor several blocks, else one; few numbers are spread over more threads by the form for
+      // any sizes
       const bool many = (long long)(tokens / 16) * gy >= 4 * 148;
       ROOST_DISPATCH_DTYPE(dtype, T, {
         auto kernel = many ? mamba2_conv_vec_kernel<T, 16> : mamba2_conv_vec_kernel<T, 1>;
@@ -613,16 +613,15 @@ extern "C" int roost_gated_group_norm(const float* y, const void* u, int64_t ld_
   if (groups > 65535) return fail(ROOST_ERR_UNSUPPORTED, "gated_group_norm: too many groups");
   const int gs = inner / groups;
   const uintptr_t at = (uintptr_t)y | (uintptr_t)w, half = (uintptr_t)u | (uintptr_t)out;
-  if (gs % 4 == 0 && gs <= 8192 && ld_u % 4 == 0 && at % 16 == 0 && half % (dtype == ROOST_F32 ? 16 : 8) == 0 && (long long)tokens * groups <= INT32_MAX) {
+  // a warp a group leaves the processors idle where there are few: then a block a group, as for any sizes
+  if (dtype == ROOST_BF16 && (gs > 1024 || (long long)tokens * groups >= kNormVecMin) && gs % 4 == 0 && gs <= 8192 && ld_u % 4 == 0 && at % 16 == 0 && half % 8 == 0 &&
+      (long long)tokens * groups <= INT32_MAX) {
     const bool warp = gs <= 1024;
     const dim3 blocks((unsigned)(warp ? ((long long)tokens * groups + 7) / 8 : (long long)tokens * groups));
-    ROOST_DISPATCH_DTYPE(dtype, T, {
-      auto kernel = warp ? (gs <= 256 ? gated_group_norm_vec_kernel<T, 2, true> : gs <= 512 ? gated_group_norm_vec_kernel<T, 4, true>
-                                                                                            : gated_group_norm_vec_kernel<T, 8, true>)
-                         : (gs <= 2048 ? gated_group_norm_vec_kernel<T, 2, false> : gs <= 4096 ? gated_group_norm_vec_kernel<T, 4, false>
-                                                                                               : gated_group_norm_vec_kernel<T, 8, false>);
-      launch_kernel(kernel, blocks, dim3(256), 0, (cudaStream_t)stream, y, (const T*)u, ld_u, w, (T*)out, tokens, inner, groups, eps);
-    });
+    auto kernel = warp ? (gs <= 256 ? gated_group_norm_vec_kernel<2, true> : gs <= 512 ? gated_group_norm_vec_kernel<4, true> : gated_group_norm_vec_kernel<8, true>)
+                       : (gs <= 2048 ? gated_group_norm_vec_kernel<2, false> : gs <= 4096 ? gated_group_norm_vec_kernel<4, false>
+                                                                                          : gated_group_norm_vec_kernel<8, false>);
+    launch_kernel(kernel, blocks, dim3(256), 0, (cudaStream_t)stream, y, (const __nv_bfloat16*)u, ld_u, w, (__nv_bfloat16*)out, tokens, inner, groups, eps);
     return check_launch("gated_group_norm");
   }
   const size_t smem = ((size_t)gs + 32) * sizeof(float);

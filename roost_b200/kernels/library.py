@@ -1468,7 +1468,9 @@ class KernelLibrary:
 
     SIGMOID_MMA_MIN_TOKENS = 32     # tokens from which a bfloat16 step that brings prompt portions runs the tensor-core form
     SIGMOID_MMA_CHUNK_TILES = 8     # tiles of 64 keys a block of the tensor-core form takes of a long row
-    SIGMOID_TC_CHUNK_TILES = 16     # tiles of 128 keys a block of the tcgen05 form takes of a long row
+    # Tiles of 128 keys a block of the tcgen05 form takes of a long row. With 8 a layer of 64 tokens at 4,000 keys takes 34 us (46 with 16, 76 with all keys
+    # in one block), 1,024 tokens at 16,000 keys 262 (235, 239); 16 is no slower than one block at any size that was measured.
+    SIGMOID_TC_CHUNK_TILES = 16
 
     def sigmoid_attention_mma_supported(self, dim: int, vdim: int, two_planes: bool) -> bool:
         return bool(self._lib.roost_sigmoid_attention_mma_supported(int(dim), int(vdim), int(dim if two_planes else dim + vdim)))

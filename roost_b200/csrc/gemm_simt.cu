@@ -297,6 +297,7 @@ static int launch_gemm_simt(const void* a, const void* w, void* out, int batch, 
   ROOST_REQUIRE(m >= 0 && n > 0 && k > 0 && batch >= 0, "gemm: m, n and k must be positive");
   ROOST_REQUIRE(lda >= k && ldw >= k && ldo >= n, "gemm: a leading dimension is smaller than its row");
   if (m == 0 || batch == 0) return ROOST_OK;
+  // the bound that callers have always had (tiles lay along the grid's y once)
   if (m > 64 * 65535) return fail(ROOST_ERR_UNSUPPORTED, "gemm: more than 4194240 rows in one product");
   if (batch > 65535) return fail(ROOST_ERR_UNSUPPORTED, "gemm: more than 65535 products in one batch");
   const SimtArgs g = {a, w, out, batch, m, n, k, lda, ldw, ldo, batch_a, batch_w, batch_o, (cudaStream_t)stream};

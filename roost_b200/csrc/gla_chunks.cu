@@ -13,7 +13,7 @@
 // channels walks the queries after it) and leave them in shared memory; the next chunk's inputs arrive meanwhile. Rows are cut into segments as in
 // mamba2_chunks.cu (by the step's tokens): MODE 1 leaves a segment's own state and the products of its decays, the carry kernel every segment's true starting state, MODE
 // 2 makes the outputs; MODE 0 walks whole rows. A chunk whose outputs are not finite is taken again a token at a time (a product multiplies what a
-// token must not see by zero). What bounds it is the chain of a chunk's phases. Rows of 3,000 and 1,096 tokens, 16 heads: the layer 260 us (256 with the chains), 447 with the
+// token must not see by zero). What bounds it is the chain of a chunk's phases. Rows of 3,000 and 1,096 tokens, 16 heads: the layer 263 us (256 to 259 with the chains), 447 with the
 // two walks on the FMA pipe (97 + 194 us of it) and a number a thread in the norm after it; 382 tokens 73 us, 293 before.
 #include "mma.cuh"
 

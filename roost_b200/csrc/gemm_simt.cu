@@ -1,5 +1,5 @@
-// out[m,n] = sum_k a[m,k] * w[n,k] with plain 32-bit FFMA: the matrix product of the float32 model (no tensor
-// cores, no reduced-precision mode), also usable with bfloat16 operands for checks. Every output element sums
+// out[m,n] = sum_k a[m,k] * w[n,k] with plain 32-bit FFMA: the products of the float32 model that gemm_f32_tc.cu does not take
+// (short reductions, vocabulary-sized heads, rows of w that do not start on 16 bytes), also usable with bfloat16 operands for checks. Every output element sums
 // over k in increasing order in one thread, so its bits do not depend on m's or n's extent or on the tile a
 // row falls in. Definition: src/Starlings.Roost.Ops/CpuOps.cs:395-437 (TransposeB, Alpha 1, no bias).
 //
@@ -16,6 +16,10 @@
 #include "common.cuh"
 
 namespace roost {
+
+// gemm_f32_tc.cu
+bool gemm_f32_tc_takes(const void* w, int n, int k, int64_t ldw);
+int launch_gemm_f32_tc(const float* a, const float* w, float* out, int m, int n, int k, int64_t lda, int64_t ldw, int64_t ldo, cudaStream_t stream);
 
 constexpr int kSimtK = 32;           // k of a stage
 constexpr int kSimtLd = kSimtK + 4;  // eight rows' 16-byte pieces of one k fall in different banks
@@ -309,6 +313,9 @@ static int launch_gemm_simt(const void* a, const void* w, void* out, int batch, 
 
 extern "C" int roost_gemm_simt(const void* a, const void* w, void* out, int m, int n, int k, int64_t lda, int64_t ldw,
                                int64_t ldo, int in_dtype, int out_dtype, roost_stream_t stream) {
+  if (in_dtype == ROOST_F32 && out_dtype == ROOST_F32 && m > 0 && m <= 64 * 65535 && n > 0 && k > 0 && lda >= k && ldw >= k && ldo >= n &&
+      gemm_f32_tc_takes(w, n, k, ldw))
+    return launch_gemm_f32_tc((const float*)a, (const float*)w, (float*)out, m, n, k, lda, ldw, ldo, (cudaStream_t)stream);
   return launch_gemm_simt(a, w, out, 1, m, n, k, lda, ldw, ldo, 0, 0, 0, in_dtype, out_dtype, stream);
 }
 

@@ -190,8 +190,9 @@ int roost_attention_decode_static(const void* q, void* out, const void* k_pool, 
                                   int q_heads, int kv_heads, int head_dim, int page_size, float scale, int window,
                                   roost_stream_t stream);
 
-/* out[m,n] = sum_k a[m,k] * w[n,k], plain FFMA in 32-bit (no tensor cores, no reduced-precision mode), the
- * sum over k in increasing order for every output, whatever m is. in_dtype/out_dtype: 0 or 1. */
+/* out[m,n] = sum_k a[m,k] * w[n,k] in 32 bits (no reduced-precision mode): FFMAs over k in increasing order for every output or, float32 with
+ * k >= 512 and n < 65536, all 24 bits of the operands on the tensor cores (gemm_f32_tc.cu; its waits are bounded, see
+ * roost_gemm_tcgen05_status). A row's bits do not depend on m. in_dtype/out_dtype: 0 or 1. */
 int roost_gemm_simt(const void* a, const void* w, void* out, int m, int n, int k, int64_t lda, int64_t ldw,
                     int64_t ldo, int in_dtype, int out_dtype, roost_stream_t stream);
 

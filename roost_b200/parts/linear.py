@@ -1,8 +1,7 @@
 """y = x W^T for a weight stored [out, in] (src/Starlings.Roost.Ops/CpuOps.cs:395-437), with a bias where a part asks for one.
 
-float32 runs the library's FFMA product (true 32-bit, the same bits for a row whatever the batch). bfloat16
-with 32-bit accumulation goes to cuBLAS through torch, the place where the reference's engine also calls a
-library (kernels/src/gemm.cu:235), except where a kernel of this library is faster. ``Runtime.small_gemm`` decides for
+float32 runs the library's 32-bit product (operands of 24 bits on the tensor cores, or FFMAs; the same bits for a row whatever
+the batch). bfloat16 with 32-bit accumulation goes to cuBLAS through torch, the place where the reference's engine also calls a library (kernels/src/gemm.cu:235), except where a kernel of this library is faster. ``Runtime.small_gemm`` decides for
 products of at most 64 rows (decode steps): "auto" takes this library's TMA/tcgen05 kernels where they were measured
 faster than cuBLAS on a B200 (the product with k split over thread-block clusters for weights of few tiles and a long k:
 output and down projections of at most 8 rows; the weight-streaming product for at most 16 rows and a reduction length

@@ -190,6 +190,13 @@ int roost_attention_decode_static(const void* q, void* out, const void* k_pool, 
                                   int q_heads, int kv_heads, int head_dim, int page_size, float scale, int window,
                                   roost_stream_t stream);
 
+/* out[m,n] = sum_k x[m,k] * w[n,k] for 1 <= m <= 16 rows and weights that fit the processors' registers (roost_gemm_rows_supported), bfloat16 operands
+ * that start on 16 bytes, 32-bit sums; out bfloat16 or float32. swiglu: w's rows in blocks of 128 gate rows and their 128 up rows, out[m, n / 2] =
+ * silu(gate) * up in bfloat16. w must not be written by a kernel of the stream: it is read ahead of the kernels in front. */
+int roost_gemm_rows_supported(int m, int n, int k, int64_t ldx, int64_t ldw, int swiglu);
+int roost_gemm_rows(const void* x, const void* w, void* out, int m, int n, int k, int64_t ldx, int64_t ldw, int64_t ldo, int out_dtype, int swiglu,
+                    roost_stream_t stream);
+
 /* out[m,n] = sum_k a[m,k] * w[n,k] in 32 bits (no reduced-precision mode): FFMAs over k in increasing order for every output or, float32 with
  * k >= 512 and n < 65536, all 24 bits of the operands on the tensor cores (gemm_f32_tc.cu; its waits are bounded, see
  * roost_gemm_tcgen05_status). A row's bits do not depend on m. in_dtype/out_dtype: 0 or 1. */

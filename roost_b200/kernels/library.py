@@ -98,6 +98,8 @@ _SIGNATURES = {
     "roost_sample_count_tokens": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p],
     "roost_sample_prompt_bits": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "roost_sample_logprobs": [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
+    "roost_gemm_rows_supported": [c_int, c_int, c_int, c_int64, c_int64, c_int],
+    "roost_gemm_rows": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64, c_int, c_int, c_void_p],
     "roost_gemm_simt": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64, c_int, c_int, c_void_p],
     "roost_gemm_tcgen05_supported": [c_int, c_int, c_int, c_int64, c_int64],
     "roost_gemm_tcgen05": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64, c_int, c_void_p],
@@ -514,6 +516,22 @@ class KernelLibrary:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
         self._call("roost_gemm_simt", _ptr(a), _ptr(w), _ptr(out), M, N, K, a.stride(0), w.stride(0), out.stride(0),
                    dtype_code(a.dtype), dtype_code(out_dtype), _stream())
+        return out
+
+    def gemm_rows_supported(self, x: torch.Tensor, w: torch.Tensor, swiglu: bool = False) -> bool:
+        """The product of the few rows of a decode step over weights that fit the processors' registers."""
+        return (x.stride(1) == 1 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+                and bool(self._lib.roost_gemm_rows_supported(x.shape[0], w.shape[0], w.shape[1], x.stride(0), w.stride(0), int(swiglu))))
+
+    def gemm_rows(self, x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None, swiglu: bool = False) -> torch.Tensor:
+        """x [M <= 16, K] times w [N, K] transposed; ``swiglu``: w holds gate and up rows interleaved in blocks of 128, silu(gate) * up."""
+        if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or x.shape[1] != w.shape[1]:
+            raise KernelError("gemm_rows: the operands are not bfloat16 matrices of one reduction length")
+        out_dtype = out_dtype or torch.bfloat16
+        N = w.shape[0] // 2 if swiglu else w.shape[0]
+        out = torch.empty((x.shape[0], N), dtype=out_dtype, device=x.device)
+        self._call("roost_gemm_rows", _ptr(x), _ptr(w), _ptr(out), x.shape[0], w.shape[0], w.shape[1], x.stride(0), w.stride(0), out.stride(0), dtype_code(out_dtype),
+                   int(swiglu), _stream())
         return out
 
     def gemm_tcgen05_supported(self, m: int, n: int, k: int, lda: int, ldw: int) -> bool:

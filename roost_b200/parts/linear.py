@@ -55,6 +55,8 @@ class Linear:
         M = x.shape[0]
         if M <= 64 and x.is_contiguous():
             policy = self.rt.small_gemm
+            if policy == "auto" and M <= 16 and getattr(k, "gemm_rows_supported", None) and k.gemm_rows_supported(x, self.weight):
+                return k.gemm_rows(x, self.weight, out_dtype)         # weights held in registers ahead of x, mma.sync products
             if policy in ("auto", "split") and getattr(k, "gemm_split_supported", None):
                 choose = k.gemm_split_supported if policy == "split" else k.gemm_split_preferred
                 if choose(M, self.out_features, self.in_features, x.stride(0), self.weight.stride(0)):

@@ -72,6 +72,9 @@ class GatedMlp(FeedForward):
         if (self.interleave and x.shape[0] >= self.fused_min_rows and x.is_contiguous()
                 and float(x.shape[0]) * self.spec.intermediate * self.spec.hidden >= self.fused_min_work):
             return self.down(k.gemm_tcgen05_swiglu(x, self.gate_up.weight))
+        if (self.interleave and x.shape[0] <= 16 and self.rt.small_gemm == "auto" and hasattr(k, "gemm_rows_supported")
+                and k.gemm_rows_supported(x, self.gate_up.weight, swiglu=True)):
+            return self.down(k.gemm_rows(x, self.gate_up.weight, swiglu=True))
         if (self.interleave and x.shape[0] <= self.fused_max_split_rows and x.is_contiguous()
                 and self.rt.small_gemm in self.fused_split_policies and hasattr(k, "gemm_split_swiglu")):
             w = self.gate_up.weight

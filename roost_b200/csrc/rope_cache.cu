@@ -263,6 +263,84 @@ __global__ void __launch_bounds__(256, 4) qk_norm_rope_cache_parts_kernel(
   }
 }
 
+// The same arithmetic for few tokens, where the kernel's latency is its cost: D / 8 lanes a head slot. Weights, angles and the place in the cache come from
+// the step's tables and are in registers before pdl_wait(), and what follows it runs once ahead of it, without a head, so that its instructions are in
+// the processor's cache (see gemm_rows.cu): a token of 16 + 8 + 8 heads of 128 takes 1.4 us from the end of the product in front, 3.6 with a warp a
+// head in the kernel for any sizes.
+template <int D>
+__global__ void __launch_bounds__(128) qk_norm_rope_cache_few_kernel(
+    const __nv_bfloat16* qkv, int64_t qkv_stride, __nv_bfloat16* q_out, __nv_bfloat16* k_pool, __nv_bfloat16* v_pool, const void* __restrict__ q_w,
+    const void* __restrict__ k_w, const double* __restrict__ inv_freq, const int32_t* __restrict__ positions, const int32_t* __restrict__ slot_mapping, int tokens,
+    int q_heads, int kv_heads, float eps, int page_size, int64_t pool_pages, int slots_per_token, int wdtype) {
+  constexpr int kLanes = D / 8, kHalf = D / 2;
+  const int lane = threadIdx.x & 31, sub = lane / kLanes, c = lane % kLanes;
+  const unsigned part_lanes = kLanes == 32 ? 0xffffffffu : ((1u << kLanes) - 1u) << (sub * kLanes);
+  pdl_launch_dependents(3);
+  const int64_t group = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  const int t = (int)(group / slots_per_token), slot_idx = (int)(group - (int64_t)t * slots_per_token);
+  bool live = t < tokens;
+  const bool is_q = slot_idx < q_heads, is_v = slot_idx >= q_heads + kv_heads;
+  float w_lo[4], w_hi[4], cs[4], sn[4];
+  __nv_bfloat16* dst = q_out;
+  const __nv_bfloat16* src = qkv;
+  const void* w = is_q ? q_w : k_w;
+  const bool normed = w != nullptr;
+  if (live) {
+    src = qkv + (size_t)t * qkv_stride + (size_t)slot_idx * D + 4 * c;
+    if (is_q) {
+      dst = q_out + ((size_t)t * q_heads + slot_idx) * D + 4 * c;
+    } else {
+      const int slot = slot_mapping[t], head = slot_idx - q_heads - (is_v ? kv_heads : 0);
+      const int64_t page = slot < 0 ? pool_pages : slot / page_size;
+      live = page < pool_pages;      // a skipped token, or never write beyond the pool
+      dst = (is_v ? v_pool : k_pool) + (((size_t)page * kv_heads + head) * page_size + slot % page_size) * D + 4 * c;
+    }
+    const double pos = (double)positions[t];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      w_lo[e] = normed && !is_v ? load_w(w, 4 * c + e, wdtype) : 1.0f;
+      w_hi[e] = normed && !is_v ? load_w(w, kHalf + 4 * c + e, wdtype) : 1.0f;
+      double ang = pos * inv_freq[4 * c + e];
+      ang -= 6.283185307179586476925286766559 * rint(ang * 0.15915494309189533576888376337251);
+      sincosf((float)ang, &sn[e], &cs[e]);
+    }
+  }
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    if (pass) pdl_wait(3);
+    uint2 raw_lo = make_uint2(0, 0), raw_hi = make_uint2(0, 0);
+    if (pass && live) {
+      raw_lo = *reinterpret_cast<const uint2*>(src);
+      raw_hi = *reinterpret_cast<const uint2*>(src + kHalf);
+    }
+    float lo[4] = {__uint_as_float(raw_lo.x << 16), __uint_as_float(raw_lo.x & 0xffff0000u), __uint_as_float(raw_lo.y << 16), __uint_as_float(raw_lo.y & 0xffff0000u)};
+    float hi[4] = {__uint_as_float(raw_hi.x << 16), __uint_as_float(raw_hi.x & 0xffff0000u), __uint_as_float(raw_hi.y << 16), __uint_as_float(raw_hi.y & 0xffff0000u)};
+    float inv = 1.0f;
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ss += lo[e] * lo[e] + hi[e] * hi[e];
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(part_lanes, ss, o, kLanes);
+    if (normed) inv = 1.0f / sqrtf(ss / (float)D + eps);
+    if (!is_v) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float x1 = lo[e] * inv * w_lo[e], x2 = hi[e] * inv * w_hi[e];
+        lo[e] = x1 * cs[e] - x2 * sn[e];
+        hi[e] = x2 * cs[e] + x1 * sn[e];
+      }
+      const __nv_bfloat162 a = __floats2bfloat162_rn(lo[0], lo[1]), b = __floats2bfloat162_rn(lo[2], lo[3]);
+      const __nv_bfloat162 d = __floats2bfloat162_rn(hi[0], hi[1]), f = __floats2bfloat162_rn(hi[2], hi[3]);
+      raw_lo = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+      raw_hi = make_uint2(*reinterpret_cast<const uint32_t*>(&d), *reinterpret_cast<const uint32_t*>(&f));
+    }
+    if (pass && live) {
+      *reinterpret_cast<uint2*>(dst) = raw_lo;
+      *reinterpret_cast<uint2*>(dst + kHalf) = raw_hi;
+    }
+  }
+}
+
 }  // namespace roost
 
 using namespace roost;
@@ -321,6 +399,20 @@ extern "C" int roost_qk_norm_rope_cache(const void* qkv, int64_t qkv_stride, voi
     if (head_dim == 64) launch(qk_norm_rope_cache_parts_kernel<64>);
     else if (head_dim == 128) launch(qk_norm_rope_cache_parts_kernel<128>);
     else launch(qk_norm_rope_cache_parts_kernel<256>);
+    return check_launch("qk_norm_rope_cache");
+  }
+  // fewer tokens, the angles not from a step's table (a kernel of the step may write that): the latency form
+  if (dtype == ROOST_BF16 && vector_ok && rotary_dim == head_dim && cos_sin == nullptr && (head_dim == 64 || head_dim == 128 || head_dim == 256)) {
+    const int64_t blocks = ((int64_t)tokens * slots * (head_dim / 8) + 127) / 128;
+    if (blocks > 0x7fffffff) return fail(ROOST_ERR_UNSUPPORTED, "qk_norm_rope_cache: more blocks than a grid holds");
+    auto launch = [&](auto kernel) {
+      launch_kernel(kernel, dim3((unsigned)blocks), dim3(128), 0, (cudaStream_t)stream, (const __nv_bfloat16*)qkv, qkv_stride, (__nv_bfloat16*)q_out,
+                    (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, q_w, k_w, inv_freq, positions, slot_mapping, tokens, q_heads, kv_heads, eps, page_size,
+                    pool_pages, slots, wdtype);
+    };
+    if (head_dim == 64) launch(qk_norm_rope_cache_few_kernel<64>);
+    else if (head_dim == 128) launch(qk_norm_rope_cache_few_kernel<128>);
+    else launch(qk_norm_rope_cache_few_kernel<256>);
     return check_launch("qk_norm_rope_cache");
   }
   ROOST_DISPATCH_DTYPE(dtype, T, {

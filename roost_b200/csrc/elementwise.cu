@@ -174,6 +174,23 @@ __global__ void silu_mul_vec_kernel(const T* __restrict__ x, T* __restrict__ out
   Vec<T>::store(out + t * inter + (size_t)vi * N, o);
 }
 
+// The state of every row whose request begins set to zero: state [runs][slots][bytes], block (row, run, piece).
+__global__ void zero_slots_kernel(char* state, const int32_t* __restrict__ slots, const int32_t* __restrict__ fresh, int64_t run_bytes, int64_t slot_bytes,
+                                  int64_t bytes, int n_slots) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int r = blockIdx.x, slot = slots[r];
+  if (fresh[r] == 0 || slot < 0 || slot >= n_slots) return;
+  char* p = state + blockIdx.y * run_bytes + slot * slot_bytes;
+  const bool whole = (((uintptr_t)p | (uintptr_t)bytes) % 16) == 0;
+  const int64_t at = (int64_t)blockIdx.z * blockDim.x + threadIdx.x, step = (int64_t)gridDim.z * blockDim.x;
+  if (whole) {
+    for (int64_t i = at * 16; i < bytes; i += step * 16) *reinterpret_cast<uint4*>(p + i) = make_uint4(0, 0, 0, 0);
+  } else {
+    for (int64_t i = at; i < bytes; i += step) p[i] = 0;
+  }
+}
+
 // The error words of the kernels that wait with a limit (defined beside those kernels).
 int* gemm_tcgen05_error_address();
 int* attention_error_address();
@@ -210,6 +227,18 @@ extern "C" int roost_status_snapshot(int32_t* out, int out_is_host, roost_stream
   cudaError_t e = launch_kernel(status_snapshot_kernel, dim3(1), dim3(32), 0, (cudaStream_t)stream, a, b, c, dst);
   if (e != cudaSuccess) return fail(ROOST_ERR_CUDA, std::string("status_snapshot: ") + cudaGetErrorString(e));
   return ROOST_OK;
+}
+
+extern "C" int roost_zero_slots(void* state, const int32_t* slots, const int32_t* fresh, int rows, int runs, int64_t run_bytes, int64_t slot_bytes, int64_t bytes,
+                               int n_slots, roost_stream_t stream) {
+  ROOST_REQUIRE(state && slots && fresh, "zero_slots: a pointer is null");
+  ROOST_REQUIRE(rows >= 0 && runs > 0 && n_slots > 0 && bytes >= 0 && slot_bytes >= bytes, "zero_slots: the sizes do not fit");
+  if (runs > 65535) return fail(ROOST_ERR_UNSUPPORTED, "zero_slots: more than 65535 runs");
+  if (rows == 0 || bytes == 0) return ROOST_OK;
+  const int64_t pieces = (bytes + 16 * 256 * 4 - 1) / (16 * 256 * 4);
+  launch_kernel(zero_slots_kernel, dim3(rows, runs, (unsigned)(pieces < 256 ? pieces : 256)), dim3(256), 0, (cudaStream_t)stream, (char*)state, slots, fresh,
+                run_bytes, slot_bytes, bytes, n_slots);
+  return check_launch("zero_slots");
 }
 
 extern "C" int roost_abi_version(void) { return ROOST_ABI_VERSION; }

@@ -190,6 +190,11 @@ int roost_attention_decode_static(const void* q, void* out, const void* k_pool, 
                                   int q_heads, int kv_heads, int head_dim, int page_size, float scale, int window,
                                   roost_stream_t stream);
 
+/* state [runs][n_slots][bytes] (strides run_bytes and slot_bytes): zeros where fresh[r] is not 0, in slot slots[r] of every run, for each of `rows` rows. A slot
+ * outside 0 .. n_slots - 1 is skipped. */
+int roost_zero_slots(void* state, const int32_t* slots, const int32_t* fresh, int rows, int runs, int64_t run_bytes, int64_t slot_bytes, int64_t bytes, int n_slots,
+                     roost_stream_t stream);
+
 /* out[m,n] = sum_k x[m,k] * w[n,k] for 1 <= m <= 16 rows and weights that fit the processors' registers (roost_gemm_rows_supported), bfloat16 operands
  * that start on 16 bytes, 32-bit sums; out bfloat16 or float32. swiglu: w's rows in blocks of 128 gate rows and their 128 up rows, out[m, n / 2] =
  * silu(gate) * up in bfloat16. w must not be written by a kernel of the stream: it is read ahead of the kernels in front. */

@@ -434,6 +434,9 @@ class StepExecutor:
                 continue
             tables = batch.groups[gi]
             state = self.storage.tensors[gi]                        # [runs, slots + 1, *shape]
+            if hasattr(self.rt.kernels, "zero_slots") and state.is_cuda:
+                self.rt.kernels.zero_slots(state, tables.state_slots, tables.fresh)
+                continue
             slots = tables.state_slots.long()
             keep = (1 - tables.fresh).to(state.dtype).view(1, -1, *([1] * (state.dim() - 2)))
             state.index_copy_(1, slots, state.index_select(1, slots) * keep)

@@ -98,6 +98,7 @@ _SIGNATURES = {
     "roost_sample_count_tokens": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p],
     "roost_sample_prompt_bits": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "roost_sample_logprobs": [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
+    "roost_zero_slots": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_int, c_void_p],
     "roost_gemm_rows_supported": [c_int, c_int, c_int, c_int64, c_int64, c_int],
     "roost_gemm_rows": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64, c_int, c_int, c_void_p],
     "roost_gemm_simt": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64, c_int, c_int, c_void_p],
@@ -517,6 +518,15 @@ class KernelLibrary:
         self._call("roost_gemm_simt", _ptr(a), _ptr(w), _ptr(out), M, N, K, a.stride(0), w.stride(0), out.stride(0),
                    dtype_code(a.dtype), dtype_code(out_dtype), _stream())
         return out
+
+    def zero_slots(self, state: torch.Tensor, slots: torch.Tensor, fresh: torch.Tensor) -> None:
+        """``state`` [runs, slots, ...]: zeros in the slots of the rows with ``fresh`` set, in every run."""
+        _need(state, "state", state.dtype); _need(slots, "slots", torch.int32); _need(fresh, "fresh", torch.int32)
+        if slots.numel() != fresh.numel():
+            raise KernelError("zero_slots: slots and fresh differ in length")
+        size = state.element_size()
+        self._call("roost_zero_slots", _ptr(state), _ptr(slots), _ptr(fresh), slots.numel(), state.shape[0], state.stride(0) * size, state.stride(1) * size,
+                   state[0, 0].numel() * size, state.shape[1], _stream())
 
     def gemm_rows_supported(self, x: torch.Tensor, w: torch.Tensor, swiglu: bool = False) -> bool:
         """The product of the few rows of a decode step over weights that fit the processors' registers."""

@@ -26,7 +26,7 @@ namespace roost {
 constexpr int kRtChunkTokens = 64;
 
 template <typename T>
-__global__ void __launch_bounds__(128) retention_prepare_kernel(const T* __restrict__ u, int64_t ld, float* __restrict__ qk,
+__global__ void __launch_bounds__(128) retention_prepare_kernel(const T* u, int64_t ld, float* qk,
                                                                const double* __restrict__ inv_freq, const int32_t* __restrict__ positions,
                                                                int heads, int dim, int rot_dims, float k_scale, int act) {
   extern __shared__ float sm[];      // rot_dims/2 cosines, rot_dims/2 sines
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(128) retention_prepare_kernel(const T* __restr
   const T* row = u + (size_t)t * ld;
   float* dst = qk + (size_t)t * 2 * heads * dim;
   const int n = 2 * heads * dim;
-  for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
+  for (int idx = blockIdx.y * blockDim.x + threadIdx.x; idx < n; idx += gridDim.y * blockDim.x) {
     const int j = idx % dim;
     const float x = to_float(row[idx]);
     float y = act ? silu_f(x) : x;
@@ -231,7 +231,9 @@ extern "C" int roost_retention_prepare(const void* u, int64_t ld, float* qk, con
   if (tokens == 0) return ROOST_OK;
   const size_t smem = ((size_t)rot_dims + 2) * sizeof(float);
   if (smem > 48 * 1024) return fail(ROOST_ERR_UNSUPPORTED, "retention_prepare: a rotation of more than 12286 elements");
-  ROOST_DISPATCH_DTYPE(dtype, T, launch_kernel(retention_prepare_kernel<T>, dim3(tokens), dim3(128), smem, (cudaStream_t)stream, (const T*)u, ld, qk,
+  // a token's columns over as many blocks as fill the processors a few times (8 tokens of 1,024 columns by a block a token: 4.8 us)
+  const int pieces = (2 * heads * dim + 127) / 128, spread = 600 / tokens < 1 ? 1 : 600 / tokens;
+  ROOST_DISPATCH_DTYPE(dtype, T, launch_kernel(retention_prepare_kernel<T>, dim3(tokens, pieces < spread ? pieces : spread), dim3(128), smem, (cudaStream_t)stream, (const T*)u, ld, qk,
                                                inv_freq, positions, heads, dim, rot_dims, k_scale, act));
   return check_launch("retention_prepare");
 }

@@ -190,6 +190,16 @@ int roost_attention_decode_static(const void* q, void* out, const void* k_pool, 
                                   int q_heads, int kv_heads, int head_dim, int page_size, float scale, int window,
                                   roost_stream_t stream);
 
+/* Attention of one query token a row over at most kv_cap keys (roost_attention_rows_supported: groups of up to 16 query heads of 64 or 128 numbers, pages of
+ * 16, 32, 64, ... keys), bfloat16. A key's entry of (page, kv head, offset) starts at ((page * kv_heads + head) * page_size + offset) * entry from k_base, its
+ * value's from v_base. sigmoid 0: softmax, lens [tokens] the rows' keys, row t's pages from kv_indptr[t] (token_row null). sigmoid 1: weights
+ * sigmoid((q . k) scale - slopes[h] (p - j) + head_bias[h]), lens the tokens' positions, pages of row token_row[t]; out times sigmoid(gate) where a gate
+ * is given. A row without keys is not written. */
+int roost_attention_rows_supported(int tokens, int q_heads, int kv_heads, int head_dim, int page_size, int kv_cap, int sigmoid);
+int roost_attention_rows(const void* q, void* out, const void* k_base, const void* v_base, int entry, const int32_t* lens, const int32_t* token_row,
+                         const int32_t* kv_indptr, const int32_t* kv_indices, int tokens, int q_heads, int kv_heads, int head_dim, int page_size, float scale,
+                         int kv_cap, int sigmoid, const float* slopes, const float* head_bias, const void* gate, int64_t ld_gate, roost_stream_t stream);
+
 /* state [runs][n_slots][bytes] (strides run_bytes and slot_bytes): zeros where fresh[r] is not 0, in slot slots[r] of every run, for each of `rows` rows. A slot
  * outside 0 .. n_slots - 1 is skipped. */
 int roost_zero_slots(void* state, const int32_t* slots, const int32_t* fresh, int rows, int runs, int64_t run_bytes, int64_t slot_bytes, int64_t bytes, int n_slots,

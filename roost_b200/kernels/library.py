@@ -98,6 +98,9 @@ _SIGNATURES = {
     "roost_sample_count_tokens": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p],
     "roost_sample_prompt_bits": [c_void_p, c_void_p, c_int, c_int, c_void_p],
     "roost_sample_logprobs": [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
+    "roost_attention_rows_supported": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
+    "roost_attention_rows": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
+                             c_int, c_void_p, c_void_p, c_void_p, c_int64, c_void_p],
     "roost_zero_slots": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_int, c_void_p],
     "roost_gemm_rows_supported": [c_int, c_int, c_int, c_int64, c_int64, c_int],
     "roost_gemm_rows": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64, c_int, c_int, c_void_p],
@@ -517,6 +520,26 @@ class KernelLibrary:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
         self._call("roost_gemm_simt", _ptr(a), _ptr(w), _ptr(out), M, N, K, a.stride(0), w.stride(0), out.stride(0),
                    dtype_code(a.dtype), dtype_code(out_dtype), _stream())
+        return out
+
+    def attention_rows_supported(self, q: torch.Tensor, k_pool: torch.Tensor, kv_heads: int, kv_cap: int, sigmoid: bool = False) -> bool:
+        """One query token a row over short contexts: keys straight into registers, a cluster a (row, key/value head)."""
+        T, heads, dim = q.shape
+        return (q.dtype == torch.bfloat16 and q.data_ptr() % 16 == 0 and k_pool.data_ptr() % 16 == 0
+                and bool(self._lib.roost_attention_rows_supported(T, heads, kv_heads, dim, k_pool.shape[2], kv_cap, int(sigmoid))))
+
+    def attention_rows(self, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, kv_lens: torch.Tensor, kv_indptr: torch.Tensor, kv_indices: torch.Tensor,
+                       scale: float, kv_cap: int) -> torch.Tensor:
+        """softmax(q k^T scale) v of one token a row: [T, heads * dim]; ``kv_cap`` bounds the rows' keys."""
+        _need(q, "q", torch.bfloat16); _need(k_pool, "k_pool", torch.bfloat16); _need(v_pool, "v_pool", torch.bfloat16)
+        for n, t in (("kv_lens", kv_lens), ("kv_indptr", kv_indptr), ("kv_indices", kv_indices)):
+            _need(t, n, torch.int32)
+        T, heads, dim = q.shape
+        if kv_lens.numel() < T or kv_indptr.numel() < T + 1 or k_pool.shape[3] != dim or v_pool.shape != k_pool.shape:
+            raise KernelError("attention_rows: the tables or the pools do not fit the queries")
+        out = torch.empty((T, heads * dim), dtype=q.dtype, device=q.device)
+        self._call("roost_attention_rows", _ptr(q), _ptr(out), _ptr(k_pool), _ptr(v_pool), dim, _ptr(kv_lens), None, _ptr(kv_indptr), _ptr(kv_indices), T, heads,
+                   k_pool.shape[1], dim, k_pool.shape[2], float(scale), kv_cap, 0, None, None, None, 0, _stream())
         return out
 
     def zero_slots(self, state: torch.Tensor, slots: torch.Tensor, fresh: torch.Tensor) -> None:
@@ -1538,6 +1561,11 @@ class KernelLibrary:
             self._call("roost_sigmoid_attention_tc_chunks", _ptr(q), _ptr(out), kb, vb, k_pool.shape[0], gate_ptr, ld_gate, _ptr(slopes), _ptr(head_bias),
                        _ptr(q_indptr), _ptr(kv_lens), _ptr(kv_indptr), _ptr(kv_indices), T, rows, heads, kv_heads, dim, k_pool.shape[2], float(scale),
                        _ptr(positions), _ptr(sums), per, chunks, _stream(), launches=2 if chunks > 1 else 1)
+            return out
+        if (q_indptr is None and kv_cap and dim == vdim and entry % 8 == 0 and kb % 16 == 0 and vb % 16 == 0
+                and self.attention_rows_supported(q, k_pool, kv_heads, kv_cap, sigmoid=True)):
+            self._call("roost_attention_rows", _ptr(q), _ptr(out), kb, vb, entry, _ptr(positions), _ptr(token_row), _ptr(kv_indptr), _ptr(kv_indices), T, heads, kv_heads,
+                       dim, k_pool.shape[2], float(scale), kv_cap, 1, _ptr(slopes), _ptr(head_bias), gate_ptr, ld_gate, _stream())
             return out
         if q_indptr is not None and q.dtype == torch.bfloat16 and self.sigmoid_attention_mma_supported(dim, vdim, v_pool is not None):
             _need(q_indptr, "q_indptr", torch.int32)

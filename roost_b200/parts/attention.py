@@ -107,6 +107,9 @@ class PagedAttention(Mixer):
         s, k = self.spec, self.rt.kernels
         if q.dtype == torch.bfloat16 and getattr(k, "attention_mma_supported", lambda d: False)(s.head_dim):
             group = s.num_heads // s.num_kv_heads
+            if (s.window is None and batch.all_single and batch.kv_cap and hasattr(k, "attention_rows")
+                    and k.attention_rows_supported(q, cache.k_pool, s.num_kv_heads, batch.kv_cap)):
+                return k.attention_rows(q, cache.k_pool, cache.v_pool, batch.kv_lens, tables.kv_indptr, tables.kv_indices, s.scale, batch.kv_cap)
             tile_rows = k.attention_prefill_tile_rows(s.num_heads, cache.k_pool, cache.v_pool, batch.num_tokens * group)
             split_for = getattr(k, "decode_split_for", None)
             chunk, cluster = split_for(batch.num_rows, batch.kv_cap, cache.k_pool, cache.v_pool) if split_for and batch.kv_cap else (k.decode_chunk, 0)

@@ -42,7 +42,7 @@ __global__ void mamba2_conv_kernel(const T* __restrict__ u, int64_t ld, int col,
 }
 
 // Four taps, whole 16-byte pieces of channels everywhere: a thread takes one piece of TT consecutive tokens and keeps the inputs of the last
-// three, so that an input is read once. Bound by memory where a step has many tokens (4,096 x 6,144: 202 us a number at a time, 24 us here).
+// three, so that an input is read once. 4,096 x 6,144: 202 us a number at a time, 42 here (59 with the exact exponential and quotient; 100 MB).
 // The same sums in the same order as above.
 template <typename T, int TT>
 __global__ void __launch_bounds__(128) mamba2_conv_vec_kernel(const T* u, int64_t ld, int col, T* out, const float* __restrict__ w,
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(128) mamba2_conv_vec_kernel(const T* u, int64_
 #pragma unroll
       for (int i = 0; i < V; ++i) {
         const float acc = fmaf(wt[i].w, in[j][i], fmaf(wt[i].z, x[2][i], fmaf(wt[i].y, x[1][i], fmaf(wt[i].x, x[0][i], b[i]))));
-        o[i] = act ? silu_f(acc) : acc;
+        o[i] = act ? gated_f<T>(acc, acc) : acc;
         x[0][i] = x[1][i];
         x[1][i] = x[2][i];
         x[2][i] = in[j][i];
@@ -459,7 +459,8 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
       const float4 a = *reinterpret_cast<const float4*>(y + (size_t)t * inner + c0 + j);
       const uint2 q = *reinterpret_cast<const uint2*>(u + (size_t)t * ld_u + c0 + j);
       const float z[4] = {__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xffff0000u), __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xffff0000u)};
-      v[i][0] = a.x * silu_f(z[0]); v[i][1] = a.y * silu_f(z[1]); v[i][2] = a.z * silu_f(z[2]); v[i][3] = a.w * silu_f(z[3]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[i][e] = (e == 0 ? a.x : (e == 1 ? a.y : (e == 2 ? a.z : a.w))) * gated_f<__nv_bfloat16>(z[e], z[e]);
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) ss = fmaf(v[i][e], v[i][e], ss);
@@ -499,12 +500,12 @@ extern "C" int roost_mamba2_conv(const void* u, int64_t ld, int col, void* out, 
     if ((long long)tokens * channels >= kConvVecMin && (dtype == ROOST_F32 || dtype == ROOST_BF16) && taps == 4 && channels % vec == 0 && ld % vec == 0 && col % vec == 0 && at % 16 == 0 && state_stride % 4 == 0 &&
         conv_off % 4 == 0) {
       const unsigned gy = (unsigned)((channels / vec + 127) / 128);
-      // sixteen tokens a thread where that leaves every processor several blocks, else one; few numbers are spread over more threads by the form for
-      // any sizes
-      const bool many = (long long)(tokens / 16) * gy >= 4 * 148;
+      // sixteen or four tokens a thread where that leaves every processor several blocks, else one (whose weights are ten times what it reads and writes:
+      // 2,348 tokens x 2,048 channels 28 us, 12 with four); few numbers are spread over more threads by the form for any sizes
+      const int each = (long long)(tokens / 16) * gy >= 4 * 148 ? 16 : ((long long)(tokens / 4) * gy >= 2 * 148 ? 4 : 1);
       ROOST_DISPATCH_DTYPE(dtype, T, {
-        auto kernel = many ? mamba2_conv_vec_kernel<T, 16> : mamba2_conv_vec_kernel<T, 1>;
-        launch_kernel(kernel, dim3(many ? (tokens + 15) / 16 : tokens, gy), dim3(128), 0, (cudaStream_t)stream, (const T*)u, ld, col, (T*)out, w, bias, state,
+        auto kernel = each == 16 ? mamba2_conv_vec_kernel<T, 16> : (each == 4 ? mamba2_conv_vec_kernel<T, 4> : mamba2_conv_vec_kernel<T, 1>);
+        launch_kernel(kernel, dim3((tokens + each - 1) / each, gy), dim3(128), 0, (cudaStream_t)stream, (const T*)u, ld, col, (T*)out, w, bias, state,
                       state_stride, conv_off, token_row, q_indptr, slots, tokens, channels, act);
       });
       return check_launch("mamba2_conv");

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_vec_kernel(const float* o,
     float y[4] = {v[i].x * inv * ww.x, v[i].y * inv * ww.y, v[i].z * inv * ww.z, v[i].w * inv * ww.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      y[e] = y[e] / (1.0f + expf(-g[i][e]));
+      y[e] = gated_f<T>(y[e], g[i][e]);
       if (gate_silu) y[e] *= g[i][e];
     }
     T* to = out + row * vdim + j;

@@ -38,7 +38,7 @@ __global__ void mamba2_conv_kernel(const T* __restrict__ u, int64_t ld, int col,
     const float v = i >= start ? to_float(u[(size_t)i * ld + col + c]) : st[(size_t)(i - start + taps - 1) * channels + c];
     acc = fmaf(w[(size_t)c * taps + k], v, acc);
   }
-  out[(size_t)t * channels + c] = from_float<T>(act ? silu_f(acc) : acc);
+  out[(size_t)t * channels + c] = from_float<T>(act ? gated_f<T>(acc, acc) : acc);
 }
 
 // Four taps, whole 16-byte pieces of channels everywhere: a thread takes one piece of TT consecutive tokens and keeps the inputs of the last
@@ -424,7 +424,7 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const T* __
   float ss = 0.f;
   for (int i = threadIdx.x; i < gs; i += blockDim.x) {
     const int c = g * gs + i;
-    const float v = y[(size_t)t * inner + c] * silu_f(to_float(u[(size_t)t * ld_u + c]));
+    const float z = to_float(u[(size_t)t * ld_u + c]), v = y[(size_t)t * inner + c] * gated_f<T>(z, z);
     vals[i] = v;
     ss += v * v;
   }

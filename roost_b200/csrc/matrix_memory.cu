@@ -245,7 +245,7 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const T* __re
     for (int i = lane; i < vdim; i += 32) {
       const size_t c = (size_t)h * vdim + i;
       const float g = to_float(u[t * ld_u + col + c]);
-      const float y = x[i] * inv * (w != nullptr ? w[c] : 1.0f) / (1.0f + expf(-g));
+      const float y = gated_f<T>(x[i] * inv * (w != nullptr ? w[c] : 1.0f), g);
       out[t * heads * vdim + c] = from_float<T>(gate_silu ? y * g : y);
     }
   }
@@ -318,7 +318,7 @@ __global__ void row_norm_gate_kernel(const float* __restrict__ o, const T* __res
   const float inv = 1.0f / sqrtf(ss / (float)width + eps);
   for (int i = threadIdx.x; i < width; i += blockDim.x) {
     const float g = to_float(u[t * ld_u + col + i]);
-    const float y = x[i] * inv * (w != nullptr ? w[i] : 1.0f) / (1.0f + expf(-g));
+    const float y = gated_f<T>(x[i] * inv * (w != nullptr ? w[i] : 1.0f), g);
     out[t * width + i] = from_float<T>(gate_silu ? y * g : y);
   }
 }

@@ -44,8 +44,9 @@ __device__ __forceinline__ float ar_remote(const float* p, uint32_t rank) {
   return v;
 }
 __device__ __forceinline__ void ar_cluster_sync() { asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory"); }
-// 2^(a - b) for a <= b; 0 where nothing was seen (a = -inf)
-__device__ __forceinline__ float ar_fade(float a, float b) { return a > -INFINITY ? exp2f(a - b) : 0.f; }
+// What scores are taken relative to: their maximum, or 0 where there was none (no key, or none but -inf or NaN). Every weight is then exp2f of a difference: 0 for
+// -inf, NaN for a NaN score, which so reaches the sums, the denominator and the output whatever the maximum is.
+__device__ __forceinline__ float ar_base(float top) { return top == -INFINITY ? 0.f : top; }
 
 template <int D, bool SIGMOID>
 __global__ void __launch_bounds__(kArWarps * 32, 1) attention_rows_kernel(const AttentionRows a) {
@@ -147,13 +148,13 @@ __global__ void __launch_bounds__(kArWarps * 32, 1) attention_rows_kernel(const 
             }
           top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
           top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-          const float now = fmaxf(m[r], top), fade = ar_fade(m[r], now);
+          const float now = fmaxf(m[r], top), base = ar_base(now), fade = exp2f(m[r] - base);
           float sum = 0.f;
 #pragma unroll
           for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              s[h][2 * r + e] = ar_fade(s[h][2 * r + e], now);
+              s[h][2 * r + e] = exp2f(s[h][2 * r + e] - base);
               sum += s[h][2 * r + e];
             }
           l[r] = l[r] * fade + sum;               // of this lane's keys; the row's lanes are added at the end
@@ -216,9 +217,10 @@ __global__ void __launch_bounds__(kArWarps * 32, 1) attention_rows_kernel(const 
 #pragma unroll
         for (int w = 0; w < kArWarps; ++w) top = fmaxf(top, sml[(w * group + h) * 2]);
       }
+      const float base = ar_base(top);
 #pragma unroll
       for (int w = 0; w < kArWarps; ++w) {
-        const float f = SIGMOID ? 1.f : ar_fade(sml[(w * group + h) * 2], top);
+        const float f = SIGMOID ? 1.f : exp2f(sml[(w * group + h) * 2] - base);
         sum += so[(w * group + h) * LD + d] * f;
         den += sml[(w * group + h) * 2 + 1] * f;
       }
@@ -244,9 +246,10 @@ __global__ void __launch_bounds__(kArWarps * 32, 1) attention_rows_kernel(const 
         pl[z] = !SIGMOID && z < splits ? ar_remote(bml + h * 2 + 1, z) : 0.f;
         top = fmaxf(top, pm[z]);
       }
+      const float base = ar_base(top);
 #pragma unroll
       for (int z = 0; z < kArMaxSplits; ++z) {
-        const float f = SIGMOID ? 1.f : ar_fade(pm[z], top);
+        const float f = SIGMOID ? 1.f : exp2f(pm[z] - base);
         sum += part[z] * f;
         den += pl[z] * f;
       }
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(kArWarps * 32, 1) attention_rows_kernel(const 
       if constexpr (SIGMOID) {
         if (a.gate) y *= sigmoid_f(to_float(a.gate[(size_t)t * a.ld_gate + (size_t)(kvh * group + h) * D + d]));
       } else {
-        y = den > 0.f ? sum / den : 0.f;
+        y = den > 0.f ? sum / den : sum * 0.f;        // no weight at all: 0; a denominator of NaN: NaN, as the sum
       }
       a.out[head * D + d] = from_float<__nv_bfloat16>(y);
     }

@@ -92,3 +92,60 @@ def test_sigmoid(kernels, lens, heads, kv_heads, dim, two, gated):
             want, size = w @ x[:, dim:] * scale, w @ x[:, dim:].abs() * scale
             # 32-bit weights and sums (products cut off, 2^-23 of the sum each, at most 3 a block of 16 keys and warp), one rounding
             assert ((out[r, h * dim : (h + 1) * dim].double() - want).abs() <= (2.0 ** -20 + n / 16 * 3 * 2.0 ** -23) * size + 2.0 ** -8 * want.abs()).all(), (r, h)
+
+
+def _softmax_64(q, keys, values, heads, kv_heads):
+    """[rows, heads, dim] of softmax(q k^T / sqrt(dim)) v in 64 bits."""
+    out = torch.empty(q.shape, dtype=torch.float64, device="cuda")
+    for r in range(q.shape[0]):
+        for h in range(heads):
+            k, v = keys[r][:, h * kv_heads // heads].double(), values[r][:, h * kv_heads // heads].double()
+            out[r, h] = torch.softmax(k @ q[r, h].double() * q.shape[2] ** -0.5, 0) @ v
+    return out
+
+
+# one block of keys and one warp; a warp a block; several CTAs a row
+@pytest.mark.parametrize("lens", [[9, 16, 12, 10], [100, 128, 40, 90], [300, 1000, 700, 513]])
+@pytest.mark.parametrize("heads,kv_heads,dim", [(16, 4, 64), (16, 8, 128)])
+def test_a_score_that_is_not_finite_reaches_the_output(kernels, lens, heads, kv_heads, dim):
+    """A NaN score makes its row and head NaN, and so does one of +inf; -inf is a weight of zero. No other row or head sees them."""
+    page, group = 16, heads // kv_heads
+    k_pool, indptr, indices, keys = _cache(lens, kv_heads, page, dim, 1)
+    v_pool, values = k_pool * -1.5, [k * -1.5 for k in keys]
+    q = _rand((len(lens), heads, dim), 7)
+    starts = indptr.tolist()
+
+    def set_key(r, j, head, d, value):
+        keys[r][j, head, d] = value
+        k_pool[indices[starts[r] + j // page], head, j % page, d] = value
+
+    q[0, 1] = float("nan")                                     # every score of a head
+    set_key(1, 7, 1, 3, float("nan"))                          # a score of a group of heads
+    q[2, :, 5] = -q[2, :, 5].abs() - 0.1
+    set_key(2, 4, 0, 5, float("inf"))                          # a score of -inf
+    q[3, :, 5] = q[3, :, 5].abs() + 0.1
+    set_key(3, 8, 2, 5, float("inf"))                          # a score of +inf
+    cap = 1024
+    assert kernels.attention_rows_supported(q, k_pool, kv_heads, cap)
+    out = kernels.attention_rows(q, k_pool, v_pool, _i32(lens), indptr, indices, dim ** -0.5, cap).reshape(len(lens), heads, dim)
+    want = _softmax_64(q, keys, values, heads, kv_heads)
+    assert torch.equal(torch.isnan(out), torch.isnan(want))
+    assert torch.isnan(want[0, 1]).all() and torch.isnan(want[1, group : 2 * group]).all() and not torch.isnan(want[2]).any() and torch.isnan(want[3, 2 * group]).all()
+    fine = torch.isfinite(want)
+    # as above; what |v| a weight meets is below 8 here
+    assert ((out.double() - want).abs()[fine] <= 2.0 ** -15 * 8 + 2.0 ** -8 * want.abs()[fine]).all()
+
+
+@pytest.mark.parametrize("lens", [[9, 16], [300, 1000]])
+def test_a_sigmoid_weight_that_is_not_a_number_reaches_the_output(kernels, lens):
+    heads, kv_heads, dim, page = 8, 4, 64, 16
+    k_pool, indptr, indices, _ = _cache(lens, kv_heads, page, dim, 1)
+    v_pool = k_pool * -1.5
+    q, T = _rand((len(lens), heads, dim), 7), len(lens)
+    q[0, 3] = float("nan")
+    k_pool[indices[indptr[1]], 1, 2, 9] = float("nan")          # key 2 of row 1, head 1
+    out = kernels.sigmoid_attention(q, k_pool, v_pool, None, None, torch.zeros(heads, device="cuda"), torch.zeros(heads, device="cuda"), _i32([n - 1 for n in lens]),
+                                    _i32(list(range(T))), indptr, indices, kv_heads, dim, dim ** -0.5, kv_cap=1024).reshape(T, heads, dim)
+    want = torch.zeros((T, heads), dtype=torch.bool, device="cuda")
+    want[0, 3], want[1, 2:4] = True, True
+    assert torch.equal(torch.isnan(out), want[:, :, None].expand_as(out))

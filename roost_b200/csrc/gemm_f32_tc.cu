@@ -9,7 +9,7 @@
 // parts, each a chain of such additions of its own, and the parts are added in order. What an output's bits depend on is therefore its
 // row of a, its row of w and k; not m, n, the tile, or which of the forms below ran.
 // A result that is not finite (an operand that is not, or whose bf16 rounding overflows, or sums that do) is formed once more as a chain of
-// FFMAs over k, so infinities and NaN come out where they do there.
+// FFMAs over k when the CTA's tiles are done, so infinities and NaN come out where they do there.
 //
 // Roles of a CTA, which owns a tile of 128 rows of w by NT rows of a (the accumulator lies transposed: a lane of tensor memory is a
 // row of w, so that a warp's stores are 128 consecutive bytes of out):
@@ -107,12 +107,42 @@ __device__ __forceinline__ float4 load16(uint32_t addr) {
   return v;
 }
 
-__device__ __forceinline__ float ffma_chain(const float* a, const float* w, int K) {
-  float s = 0.f;
-  for (int k = 0; k < K; ++k) s = fmaf(a[k], w[k], s);
-  return s;
-}
 __device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7F800000u) != 0x7F800000u; }
+
+// The outputs of rows m0 .. m1 - 1 of a and n0 .. n1 - 1 of w that are not finite, formed once more as chains of FFMAs over k. By all threads of a CTA when its
+// tiles are done: inside the pipeline the roles that wait for one another with a limit would wait for it. A lane a row of w, eight rows of a at a time, so
+// that a piece of w is read once for eight chains.
+template <int THREADS>
+__device__ __forceinline__ void redo_not_finite(const float* a, const float* w, float* out, int m0, int m1, int n0, int n1, int K, int64_t lda, int64_t ldw, int64_t ldo) {
+  const int width = (n1 - n0 + 31) / 32 * 32, tasks = (m1 - m0 + 7) / 8 * width;      // whole warps
+  for (int idx = threadIdx.x; idx < tasks; idx += THREADS) {
+    const int n = n0 + idx % width, m = m0 + idx / width * 8;
+    unsigned need = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (n < n1 && m + i < m1 && !finite(out[(int64_t)(m + i) * ldo + n])) need |= 1u << i;
+    const unsigned any = __reduce_or_sync(0xffffffffu, need);
+    if (any == 0) continue;
+    const float* wr = w + (int64_t)min(n, n1 - 1) * ldw;
+    const float* ar = a + (int64_t)m * lda;
+    float s[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = 0.f;
+    for (int k = 0; k < K; k += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(wr + k);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (any >> i & 1) {
+          const float* p = ar + i * lda + k;
+          s[i] = fmaf(p[3], v.w, fmaf(p[2], v.z, fmaf(p[1], v.y, fmaf(p[0], v.x, s[i]))));
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (need >> i & 1) out[(int64_t)(m + i) * ldo + n] = s[i];
+  }
+}
 
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t rank) {
   uint32_t remote;
@@ -146,7 +176,7 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
   float* red = reinterpret_cast<float*>(smem_raw + (base - raw));          // [NT][128], over the stages (CL)
   __shared__ __align__(8) uint64_t bars[2 * C::kStages + 4 + 2 * R];
   __shared__ uint32_t tmem_slot;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, redo_flag;       // redo: an output of this CTA is not finite
   const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
   auto full = [&](int s) { return bar0 + 8u * s; };
   auto empty = [&](int s) { return bar0 + 8u * (C::kStages + s); };
@@ -158,6 +188,7 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
   constexpr int kProducer = C::kThreads / 32 - 3, kIssuer = kProducer + 1;      // two issuers
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    redo_flag = 0;
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(full(s), 4);
       mbar_init(empty(s), 1);
@@ -353,7 +384,7 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
 #pragma unroll
           for (int j = 0; j < C::kColumns; ++j) {
             if (m0 + j < M) {
-              if (!finite(acc[j])) acc[j] = ffma_chain(a + (int64_t)(m0 + j) * lda, w + (int64_t)n * ldw, K);
+              if (!finite(acc[j])) redo_flag = 1;
               out[(int64_t)(m0 + j) * ldo + n] = acc[j];
             }
           }
@@ -377,7 +408,7 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
 #pragma unroll
         for (int p = 1; p < kParts; ++p) sum += v[p];
         if (n < N) {
-          if (!finite(sum)) sum = ffma_chain(a + (int64_t)(m0 + m) * lda, w + (int64_t)n * ldw, K);
+          if (!finite(sum)) redo_flag = 1;
           out[(int64_t)(m0 + m) * ldo + n] = sum;
         }
       }
@@ -393,6 +424,12 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
   if (warp == kIssuer) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(C::kTmem) : "memory");
+  }
+  if (redo_flag && !*abortp) {
+    for (int t = first; t < tiles; t += step) {
+      const int m0 = t % m_tiles * NT, n0 = t / m_tiles * pitch + (CL ? rank * (kWRows / kParts) : 0);
+      if (n0 < N) redo_not_finite<C::kThreads>(a, w, out, m0, min(m0 + NT, M), n0, min(n0 + (CL ? kWRows / kParts : pitch), N), K, lda, ldw, ldo);
+    }
   }
 }
 

@@ -60,3 +60,20 @@ def test_what_is_not_finite_comes_out_as_a_chain_of_sums_has_it(kernels):
     fine = torch.isfinite(want)
     assert ((got.double() - want).abs()[fine] <= _bound(a, w).nan_to_num(0.0, 0.0)[fine] + 2.0 ** -20 * want.abs()[fine]).all()
     assert got[9, 0].item() == pytest.approx(0.85e38, rel=1e-5) and torch.isfinite(clean).all()
+
+
+def test_rows_that_are_not_finite_do_not_hold_up_the_other_tiles(kernels):
+    """Half the rows of every tile NaN, several tiles a CTA and a long reduction: the chains of FFMAs that those outputs become run when nobody waits for them, and
+    what is finite is what it is without them."""
+    m, n, k = 1920, 1280, 24576
+    a, w = _rand((m, k), 11), _rand((n, k), 12)
+    clean = kernels.gemm_simt(a, w)
+    bad = torch.arange(m, device="cuda") % 2 == 1
+    a[bad, 3] = float("nan")
+    w[7, 100] = float("inf")
+    got = kernels.gemm_simt(a, w)
+    assert kernels._lib.roost_gemm_tcgen05_status() == 0
+    assert torch.isnan(got[bad]).all()
+    others = torch.arange(n, device="cuda") != 7
+    assert torch.equal(got[~bad][:, others], clean[~bad][:, others])
+    assert torch.equal(got[~bad][:, 7], torch.where(a[~bad, 100] > 0, float("inf"), float("-inf")))

@@ -134,13 +134,6 @@ __device__ __forceinline__ float exp_nearest(float x) {
 
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-// y sigmoid(z) for results of type T. What is rounded to bfloat16 right away takes the quick exponential and quotient: their relative error, below 2^-16 for
-// any z above -87 (below it the result, less than 2^-119 of y, is zero), is 2^-7 of that rounding's, and they take 6 instructions where the others take 25 (a
-// convolution of 25 M numbers was bound by them).
-template <typename T>
-__device__ __forceinline__ float gated_f(float y, float z) {
-  return sizeof(T) == 2 ? __fdividef(y, 1.0f + __expf(-z)) : y / (1.0f + expf(-z));
-}
 
 __device__ __forceinline__ float gelu_tanh_f(float z) { return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))); }
 

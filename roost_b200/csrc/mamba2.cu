@@ -38,11 +38,11 @@ __global__ void mamba2_conv_kernel(const T* __restrict__ u, int64_t ld, int col,
     const float v = i >= start ? to_float(u[(size_t)i * ld + col + c]) : st[(size_t)(i - start + taps - 1) * channels + c];
     acc = fmaf(w[(size_t)c * taps + k], v, acc);
   }
-  out[(size_t)t * channels + c] = from_float<T>(act ? gated_f<T>(acc, acc) : acc);
+  out[(size_t)t * channels + c] = from_float<T>(act ? silu_f(acc) : acc);
 }
 
 // Four taps, whole 16-byte pieces of channels everywhere: a thread takes one piece of TT consecutive tokens and keeps the inputs of the last
-// three, so that an input is read once. 4,096 x 6,144: 202 us a number at a time, 42 here (59 with the exact exponential and quotient; 100 MB).
+// three, so that an input is read once. 4,096 x 6,144: 202 us a number at a time, 59 here, most of it the 25 instructions of an exponential and a quotient a number (100 MB).
 // The same sums in the same order as above.
 template <typename T, int TT>
 __global__ void __launch_bounds__(128) mamba2_conv_vec_kernel(const T* u, int64_t ld, int col, T* out, const float* __restrict__ w,
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(128) mamba2_conv_vec_kernel(const T* u, int64_
 #pragma unroll
       for (int i = 0; i < V; ++i) {
         const float acc = fmaf(wt[i].w, in[j][i], fmaf(wt[i].z, x[2][i], fmaf(wt[i].y, x[1][i], fmaf(wt[i].x, x[0][i], b[i]))));
-        o[i] = act ? gated_f<T>(acc, acc) : acc;
+        o[i] = act ? silu_f(acc) : acc;
         x[0][i] = x[1][i];
         x[1][i] = x[2][i];
         x[2][i] = in[j][i];
@@ -424,7 +424,7 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const T* __
   float ss = 0.f;
   for (int i = threadIdx.x; i < gs; i += blockDim.x) {
     const int c = g * gs + i;
-    const float z = to_float(u[(size_t)t * ld_u + c]), v = y[(size_t)t * inner + c] * gated_f<T>(z, z);
+    const float v = y[(size_t)t * inner + c] * silu_f(to_float(u[(size_t)t * ld_u + c]));
     vals[i] = v;
     ss += v * v;
   }
@@ -459,8 +459,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
       const float4 a = *reinterpret_cast<const float4*>(y + (size_t)t * inner + c0 + j);
       const uint2 q = *reinterpret_cast<const uint2*>(u + (size_t)t * ld_u + c0 + j);
       const float z[4] = {__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xffff0000u), __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xffff0000u)};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[i][e] = (e == 0 ? a.x : (e == 1 ? a.y : (e == 2 ? a.z : a.w))) * gated_f<__nv_bfloat16>(z[e], z[e]);
+      v[i][0] = a.x * silu_f(z[0]); v[i][1] = a.y * silu_f(z[1]); v[i][2] = a.z * silu_f(z[2]); v[i][3] = a.w * silu_f(z[3]);
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) ss = fmaf(v[i][e], v[i][e], ss);

@@ -245,7 +245,7 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const T* __re
     for (int i = lane; i < vdim; i += 32) {
       const size_t c = (size_t)h * vdim + i;
       const float g = to_float(u[t * ld_u + col + c]);
-      const float y = gated_f<T>(x[i] * inv * (w != nullptr ? w[c] : 1.0f), g);
+      const float y = x[i] * inv * (w != nullptr ? w[c] : 1.0f) / (1.0f + expf(-g));
       out[t * heads * vdim + c] = from_float<T>(gate_silu ? y * g : y);
     }
   }
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_vec_kernel(const float* o,
     float y[4] = {v[i].x * inv * ww.x, v[i].y * inv * ww.y, v[i].z * inv * ww.z, v[i].w * inv * ww.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      y[e] = gated_f<T>(y[e], g[i][e]);
+      y[e] = y[e] / (1.0f + expf(-g[i][e]));
       if (gate_silu) y[e] *= g[i][e];
     }
     T* to = out + row * vdim + j;
@@ -318,7 +318,7 @@ __global__ void row_norm_gate_kernel(const float* __restrict__ o, const T* __res
   const float inv = 1.0f / sqrtf(ss / (float)width + eps);
   for (int i = threadIdx.x; i < width; i += blockDim.x) {
     const float g = to_float(u[t * ld_u + col + i]);
-    const float y = gated_f<T>(x[i] * inv * (w != nullptr ? w[i] : 1.0f), g);
+    const float y = x[i] * inv * (w != nullptr ? w[i] : 1.0f) / (1.0f + expf(-g));
     out[t * width + i] = from_float<T>(gate_silu ? y * g : y);
   }
 }

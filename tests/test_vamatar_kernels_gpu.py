@@ -402,6 +402,49 @@ def test_convolution_forms_agree_bit_for_bit(kernels, dtype, lengths, channels):
     assert torch.equal(kernels.mamba2_conv(u, 8, *args), kernels.mamba2_conv(shifted, 9, *args))
 
 
+GATES = (-88.0, -87.5, -87.0, -60.0, -20.0, -1.0)      # exp(88) is still a number, and so is what a gate of -88 leaves
+# one rounding of the result; the 32-bit gate itself, below the smallest normal number, is a multiple of 2^-149
+FAR_BELOW_ZERO = {torch.bfloat16: 2.0 ** -8, torch.float32: 2.0 ** -19}
+
+
+def within_a_rounding(got, want, dtype):
+    assert ((got.double() - want).abs() <= FAR_BELOW_ZERO[dtype] * want.abs()).all() and (got != 0).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens,channels", [(7, 24), (600, 1032), (1100, 1032), (5000, 1032)])
+def test_the_convolution_of_sums_far_below_zero(kernels, dtype, tokens, channels):
+    bias = torch.tensor(GATES).repeat(-(-channels // 6))[:channels].cuda()
+    u, w = torch.zeros(tokens, channels, dtype=dtype, device="cuda"), torch.zeros(channels, 4, device="cuda")
+    state, one = torch.zeros(1, 3 * channels, device="cuda"), torch.zeros(tokens, dtype=torch.int32, device="cuda")
+    q_indptr, slots = torch.tensor([0, tokens], dtype=torch.int32).cuda(), one[:1].contiguous()
+    got = kernels.mamba2_conv(u, 0, channels, w, bias, state, 0, one, q_indptr, slots)
+    z = bias.double()
+    within_a_rounding(got, (z / (1.0 + torch.exp(-z))).expand_as(got), dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens,heads,vdim", [(9, 1, 96), (9, 4, 30), (9, 4, 96)])      # a row a block, a number a lane, a head a warp
+@pytest.mark.parametrize("gate", ["sigmoid", "silu"])
+def test_the_head_norm_behind_gates_far_below_zero(kernels, dtype, tokens, heads, vdim, gate):
+    width = heads * vdim
+    g = torch.tensor(GATES).repeat(width)[:width].expand(tokens, width)
+    o, w = torch.ones(tokens, width, device="cuda"), torch.full((width,), 1e25, device="cuda")
+    got = kernels.head_norm_gate(o, g.to(dtype).cuda(), 0, w, heads, 1e-12, dtype, gate=gate)
+    z = g.double().cuda()
+    within_a_rounding(got, float(torch.tensor(1e25)) / (1.0 + torch.exp(-z)) * (z if gate == "silu" else 1.0), dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens,size", [(5, 30), (5, 96), (1536, 96)])                  # a number at a time, a group a block, a group a warp
+def test_the_gated_norm_behind_gates_far_below_zero(kernels, dtype, tokens, size):
+    z = torch.tensor([-88.0, -87.5]).repeat(size)[:size].expand(tokens, size)
+    y, w = torch.full((tokens, size), 1e36, device="cuda"), torch.ones(size, device="cuda")
+    got = kernels.gated_group_norm(y, z.to(dtype).cuda(), w, 1, 1e-12, dtype)
+    v = (float(torch.tensor(1e36)) * z.double() / (1.0 + torch.exp(-z.double()))).cuda()
+    within_a_rounding(got, v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-12), dtype)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("tokens", [5, 1536])        # a group a block, a group a warp
 @pytest.mark.parametrize("size,groups", [(4, 3), (36, 2), (256, 2), (512, 8), (1024, 1), (1028, 3), (2048, 1), (4100, 1), (8192, 1), (8196, 1), (50, 1)])

@@ -236,14 +236,12 @@ __global__ void __launch_bounds__(192, 1)
 // expert each (tile_list: (expert, first row, one past the last row) triples, expert -1 for the unused tail of the list);
 // w holds the experts' matrices one after the other ([experts * N, K], so expert e's rows start at e * N). A tile of a is
 // loaded from its first row whatever that is (rows beyond the expert's are computed and not stored); a tile of w that runs
-// past the expert's N rows reads the next expert's and those columns are not stored either. The CTAs that run at once take few experts, whose rows and
-// weights so come from memory once, and the two that share a tile of w take it together (all rows for one n after the other read the rows again for every
-// n and brought 636 MB for 452: 64 experts of 192 rows by 1,536 x 2,048 137 us, 120 so, of 256 rows 140 and 111). Everything else is the kernel
-// above: the same roles, stages, accumulators, epilogues and bounded waits.
+// past the expert's N rows reads the next expert's and those columns are not stored either. `run` entries of the list are taken together (grouped_run). Everything
+// else is the kernel above: the same roles, stages, accumulators, epilogues and bounded waits.
 template <typename TOut, int EPI>
 __global__ void __launch_bounds__(192, 1)
     gemm_tcgen05_grouped_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, TOut* __restrict__ out,
-                                const int32_t* __restrict__ tile_list, int m_tiles, int N, int K, int64_t ldo, int act, float limit) {
+                                const int32_t* __restrict__ tile_list, int m_tiles, int run, int N, int K, int64_t ldo, int act, float limit) {
   extern __shared__ unsigned char smem_raw[];
   // tiles want 1024-byte alignment (the swizzle pattern repeats every 1024 bytes)
   const uint32_t smem_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023u) & ~1023u;
@@ -283,10 +281,10 @@ __global__ void __launch_bounds__(192, 1)
 
   const int n_tiles = (N + BN - 1) / BN;
   const int k_blocks = (K + BK - 1) / BK;
-  const int tiles = (m_tiles + 1) / 2 * 2 * n_tiles;
-  // tile t: a pair of neighbouring entries of the list after the other, in it the tiles of w in turn, both entries with each
-  auto m_of = [&](int t) { return t / (2 * n_tiles) * 2 + (t & 1); };
-  auto n_of = [&](int t) { return t % (2 * n_tiles) / 2 * BN; };
+  const int tiles = (m_tiles + run - 1) / run * run * n_tiles;
+  // tile t: `run` neighbouring entries of the list after the others, in them the tiles of w in turn, every entry with each
+  auto m_of = [&](int t) { return t / (run * n_tiles) * run + t % run; };
+  auto n_of = [&](int t) { return t % (run * n_tiles) / run * BN; };
   auto expert_of = [&](int t) { return m_of(t) < m_tiles ? tile_list[3 * m_of(t)] : -1; };
 
   if (warp == 0) {
@@ -1287,9 +1285,22 @@ extern "C" int roost_gemm_tcgen05_status(void) {
   return code;
 }
 
+// Entries of the list that take the tiles of w together. Two: the CTAs that run at once then take few experts, whose rows and weights so come from memory
+// once, and the two entries of an expert share a tile of w (all entries for one n after the other read the rows again for every n and brought 636 MB for
+// 452). Products of 1,536 x 2,048, us, all entries / two: 64 experts of 48 rows 108 / 96, 96 rows 103 / 98, 128 rows 118 / 103, 256 rows 140 / 111; 128 experts of
+// 16 rows 165 / 160, 64 rows 184 / 166, 128 rows 201 / 163, 160 rows 251 / 216.
+// All of them, where a CTA's next entry then lies a few before its last: the entries without rows pass over all CTAs in turn, their reads of the weights do not
+// stay in step, and experts of few rows, which wait for nothing else, are faster: 64 experts of 24 rows (76 entries, 148 processors) 91 / 94, of 28 rows 92 / 95; 128
+// experts of 24 and 28 rows 150 / 163. With 12 and 10 entries it is 94 / 95 and 144 / 140 (64 experts of 32 rows; 60 of 40 by 2,816 x 2,048); with none, where the
+// same CTAs meet the empty entries every time, 183 / 161 and 181 / 139 (128 experts of 20 rows, 60 of 28).
+static int grouped_run(int rows, int experts, int m_tiles, int sms) {
+  const int back = (sms + m_tiles - 1) / m_tiles * m_tiles - sms;
+  return rows <= 32LL * experts && back >= 2 && back <= 8 ? m_tiles : 2;
+}
+
 template <int EPI>
-static int launch_tcgen05_grouped(const CUtensorMap& ma, const CUtensorMap& mb, void* out, const int32_t* tile_list, int m_tiles, int n, int k,
-                                  int64_t ldo, int act, float limit, cudaStream_t s) {
+static int launch_tcgen05_grouped(const CUtensorMap& ma, const CUtensorMap& mb, void* out, const int32_t* tile_list, int m_tiles, int rows, int experts, int n,
+                                  int k, int64_t ldo, int act, float limit, cudaStream_t s) {
   static int sms = 0;
   static bool attr_set = false;
   const size_t smem = (size_t)STAGES * kStageBytes + 1024;
@@ -1301,9 +1312,10 @@ static int launch_tcgen05_grouped(const CUtensorMap& ma, const CUtensorMap& mb, 
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr_set = true;
   }
-  const long long tiles = (long long)((m_tiles + 1) / 2 * 2) * ((n + BN - 1) / BN);
+  const int run = grouped_run(rows, experts, m_tiles, sms);
+  const long long tiles = (long long)((m_tiles + run - 1) / run) * run * ((n + BN - 1) / BN);
   const int grid = tiles < sms ? (int)tiles : sms;
-  kernel<<<grid, 192, smem, s>>>(ma, mb, (__nv_bfloat16*)out, tile_list, m_tiles, n, k, ldo, act, limit);
+  kernel<<<grid, 192, smem, s>>>(ma, mb, (__nv_bfloat16*)out, tile_list, m_tiles, run, n, k, ldo, act, limit);
   return check_launch("gemm_tcgen05_grouped");
 }
 
@@ -1324,8 +1336,8 @@ extern "C" int roost_gemm_tcgen05_grouped(const void* a, const void* w, void* ou
   rc = make_map(&mb, w, experts * n, k, k, BN);
   if (rc != ROOST_OK) return rc;
   ROOST_REQUIRE(act >= ROOST_ACT_SILU && act <= ROOST_ACT_CLAMPED_SWISH, "gemm_tcgen05_grouped: unknown gate function");
-  if (swiglu) return launch_tcgen05_grouped<1>(ma, mb, out, tile_list, m_tiles, n, k, n / 2, act, limit, (cudaStream_t)stream);
-  return launch_tcgen05_grouped<0>(ma, mb, out, tile_list, m_tiles, n, k, n, act, limit, (cudaStream_t)stream);
+  if (swiglu) return launch_tcgen05_grouped<1>(ma, mb, out, tile_list, m_tiles, rows, experts, n, k, n / 2, act, limit, (cudaStream_t)stream);
+  return launch_tcgen05_grouped<0>(ma, mb, out, tile_list, m_tiles, rows, experts, n, k, n, act, limit, (cudaStream_t)stream);
 }
 
 extern "C" int roost_gemm_tcgen05(const void* a, const void* w, void* out, int m, int n, int k, int64_t lda, int64_t ldw, int64_t ldo,

@@ -384,6 +384,31 @@ def test_recurrence_in_chunks_on_the_tensor_cores(kernels, H, N, groups, lengths
         assert off[torch.bfloat16] < max(1.1 * off[torch.float32], 2.0 ** -23), (name, off)
 
 
+# lists of 76, 77, 78 entries (all of them take a tile of w together on 148 processors), of 75, 79 and 81 (two do, a last one by itself), 128 + 24
+@pytest.mark.parametrize("E,T,top", [(64, 256, 6), (64, 266, 6), (64, 290, 6), (64, 220, 6), (64, 320, 6), (64, 350, 6), (128, 380, 8), (16, 80, 16)])
+@pytest.mark.parametrize("n", [256, 768, 520])
+def test_every_order_of_the_grouped_product_takes_every_tile(kernels, E, T, top, n):
+    hidden = 64
+    g = torch.Generator().manual_seed(T)
+    logits = torch.randn(T, E, generator=g)
+    logits[:, 3] -= 20.0                                    # an expert without rows
+    if E < 128:
+        logits[: T // 2, 5] += 20.0                         # and one of several tiles
+    route = kernels.moe_route(logits.cuda(), top)
+    assert route.wide_tiles is not None
+    x, w = torch.randn(route.rows, hidden, generator=g).to(torch.bfloat16).cuda(), (torch.randn(E, n, hidden, generator=g) * 0.15).to(torch.bfloat16).cuda()
+    want = torch.empty((route.rows, n), dtype=torch.float64, device="cuda")
+    for e in range(E):
+        mine = route.expert == e
+        want[mine] = x[mine].double() @ w[e].double().T
+    assert ((kernels._moe_gemm_tcgen05(x, w, route, False).double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16).all()
+    if n % 256 == 0:
+        gate, up = want.reshape(route.rows, n // 256, 2, 128).unbind(2)
+        act = (gate / (1.0 + torch.exp(-gate)) * up).reshape(route.rows, n // 2)
+        assert ((kernels._moe_gemm_tcgen05(x, w, route, True).double() - act).abs() <= 2.0 ** -8 * act.abs() + 2.0 ** -16).all()
+    kernels.check_device_status()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("lengths,channels", [([1, 2, 3, 4, 37], 24), ([600, 1, 2, 3, 414], 1032), ([3000, 1, 2000], 1032)])
 def test_convolution_forms_agree_bit_for_bit(kernels, dtype, lengths, channels):

@@ -3,12 +3,13 @@
 // (TransposeB, Alpha 1, no bias).
 //
 // Every operand x is written as three bfloat16 numbers, h nearest to x, m what x - h has in eight bits, l = x - h - m: all 24 bits of a
-// float32. Six of the nine products of the parts are formed (l h, h l, m m, m h, h m, h h; the three left out are below 2^-24 of the
-// result's terms, of either sign), the small ones first. The tensor cores cut the running sum of a chain of products off instead
+// float32. Both operands are taken times 2^24 first and the sums times 2^-48 last, which changes no bit of either but leaves the parts of the smallest numbers
+// within bfloat16's range. Six of the nine products of the parts are formed (l h, h l, m m, m h, h m, h h; m l and l m, which are left out, are each below 2^-24 of
+// their term and of one sign, l l is below 2^-32), the small ones first. The tensor cores cut the running sum of a chain of products off instead
 // of rounding it, so a chain ends after 32 k: its sum leaves tensor memory and is added in float32, to nearest. k is cut into four
 // parts, each a chain of such additions of its own, and the parts are added in order. What an output's bits depend on is therefore its
 // row of a, its row of w and k; not m, n, the tile, or which of the forms below ran.
-// A result that is not finite (an operand that is not, or whose bf16 rounding overflows, or sums that do) is formed once more as a chain of
+// A sum that is not finite (an operand that is not, or is above 2^104, or sums above 2^80) is formed once more as a chain of
 // FFMAs over k when the CTA's tiles are done, so infinities and NaN come out where they do there.
 //
 // Roles of a CTA, which owns a tile of 128 rows of w by NT rows of a (the accumulator lies transposed: a lane of tensor memory is a
@@ -24,7 +25,7 @@
 // Forms: whole tiles by persistent CTAs, or (CL) a cluster of four CTAs a tile, CTA r taking the r-th part of k and the sums meeting in
 // distributed shared memory, for products of few tiles.
 // What bounds it: the products, of which none takes less than 64 cycles (72 with these tiles, about 90 beside the converters' traffic), so a block's twelve
-// 1,080; their floor at NT 96 is 580. 2,048 x 4,096 x 4,096: 431 us, 159 TFLOP/s of 32-bit products (1,527 us by FFMAs). A row of `a` that does not
+// 1,080; their floor at NT 96 is 580. 2,048 x 4,096 x 4,096: 439 us, 157 TFLOP/s of 32-bit products (1,527 us by FFMAs). A row of `a` that does not
 // start on 16 bytes is read by the converters an element at a time.
 #include "tcgen05.cuh"
 
@@ -38,6 +39,8 @@ constexpr int kBlock = 32;                                 // k of a stage and o
 constexpr int kParts = 4;
 constexpr int kWRows = 128;
 constexpr int kConverters = 256;                           // two groups of four warps, which take the blocks in turn
+constexpr float kScale = 16777216.0f;                      // 2^24, of both operands: the last bit of the smallest float32 becomes 2^-125, a bfloat16 number
+constexpr float kUnscale = 1.0f / (kScale * kScale);
 constexpr uint32_t kWRaw = kWRows * kBlock * 4;            // bytes of a block of w in float32
 constexpr uint32_t kWColumns = 3 * kBlock / 2;             // tensor-memory columns of a block of w: three planes, two numbers a column
 
@@ -68,20 +71,32 @@ __device__ __forceinline__ uint64_t desc_k_major_sw64(uint32_t addr) {
 __device__ __forceinline__ void store8(uint32_t addr, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
-// Four numbers as their three parts, packed in pairs: p[part][0] the first two, p[part][1] the others. With integer additions and masks: conversion
-// instructions keep the special-function pipe at two thirds of its rate, and splitting by three additions of floats was 3 % slower.
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
+  uint64_t p;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(p) : "f"(lo), "f"(hi));
+  return p;
+}
+__device__ __forceinline__ void bits_of(uint64_t p, uint32_t& lo, uint32_t& hi) { asm("mov.b64 {%0, %1}, %2;\n" : "=r"(lo), "=r"(hi) : "l"(p)); }
+// Four numbers times kScale as their three parts, packed in pairs: p[part][0] the first two, p[part][1] the others. With integer additions and masks: conversion
+// instructions keep the special-function pipe at two thirds of its rate, and splitting by three additions of floats was 3 % slower. The scaling and the
+// differences take two numbers an instruction: 2,048 x 4,096 x 4,096 439 us, 451 with one, 437 without the scaling.
 __device__ __forceinline__ void split4(float4 v, uint32_t (&p)[3][2]) {
-  float x[4] = {v.x, v.y, v.z, v.w};
-  uint32_t b[4];
+  const uint64_t scale = pair_of(kScale, kScale), minus = pair_of(-1.0f, -1.0f);
+  uint64_t x[2] = {pair_of(v.x, v.y), pair_of(v.z, v.w)};
+  asm("mul.rn.f32x2 %0, %0, %1;\n" : "+l"(x[0]) : "l"(scale));
+  asm("mul.rn.f32x2 %0, %0, %1;\n" : "+l"(x[1]) : "l"(scale));
 #pragma unroll
   for (int part = 0; part < 3; ++part) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) b[i] = __float_as_uint(x[i]) + (part == 0 ? 0x8000u : 0u);      // h to nearest; m cut off; l is whole
-    p[part][0] = __byte_perm(b[0], b[1], 0x7632);
-    p[part][1] = __byte_perm(b[2], b[3], 0x7632);
-    if (part < 2) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] -= __uint_as_float(b[i] & 0xFFFF0000u);
+    for (int i = 0; i < 2; ++i) {
+      uint32_t b0, b1;
+      bits_of(x[i], b0, b1);
+      if (part == 0) { b0 += 0x8000u; b1 += 0x8000u; }      // h to nearest; m cut off; l is whole
+      p[part][i] = __byte_perm(b0, b1, 0x7632);
+      if (part < 2) {
+        const uint64_t h = pair_of(__uint_as_float(b0 & 0xFFFF0000u), __uint_as_float(b1 & 0xFFFF0000u));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(x[i]) : "l"(h), "l"(minus));
+      }
     }
   }
 }
@@ -385,7 +400,7 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
           for (int j = 0; j < C::kColumns; ++j) {
             if (m0 + j < M) {
               if (!finite(acc[j])) redo_flag = 1;
-              out[(int64_t)(m0 + j) * ldo + n] = acc[j];
+              out[(int64_t)(m0 + j) * ldo + n] = acc[j] * kUnscale;
             }
           }
         }
@@ -409,7 +424,7 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
         for (int p = 1; p < kParts; ++p) sum += v[p];
         if (n < N) {
           if (!finite(sum)) redo_flag = 1;
-          out[(int64_t)(m0 + m) * ldo + n] = sum;
+          out[(int64_t)(m0 + m) * ldo + n] = sum * kUnscale;
         }
       }
     }

@@ -19,7 +19,7 @@ def _rand(shape, seed):
 
 def _bound(a, w):
     """A chain of 12 products of 32 k cuts its sum off at most 12 times, 2^-23 of it each (24 units of 2^-24); k / 128 chains and three parts are added to nearest;
-    the products of parts that are left out are below 2^-24 a term. All of the sum of the terms' magnitudes."""
+    the products of parts that are left out are each below 2^-24 of a term, two of them of one sign. All of the sum of the terms' magnitudes."""
     return (24 + a.shape[1] / 128 + 8) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().T)
 
 
@@ -77,3 +77,14 @@ def test_rows_that_are_not_finite_do_not_hold_up_the_other_tiles(kernels):
     others = torch.arange(n, device="cuda") != 7
     assert torch.equal(got[~bad][:, others], clean[~bad][:, others])
     assert torch.equal(got[~bad][:, 7], torch.where(a[~bad, 100] > 0, float("inf"), float("-inf")))
+
+
+@pytest.mark.parametrize("m,n,k", [(5, 130, 512), (100, 257, 1028), (40, 20000, 512)])      # clusters, narrow and wide tiles, several tiles a CTA
+@pytest.mark.parametrize("of_a,of_w", [(0, -115), (-118, 0), (60, -126), (-126, 100), (0, -138), (-70, -70), (100, -100), (110, -60)])
+def test_operands_of_any_size_keep_their_24_bits(kernels, m, n, k, of_a, of_w):
+    """Operands down to the smallest numbers that there are and up to where sums no longer fit, as accurate as ordinary ones: relative to the sum of the
+    terms' magnitudes, and half a unit of the smallest number."""
+    a, w = _rand((m, k), 13) * 2.0 ** of_a, (_rand((n, k), 14).double() * 2.0 ** of_w).float()
+    got, want = kernels.gemm_simt(a, w), a.double() @ w.double().T
+    assert ((got.double() - want).abs() <= _bound(a, w) + 2.0 ** -149).all()
+    assert torch.equal(kernels.gemm_simt(a[m // 2 : m // 2 + 1], w), got[m // 2 : m // 2 + 1]), "a row alone"

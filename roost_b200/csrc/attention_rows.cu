@@ -47,6 +47,14 @@ __device__ __forceinline__ void ar_cluster_sync() { asm volatile("barrier.cluste
 // What scores are taken relative to: their maximum, or 0 where there was none (no key, or none but -inf or NaN). Every weight is then exp2f of a difference: 0 for
 // -inf, NaN for a NaN score, which so reaches the sums, the denominator and the output whatever the maximum is.
 __device__ __forceinline__ float ar_base(float top) { return top == -INFINITY ? 0.f : top; }
+// Two bfloat16 numbers with infinities (and NaN) as the largest finite number: what the weights' small parts, which may be zero or negative, are multiplied with. The
+// large part meets the value itself.
+__device__ __forceinline__ uint32_t ar_finite(uint32_t v) {
+  const uint32_t most = 0x7F7F7F7Fu, least = 0xFF7FFF7Fu;
+  const __nv_bfloat162 x = __hmax2(__hmin2(*reinterpret_cast<const __nv_bfloat162*>(&v), *reinterpret_cast<const __nv_bfloat162*>(&most)),
+                                   *reinterpret_cast<const __nv_bfloat162*>(&least));
+  return *reinterpret_cast<const uint32_t*>(&x);
+}
 
 template <int D, bool SIGMOID>
 __global__ void __launch_bounds__(kArWarps * 32, 1) attention_rows_kernel(const AttentionRows a) {
@@ -186,8 +194,10 @@ __global__ void __launch_bounds__(kArWarps * 32, 1) attention_rows_kernel(const 
           const uint32_t pick = j & 1 ? 0x7632 : 0x5410;
           const uint32_t b0 = __byte_perm(ar_word(vx[0][u], j >> 1), ar_word(vx[1][u], j >> 1), pick);
           const uint32_t b1 = __byte_perm(ar_word(vx[2][u], j >> 1), ar_word(vx[3][u], j >> 1), pick);
+          const uint32_t f0 = ar_finite(b0), f1 = ar_finite(b1);
 #pragma unroll
-          for (int part = 0; part < PARTS; ++part) mma_bf16(acc[u * 8 + j], p[part], b0, b1);
+          for (int part = 0; part < PARTS - 1; ++part) mma_bf16(acc[u * 8 + j], p[part], f0, f1);
+          mma_bf16(acc[u * 8 + j], p[PARTS - 1], b0, b1);
         }
     }
 #pragma unroll

@@ -149,3 +149,30 @@ def test_a_sigmoid_weight_that_is_not_a_number_reaches_the_output(kernels, lens)
     want = torch.zeros((T, heads), dtype=torch.bool, device="cuda")
     want[0, 3], want[1, 2:4] = True, True
     assert torch.equal(torch.isnan(out), want[:, :, None].expand_as(out))
+
+
+@pytest.mark.parametrize("lens", [[16, 9], [300, 1000]])
+@pytest.mark.parametrize("sigmoid", [False, True])
+def test_an_infinite_value_makes_its_column_infinite(kernels, lens, sigmoid):
+    """A weight is the sum of two or three numbers, of which the small ones may be zero or negative: an infinite value meets the largest alone."""
+    heads, kv_heads, dim, page = 8, 4, 64, 16
+    k_pool, indptr, indices, keys = _cache(lens, kv_heads, page, dim, 1)
+    v_pool, values = k_pool * -1.5, [k * -1.5 for k in keys]
+    q, T = _rand((len(lens), heads, dim), 7), len(lens)
+    for r, j, head, d, x in ((0, 2, 0, 5, "inf"), (0, 7, 1, 60, "-inf"), (1, 4, 2, 0, "inf"), (1, 3, 3, 9, "inf"), (1, 8, 3, 9, "-inf")):
+        values[r][j, head, d] = float(x)
+        v_pool[indices[indptr[r]], head, j, d] = float(x)
+    if sigmoid:
+        zeros = torch.zeros(heads, device="cuda")
+        out = kernels.sigmoid_attention(q, k_pool, v_pool, None, None, zeros, zeros, _i32([n - 1 for n in lens]), _i32(list(range(T))), indptr, indices, kv_heads, dim,
+                                        dim ** -0.5, kv_cap=1024).reshape(T, heads, dim)
+        want = torch.stack([torch.stack([torch.sigmoid(keys[r][:, h // 2].double() @ q[r, h].double() * dim ** -0.5) @ values[r][:, h // 2].double()
+                                         for h in range(heads)]) for r in range(T)])
+    else:
+        out = kernels.attention_rows(q, k_pool, v_pool, _i32(lens), indptr, indices, dim ** -0.5, 1024).reshape(T, heads, dim)
+        want = _softmax_64(q, keys, values, heads, kv_heads)
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.isinf(want).any() and torch.isnan(want).any()
+    assert torch.equal(out[torch.isinf(want)].double(), want[torch.isinf(want)])
+    fine = torch.isfinite(want)
+    # one rounding; 32-bit weights (2^-15 of the sum of |v|, which is below 2 a key here) and sums
+    assert ((out.double() - want).abs()[fine] <= 2.0 ** -15 * 2 * max(lens) + 2.0 ** -8 * want.abs()[fine]).all()

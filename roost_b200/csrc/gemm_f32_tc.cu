@@ -178,11 +178,11 @@ __device__ __forceinline__ void tmem_store16(uint32_t taddr, const float* v) {
 }
 
 // Pointers carry no __restrict__: `a` is what an earlier kernel of the step writes, and a load must not move before pdl_wait().
-// `pitch`: rows of w in a tile, at most 128 (whole tiles; 128 with CL). `a_whole`: rows of `a` are whole 16-byte pieces (tma_a is made); w's are always.
+// `a_whole`: rows of `a` are whole 16-byte pieces (tma_a is made); w's are always.
 template <int NT, bool CL>
 __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
     gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_a, const float* a, const float* w, float* out, int M,
-                       int N, int K, int64_t lda, int64_t ldw, int64_t ldo, int pitch, bool a_whole, int* error) {
+                       int N, int K, int64_t lda, int64_t ldw, int64_t ldo, bool a_whole, int* error) {
   using C = Cfg<NT>;
   constexpr int R = C::kRawStages;
   extern __shared__ unsigned char smem_raw[];
@@ -231,19 +231,19 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
   const uint32_t tmem = tmem_slot;
   volatile int* abortp = &abort_flag;
   // the tiles of this CTA (m fastest, so that neighbouring CTAs read the same rows of w) and its blocks of k
-  const int m_tiles = (M + NT - 1) / NT, tiles = m_tiles * ((N + pitch - 1) / pitch), blocks = (K + kBlock - 1) / kBlock;
+  const int m_tiles = (M + NT - 1) / NT, tiles = m_tiles * ((N + kWRows - 1) / kWRows), blocks = (K + kBlock - 1) / kBlock;
   const int first = CL ? blockIdx.x / kParts : blockIdx.x, step = CL ? tiles : gridDim.x, rank = CL ? blockIdx.x % kParts : 0;
   auto part_end = [&](int p) { return (int)((long long)blocks * (p + 1) / kParts); };
   const int kb0 = CL ? (int)((long long)blocks * rank / kParts) : 0, kb1 = CL ? part_end(rank) : blocks;
 
   if (warp == kProducer) {
     if (lane == 0) {
-      const uint32_t w_bytes = (uint32_t)pitch * kBlock * 4, bytes = w_bytes + (a_whole ? C::kRawStage - kWRaw : 0u);
+      const uint32_t bytes = a_whole ? C::kRawStage : kWRaw;
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int t = first; t < tiles && ok; t += step) {
-        const int m0 = t % m_tiles * NT, n0 = t / m_tiles * pitch;
+        const int m0 = t % m_tiles * NT, n0 = t / m_tiles * kWRows;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!(ok = mbar_wait_limited(raw_empty(s), phase ^ 1u, abortp, 1, error))) break;
           mbar_expect_tx(raw_full(s), bytes);
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
     int it = 0;
     bool ok = true;
     for (int t = first; t < tiles && ok; t += step) {
-      const int m0 = t % m_tiles * NT + col0, n = row < pitch ? t / m_tiles * pitch + row : N;
+      const int m0 = t % m_tiles * NT + col0, n = t / m_tiles * kWRows + row;
       int part = 0;
 #pragma unroll
       for (int j = 0; j < C::kColumns; ++j) acc[j] = 0.f;
@@ -442,8 +442,8 @@ __global__ void __launch_bounds__(Cfg<NT>::kThreads, Cfg<NT>::kCtasAnSm)
   }
   if (redo_flag && !*abortp) {
     for (int t = first; t < tiles; t += step) {
-      const int m0 = t % m_tiles * NT, n0 = t / m_tiles * pitch + (CL ? rank * (kWRows / kParts) : 0);
-      if (n0 < N) redo_not_finite<C::kThreads>(a, w, out, m0, min(m0 + NT, M), n0, min(n0 + (CL ? kWRows / kParts : pitch), N), K, lda, ldw, ldo);
+      const int m0 = t % m_tiles * NT, n0 = t / m_tiles * kWRows + (CL ? rank * (kWRows / kParts) : 0);
+      if (n0 < N) redo_not_finite<C::kThreads>(a, w, out, m0, min(m0 + NT, M), n0, min(n0 + (CL ? kWRows / kParts : kWRows), N), K, lda, ldw, ldo);
     }
   }
 }
@@ -471,7 +471,7 @@ static int make_map(CUtensorMap* map, const float* p, int rows, int k, int64_t l
 }
 
 template <int NT, bool CL>
-static int launch(const Args& g, long long tiles, int pitch, int sms) {
+static int launch(const Args& g, int sms) {
   using C = Cfg<NT>;
   auto kernel = gemm_f32_tc_kernel<NT, CL>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
@@ -480,42 +480,28 @@ static int launch(const Args& g, long long tiles, int pitch, int sms) {
   if (!error) return fail(ROOST_ERR_CUDA, "gemm_f32_tc: the error word has no device address");
   const bool whole = g.lda % 4 == 0 && (uintptr_t)g.a % 16 == 0;
   CUtensorMap mw, ma;
-  int rc = make_map(&mw, g.w, g.n, g.k, g.ldw, pitch, CU_TENSOR_MAP_SWIZZLE_128B);
+  int rc = make_map(&mw, g.w, g.n, g.k, g.ldw, kWRows, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != ROOST_OK) return rc;
   ma = mw;
   if (whole && (rc = make_map(&ma, g.a, g.m, g.k, g.lda, NT, CU_TENSOR_MAP_SWIZZLE_NONE)) != ROOST_OK) return rc;
-  const long long resident = (long long)sms * C::kCtasAnSm;
+  const long long tiles = (long long)((g.m + NT - 1) / NT) * ((g.n + kWRows - 1) / kWRows), resident = (long long)sms * C::kCtasAnSm;
   const unsigned grid = (unsigned)(CL ? tiles * kParts : (tiles < resident ? tiles : resident));
   launch_kernel_cluster(kernel, dim3(grid), dim3(C::kThreads), C::kSmem, g.stream, CL ? kParts : 1, mw, ma, g.a, g.w, g.out, g.m, g.n, g.k, g.lda, g.ldw, g.ldo,
-                        pitch, whole, error);
+                        whole, error);
   return check_launch("gemm_f32_tc");
 }
 
-template <int NT>
-static int launch_form(const Args& g, bool cl, int sms) {
-  const long long m_tiles = (g.m + NT - 1) / NT;
-  auto tiles = [&](int pitch) { return m_tiles * ((g.n + pitch - 1) / pitch); };
-  if (cl) return launch<NT, true>(g, tiles(kWRows), kWRows, sms);
-  // A few rows of `a` by many of w wait for w's way from memory, which a last round of few tiles leaves idle: lower tiles in whole rounds then
-  // (151,936 rows of w by 128 are 1,187 tiles, three more than four rounds).
-  int pitch = kWRows;
-  if (NT == 16) {
-    const long long at_once = (long long)sms * Cfg<NT>::kCtasAnSm;
-    auto time = [&](int p) { return (tiles(p) + at_once - 1) / at_once * p; };
-    for (int p = kWRows - 8; p >= 64; p -= 8)
-      if (time(p) < time(pitch)) pitch = p;
-  }
-  return launch<NT, false>(g, tiles(pitch), pitch, sms);
-}
-
-// Rows of `a` a tile, and the cycles of an SM that a block of k of such a tile took (151,936 x 1,024 by 16 to 96 rows; 12 products of 128 x 96 x 16 or
-// fewer cannot take less than 770, whatever NT is). 128 rows leave tensor memory for two stages of planes, which wait for one another, and are twice as
-// slow as 64; they serve where 64 would need a second round of clusters.
+// Rows of `a` a tile, the cycles of an SM that a block of k of such a tile took (on a matrix of many rounds, 151,936 x 1,024, by 16 to 96 rows; 12 products of 128 x 96 x 16
+// or fewer cannot take less than 770, whatever NT is), and how many CTAs of clusters an SM may be given in turn: they are not persistent. Narrow tiles
+// start and end quickly: a row by 20,000 x 4,096 104 us in whole tiles, 78 in clusters; by 40,000 x 4,096 154 and 133. Wider ones do not: 512 rows by 4,096 x 4,096 152 us
+// in whole tiles, 190 in clusters. 128 rows leave tensor memory for two stages of planes, which wait for one another, and are more than twice as slow as 64; they serve
+// where 64 would need a second round of clusters, and only in clusters (in whole tiles 64 rows are expected to be quicker for any k that is taken).
 struct Form {
   int rows;
   double cycles;
+  int clusters;
 };
-constexpr Form kForms[] = {{16, 760}, {32, 930}, {64, 1250}, {96, 1540}, {128, 2700}};
+constexpr Form kForms[] = {{16, 760, 16}, {32, 930, 4}, {64, 1250, 4}, {96, 1540, 4}, {128, 2700, 4}};
 
 // What a product is expected to take: rounds of tiles on an SM, blocks of k, and what starts and ends a tile.
 static double expected(const Form& f, bool cl, int m, int n, int k, int sms) {
@@ -529,8 +515,9 @@ static double expected(const Form& f, bool cl, int m, int n, int k, int sms) {
 // The rule on w alone that decides between the two products: an output's bits may not depend on how many rows are asked for together.
 // Below 512 k the chain of FFMAs is short: not measured against, and no model's projections. Vocabulary-sized heads, of which a step wants a few rows, stay
 // with the FFMAs, which read the weights at 5.2 TB/s there (3 x 151,936 x 1,024: 118 us, 130 here, where a block's 12 products take 770 cycles however few
-// their rows; 64 rows would have taken 190 instead of 911). In between the tensor cores are faster for any number of rows: a row by 24,576 x 4,096 101 us
-// (120), by 1,024 x 3,072 16 (50); 512 rows by 4,096 x 1,024 47 (113), by 1,024 x 3,072 35 (185), by 4,096 x 4,096 152 (443).
+// their rows). In between, us here (by FFMAs), for 1, 16 and 512 rows: 1,024 x 3,072 16 (50), 16 (50), 35 (185); 4,096 x 4,096 25 (72), 25 (76), 152 (448); 12,288 x 1,024
+// 23 (25), 23 (37), 103 (336); 24,576 x 4,096 94 (92), 95 (160), 703 (2,383); 40,000 x 1,024 47 (39), 47 (74), 317 (936); 50,304 x 4,096 154 (170), 156 (324), 1,525 (4,742).
+// A single row by 16,000 to 50,000 of a short k is the one shape that the FFMAs take less time for; the rows of a step, whose bits may not differ, are worth more.
 bool gemm_f32_tc_takes(const void* w, int n, int k, int64_t ldw) {
   return k >= 512 && n < 65536 && k % 4 == 0 && ldw % 4 == 0 && (uintptr_t)w % 16 == 0;
 }
@@ -552,7 +539,7 @@ int launch_gemm_f32_tc(const float* a, const float* w, float* out, int m, int n,
   for (const Form& f : kForms) {
     for (int c = 0; c < 2; ++c) {
       const long long tiles = (long long)((m + f.rows - 1) / f.rows) * ((n + kWRows - 1) / kWRows);
-      if (c && tiles * kParts > 4LL * count) continue;      // clusters are not persistent: a few rounds of them at most
+      if (c ? tiles * kParts > (long long)f.clusters * count : f.rows == 128) continue;
       const double t = expected(f, c != 0, m, n, k, count);
       if (rows == 0 || t < least) {
         least = t;
@@ -562,11 +549,11 @@ int launch_gemm_f32_tc(const float* a, const float* w, float* out, int m, int n,
     }
   }
   switch (rows) {
-    case 16: return launch_form<16>(g, cl, count);
-    case 32: return launch_form<32>(g, cl, count);
-    case 64: return launch_form<64>(g, cl, count);
-    case 96: return launch_form<96>(g, cl, count);
-    default: return launch_form<128>(g, cl, count);
+    case 16: return cl ? launch<16, true>(g, count) : launch<16, false>(g, count);
+    case 32: return cl ? launch<32, true>(g, count) : launch<32, false>(g, count);
+    case 64: return cl ? launch<64, true>(g, count) : launch<64, false>(g, count);
+    case 96: return cl ? launch<96, true>(g, count) : launch<96, false>(g, count);
+    default: return launch<128, true>(g, count);
   }
 }
 

@@ -45,6 +45,13 @@ def test_persistent_ctas_take_several_tiles(kernels):
     assert torch.equal(kernels.gemm_simt(a[:9], w), got[:9])
 
 
+def test_clusters_of_narrow_tiles_in_several_rounds(kernels):
+    a, w = _rand((300, 2048), 15), _rand((24700, 2048), 16)             # 193 tiles by 16 rows or fewer, 772 CTAs
+    got = kernels.gemm_simt(a, w)
+    assert ((got.double() - a.double() @ w.double().T).abs() <= _bound(a, w)).all()
+    assert torch.equal(kernels.gemm_simt(a[:16], w), got[:16]) and torch.equal(kernels.gemm_simt(a[299:], w), got[299:])
+
+
 def test_what_is_not_finite_comes_out_as_a_chain_of_sums_has_it(kernels):
     """Infinities, NaN and numbers whose rounding to bfloat16 overflows reach the outputs of their row and column, and no others."""
     k = 512

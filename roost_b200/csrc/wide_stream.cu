@@ -452,14 +452,18 @@ extern "C" int roost_softcap(float* logits, int64_t n, float cap, roost_stream_t
   return check_launch("softcap");
 }
 
-// bfloat16 rows in whole pieces of 16 bytes that 512 threads hold. (float32 rows keep one form, whatever their number: their bits do not depend on what
-// else is in a step.)
+// bfloat16 rows in whole pieces of 16 bytes that 512 threads hold. With several pieces a thread fewer rows are on their way at once than in the kernel for any sizes,
+// which counts once the processors have their blocks one after the other, with a gate (more to read and to hold) sooner. Any sizes / this, us: 64 rows of 8,192
+// 7.9 / 3.6; 256 rows of 8,192 12.8 / 8.4, of 5,120 7.2 / 6.4; 320 rows of 5,120 8.4 / 8.7; 3,000 rows of 4,096 46 / 39; with a gate 148 rows of 5,120 6.9 / 5.6, 192 7.4 / 9.5;
+// 512 rows of 4,096 10.0 / 9.0, 1,000 16.6 / 17.9; 1,000 rows of 2,048 9.7 / 9.2, 3,000 25.6 / 26.1; 3,000 of 1,024 13.8 / 12.5.
+// (float32 rows keep one form, whatever their number: their bits do not depend on what else is in a step.)
 static bool wide_rms_norm_vec(float* stream, const void* addend, const float* extra, const float* w, void* out, const int32_t* rows, int n_out, int hidden, float eps,
                               const float* gate, const float* gate_bias, int dtype, roost_stream_t s) {
   if (dtype != ROOST_BF16 || hidden % 4 != 0 || hidden > 8192) return false;
   if ((((uintptr_t)stream | (uintptr_t)extra | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)gate_bias) % 16) != 0) return false;
   if ((((uintptr_t)addend | (uintptr_t)out) % 8) != 0) return false;
   const int pieces = hidden / 4, v = pieces <= 512 ? 1 : (pieces <= 1024 ? 2 : 4);
+  if (v == 4 ? n_out > (gate ? 148 : 256) : (gate && hidden > 1024 && n_out > (v == 2 ? 512 : 1024))) return false;
   const int threads = ((pieces + v - 1) / v + 31) / 32 * 32;
   auto kernel = v == 1 ? wide_rms_norm_vec_kernel<1> : (v == 2 ? wide_rms_norm_vec_kernel<2> : wide_rms_norm_vec_kernel<4>);
   launch_kernel(kernel, dim3(n_out), dim3(threads), 0, (cudaStream_t)s, stream, (const __nv_bfloat16*)addend, extra, w, (__nv_bfloat16*)out, rows, hidden, eps, gate,

@@ -46,6 +46,20 @@ def test_norm_over_a_32_bit_stream(kernels, hidden, form):
     assert ((out.to(F64) - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18).all()
 
 
+# where long rows change to the kernel for any sizes: one, two, four pieces a thread
+@pytest.mark.parametrize("hidden,gated,n", [(1024, True, 1025), (1028, True, 1024), (1028, True, 1025), (4096, True, 512), (4096, True, 513), (4096, False, 700),
+                                            (4100, False, 256), (4100, False, 257), (8192, True, 148), (8192, True, 149)])
+def test_norm_over_a_32_bit_stream_of_many_rows(kernels, hidden, gated, n):
+    stream, w = _rand((n, hidden), 1), 1 + 0.1 * _rand((hidden,), 2)
+    addend, gate, bias = _rand((n, hidden), 3, torch.bfloat16), _rand((n, hidden), 5), _rand((hidden,), 6)
+    s = stream.to(F64) + addend.to(F64) * (torch.sigmoid(gate.to(F64) + bias.to(F64)) if gated else 1.0)
+    out = kernels.wide_rms_norm_gated(stream, w, 1e-6, torch.bfloat16, addend, gate, bias) if gated else kernels.wide_rms_norm(stream, w, 1e-6, torch.bfloat16, addend)
+    want = s / torch.sqrt((s * s).mean(-1, keepdim=True) + 1e-6) * w.to(F64)
+    assert (stream.to(F64) - s).abs().max() <= 2.0 ** -21 * s.abs().max()
+    # one rounding to bfloat16 beside sums in 32 bits
+    assert ((out.to(F64) - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18).all()
+
+
 @pytest.mark.parametrize("dim", [64, 128, 256])
 @pytest.mark.parametrize("tokens,heads,kv_heads", [(1, 1, 1), (7, 5, 1), (63, 8, 4)])
 @pytest.mark.parametrize("normed", [True, False])

@@ -48,10 +48,12 @@ typedef void* roost_stream_t;
 int roost_abi_version(void);
 /* Programmatic dependent launch for the library's kernels (off by default): a kernel may start its preamble, and the
  * weight-streaming product its first loads of weights, while the kernel before it on the stream is finishing.
- * With it on, a kernel reads before it waits for the kernel in front: weights (norm weights, the products' weight
- * matrices), index tables (the `rows` of the norms, the work lists of the attention kernels, q_indptr, kv_lens,
- * kv_indptr, kv_indices) and pages of the cache that hold only tokens of earlier steps. A caller must therefore not
- * have those written by the kernel launched directly before the call that reads them (a copy in between is enough);
+ * With it on, a kernel reads before it waits for the kernel in front: weights (norm weights, biases and slopes, the products'
+ * weight matrices, rotations' inv_freq), index tables (positions, slot_mapping, token_row, the `rows` of the norms, the work lists
+ * of the attention kernels, q_indptr, kv_lens, kv_indptr, kv_indices, the `slots` of states) and pages of the cache that hold only tokens
+ * of earlier steps. A caller must therefore not have those written by a kernel of this library that is still on its way: every one of
+ * them lets the next begin at once, so that not only the kernel directly in front may be running when a table is read, but the ones
+ * ahead of it as well. A copy, a memset or a kernel that is not this library's between the writer and the reader is enough;
  * activations and the pages of the step's own tokens are read after the wait. */
 void roost_set_pdl(int on);
 /* Message of the last non-OK status on this thread. */

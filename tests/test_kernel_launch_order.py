@@ -87,3 +87,22 @@ def test_a_layer_whose_rows_are_one_segment_each_gives_the_same_bits_with_and_wi
         kernels.set_pdl(was)
     for (y, s), (y2, s2) in zip(got[False], got[True]):
         assert torch.isfinite(y).all() and torch.equal(y, y2) and torch.equal(s, s2)
+
+
+def test_the_header_names_the_tables_that_are_read_ahead_of_the_wait():
+    """A caller's kernel must not be writing them: the ABI's contract of programmatic launch has to name each."""
+    header = (CSRC / "roost_kernels.h").read_text()
+    contract = re.search(r"/\* Programmatic dependent launch.*?\*/", header, re.S).group(0)
+    early = set()
+    for path in FILES:
+        src = re.sub(r"//[^\n]*", "", path.read_text())
+        for name, body in _kernels(path):
+            wait = re.search(r"pdl_wait\(\d*\)", body)
+            if not wait:
+                continue
+            head = src[: src.index(body)][-2000:]
+            for table in re.findall(r"const int32_t\*\s*(?:__restrict__\s*)?(\w+)", head[head.rindex(name) :]):
+                if re.search(rf"\b{table}\[", body[: wait.start()]):
+                    early.add((path.name, name, table))
+    assert any(table == "positions" for _, _, table in early)
+    assert not {e for e in early if e[2] not in contract}

@@ -477,8 +477,8 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
   }
 }
 
-// Where the vector forms begin to win: numbers of a step's convolution (2,048 channels: 256 tokens 6.3 us, 5.8 a number a thread; 512 9.5 and 9.9; 1,000 13.8 and 17.3;
-// 6,144 channels: 192 tokens 8.7 and 10.8), and groups of a step's norm where a warp takes one (8 of 512 a token: 148 tokens 4.3 us, 3.9 with a block a group;
+// Where the vector forms begin to win: numbers of a step's convolution (2,048 channels: 256 tokens 10.2 us either way, launch and all; 512 10.3 and 14.4 a number a
+// thread; 1,000 12.3 and 22.5; 6,144 channels: 100 tokens 10.2 either way, 171 10.2 and 14.4), and groups of a step's norm where a warp takes one (8 of 512 a token: 148 tokens 4.3 us, 3.9 with a block a group;
 // 192 4.5 and 4.7; 1,200 9.9 and 19.9).
 constexpr long long kConvVecMin = 1 << 20, kNormVecMin = 1536;
 
@@ -499,13 +499,12 @@ extern "C" int roost_mamba2_conv(const void* u, int64_t ld, int col, void* out, 
     if ((long long)tokens * channels >= kConvVecMin && (dtype == ROOST_F32 || dtype == ROOST_BF16) && taps == 4 && channels % vec == 0 && ld % vec == 0 && col % vec == 0 && at % 16 == 0 && state_stride % 4 == 0 &&
         conv_off % 4 == 0) {
       const unsigned gy = (unsigned)((channels / vec + 127) / 128);
-      // sixteen or four tokens a thread where that leaves every processor several blocks, else one (whose weights are ten times what it reads and writes:
-      // 2,348 tokens x 2,048 channels 28 us, 12 with four); few numbers are spread over more threads by the form for any sizes
-      const int each = (long long)(tokens / 16) * gy >= 4 * 148 ? 16 : ((long long)(tokens / 4) * gy >= 2 * 148 ? 4 : 1);
+      // sixteen tokens a thread where that leaves every processor several blocks, else four (one, whose weights are ten times what it reads and writes, took 14.4 us
+      // for 10.2 at 512 tokens x 2,048 channels and 32.7 for 18.5 at 2,348); few numbers are spread over more threads by the form for any sizes
+      const int each = (long long)(tokens / 16) * gy >= 4 * 148 ? 16 : 4;
       ROOST_DISPATCH_DTYPE(dtype, T, {
-        auto kernel = each == 16 ? mamba2_conv_vec_kernel<T, 16> : (each == 4 ? mamba2_conv_vec_kernel<T, 4> : mamba2_conv_vec_kernel<T, 1>);
-        launch_kernel(kernel, dim3((tokens + each - 1) / each, gy), dim3(128), 0, (cudaStream_t)stream, (const T*)u, ld, col, (T*)out, w, bias, state,
-                      state_stride, conv_off, token_row, q_indptr, slots, tokens, channels, act);
+        launch_kernel(each == 16 ? mamba2_conv_vec_kernel<T, 16> : mamba2_conv_vec_kernel<T, 4>, dim3((tokens + each - 1) / each, gy), dim3(128), 0,
+                      (cudaStream_t)stream, (const T*)u, ld, col, (T*)out, w, bias, state, state_stride, conv_off, token_row, q_indptr, slots, tokens, channels, act);
       });
       return check_launch("mamba2_conv");
     }

@@ -1,5 +1,5 @@
 """Kernels of a step of few rows whose inputs are in registers ahead of the kernel in front, against 64 bits: the rotation of few tokens, the norms over a
-32-bit stream, the states that begin at zero, the convolution four tokens a thread."""
+32-bit stream, the states that begin at zero."""
 import math
 
 import pytest

@@ -410,9 +410,10 @@ def test_every_order_of_the_grouped_product_takes_every_tile(kernels, E, T, top,
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("lengths,channels", [([1, 2, 3, 4, 37], 24), ([600, 1, 2, 3, 414], 1032), ([3000, 1, 2000], 1032)])
+@pytest.mark.parametrize("lengths,channels", [([1, 2, 3, 4, 37], 24), ([600, 1, 2, 3, 414], 1032), ([100, 1, 2, 78], 6144), ([3000, 1, 2000], 1032)])
 def test_convolution_forms_agree_bit_for_bit(kernels, dtype, lengths, channels):
-    """Sixteen tokens a thread, one, and a number at a time (columns that start off a whole piece): the same sums."""
+    """Sixteen tokens a thread, four (token counts that are no multiple of four, rows that begin inside a thread's), and a number at a time (columns that start off a
+    whole piece): the same sums."""
     T = sum(lengths)
     g = torch.Generator().manual_seed(T)
     u = torch.randn(T, channels + 16, generator=g).to(dtype).cuda()

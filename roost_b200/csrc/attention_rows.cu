@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(kArWarps * 32, 1) attention_rows_kernel(const 
     m[0] = m[1] = -INFINITY;
     l[0] = l[1] = 0.f;
     for (int i = 0, blk = first; pass ? blk < blocks : i == 0; ++i, blk += stride) {
+      // (a warp has at most eight blocks of the keys that kv_cap bounds; only rows longer than it was told come here)
       if (i > 0 && (i & 31) == 0) entry_of = blk + lane * stride < blocks ? pages[(blk + lane * stride) * 16 >> a.page_shift] : 0;
       const int page = __shfl_sync(0xffffffffu, entry_of, i & 31), key0 = blk * 16, seen = pass ? len - key0 : 0;       // the block's keys that there are
       const size_t at = (((size_t)page * a.kv_heads + kvh) * a.page_size + (key0 & (a.page_size - 1))) * a.entry;
@@ -280,8 +281,9 @@ __global__ void __launch_bounds__(kArWarps * 32, 1) attention_rows_kernel(const 
 // processors of one group, which the kernels around this one leave for few: sixteen of them were slower than sixteen of four (2 rows of Qwen3 0.6B: 220 us
 // a step of six layers, 196 in clusters of four).
 static int rows_splits(int tokens, int kv_heads, int kv_cap) {
+  const int sms = processors();
   int splits = 1;
-  while (splits < kArMaxSplits && (long long)tokens * kv_heads * splits * 2 <= (splits * 2 == 8 ? 74 : 148) && splits * 128 < kv_cap) splits *= 2;
+  while (splits < kArMaxSplits && (long long)tokens * kv_heads * splits * 2 <= (splits * 2 == 8 ? sms / 2 : sms) && splits * 128 < kv_cap) splits *= 2;
   return splits;
 }
 
@@ -294,7 +296,7 @@ extern "C" int roost_attention_rows_supported(int tokens, int q_heads, int kv_he
   if (tokens < 1 || kv_heads < 1 || q_heads % kv_heads != 0 || q_heads / kv_heads > 16 || (head_dim != 64 && head_dim != 128)) return 0;
   if (page_size < 16 || (page_size & (page_size - 1)) != 0 || kv_cap < 1 || kv_heads > 65535 || tokens > 65535) return 0;
   const int blocks = (kv_cap + 15) / 16, each = rows_splits(tokens, kv_heads, kv_cap) * kArWarps, turns = (blocks + each - 1) / each;
-  return (long long)tokens * kv_heads <= 148 && turns <= (sigmoid ? 8 : 2);
+  return (long long)tokens * kv_heads <= processors() && turns <= (sigmoid ? 8 : 2);
 }
 
 extern "C" int roost_attention_rows(const void* q, void* out, const void* k_base, const void* v_base, int entry, const int32_t* lens, const int32_t* token_row,

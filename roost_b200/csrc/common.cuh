@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <atomic>
 #include <string>
 
 #include "roost_kernels.h"
@@ -75,6 +76,20 @@ __device__ __forceinline__ void pdl_launch_dependents(int tag = 0) {
 inline int fail(int code, const std::string& msg) {
   set_error(msg);
   return code;
+}
+
+// Processors of the calling thread's device; 0 without one.
+inline int processors() {
+  static std::atomic<int> known[64];
+  int dev = 0, count = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (dev < 64 && (count = known[dev].load(std::memory_order_relaxed)) != 0) return count;
+  cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+  if (dev < 64) known[dev].store(count, std::memory_order_relaxed);
+  return count;
 }
 
 inline int check_launch(const char* what) {

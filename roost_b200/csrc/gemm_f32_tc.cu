@@ -524,14 +524,7 @@ bool gemm_f32_tc_takes(const void* w, int n, int k, int64_t ldw) {
 
 int launch_gemm_f32_tc(const float* a, const float* w, float* out, int m, int n, int k, int64_t lda, int64_t ldw, int64_t ldo, cudaStream_t stream) {
   using namespace f32tc;
-  static int sms[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int count = dev >= 0 && dev < 64 ? sms[dev] : 0;
-  if (count == 0) {
-    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
-    if (dev >= 0 && dev < 64) sms[dev] = count;
-  }
+  const int count = processors();
   const Args g = {a, w, out, m, n, k, lda, ldw, ldo, stream};
   int rows = 0;
   bool cl = false;

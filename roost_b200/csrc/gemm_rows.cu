@@ -1,5 +1,5 @@
-// out[m,n] = sum_k x[m,k] * w[n,k] in bfloat16 with 32-bit accumulation for the few rows of a decode step (m <= 16) and weights of up to about 14 MB: the
-// products of a small model, whose time is latency. Definition: src/Starlings.Roost.Ops/CpuOps.cs:395-437 (TransposeB, alpha 1, no bias, 32-bit
+// out[m,n] = sum_k x[m,k] * w[n,k] in bfloat16 with 32-bit accumulation for the few rows of a decode step (m <= 16) and weights that the processors hold
+// (19 MB at 16 pieces a lane, 14 at 8 or 12): the products of a small model, whose time is latency. Definition: src/Starlings.Roost.Ops/CpuOps.cs:395-437 (TransposeB, alpha 1, no bias, 32-bit
 // accumulation, one rounding); with SWIGLU silu(gate) * up of two products (src/Starlings.Roost.Models.Tiny/RoostTiny.cs:51-53).
 //
 // Every CTA keeps its rows of w in registers: 8 to 32 rows, k dealt to its eight warps, at most 16 pieces of 16 bytes a lane, all asked for before
@@ -138,11 +138,11 @@ static RowsShape rows_shape(int m, int n, int k, bool swiglu) {
   if (n < 1 || k % (32 * kRowsWarps) != 0) return {0, 0};
   const int kb = k / (32 * kRowsWarps);
   if (kb != 1 && kb != 2 && kb != 3 && kb != 4 && kb != 6 && kb != 8 && kb != 12 && kb != 16) return {0, 0};
-  const int groups = (n + 7) / 8;
+  const int groups = (n + 7) / 8, sms = processors();
   for (int r8 : {1, 2, 4}) {
     if (swiglu && r8 == 1) continue;
     if (r8 * kb > kRowsMaxPieces) break;
-    if ((groups + r8 - 1) / r8 <= (r8 * kb <= 8 && m <= 8 ? 3 : 2) * 148) return {r8, kb};
+    if ((groups + r8 - 1) / r8 <= (r8 * kb <= 8 && m <= 8 ? 3 : 2) * sms) return {r8, kb};
   }
   return {0, 0};
 }

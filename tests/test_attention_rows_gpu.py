@@ -52,7 +52,7 @@ def test_softmax(kernels, lens, heads, kv_heads, dim, page):
     v_pool, values = v_pool * -1.5, [v * -1.5 for v in values]
     q, cap = _rand((len(lens), heads, dim), 7), 1024 * (-(-max(lens) // 1024))
     if not kernels.attention_rows_supported(q, k_pool, kv_heads, cap):
-        assert len(lens) * kv_heads > 18, "sizes that the kernel serves"
+        assert len(lens) == 9 and kv_heads == 8, "sizes that the kernel serves: all but these, whose warps would have four blocks of keys"
         return
     out = kernels.attention_rows(q, k_pool, v_pool, _i32(lens), indptr, indices, dim ** -0.5, cap).reshape(len(lens), heads, dim)
     for r, n in enumerate(lens):
@@ -176,3 +176,14 @@ def test_an_infinite_value_makes_its_column_infinite(kernels, lens, sigmoid):
     fine = torch.isfinite(want)
     # one rounding; 32-bit weights (2^-15 of the sum of |v|, which is below 2 a key here) and sums
     assert ((out.double() - want).abs()[fine] <= 2.0 ** -15 * 2 * max(lens) + 2.0 ** -8 * want.abs()[fine]).all()
+
+
+def test_rows_longer_than_the_bound_that_was_told(kernels):
+    """More blocks of keys than a warp reads table entries for at a time: slower, and right all the same."""
+    lens, heads, kv_heads, dim, page = [5000, 17], 4, 2, 64, 16
+    k_pool, indptr, indices, keys = _cache(lens, kv_heads, page, dim, 1)
+    q = _rand((len(lens), heads, dim), 7)
+    out = kernels.attention_rows(q, k_pool, k_pool * -1.5, _i32(lens), indptr, indices, dim ** -0.5, 16).reshape(len(lens), heads, dim)
+    want = _softmax_64(q, keys, [k * -1.5 for k in keys], heads, kv_heads)
+    # as above; what |v| a weight meets is below 8 here
+    assert ((out.double() - want).abs() <= 2.0 ** -15 * 8 + 2.0 ** -8 * want.abs()).all()

@@ -24,9 +24,7 @@ SIZES = [(1, 256), (64, 512), (250, 768), (1024, 1024), (4104, 1024), (9472, 512
 @pytest.mark.parametrize("n,k", SIZES)
 def test_against_64_bits_and_rows_alone(kernels, m, n, k):
     x, w = _rand((m, k), 1), _rand((n, k), 2, 0.05)
-    if not kernels.gemm_rows_supported(x, w):
-        assert (n, k) == (4700, 2048) or (m > 8 and n > 4736), "sizes that a form serves"
-        return
+    assert kernels.gemm_rows_supported(x, w), "sizes that a form serves"
     want, size = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
     got = kernels.gemm_rows(x, w, torch.float32)
     # chains of k / 128 products a warp whose sums are cut off (2^-23 of the terms' magnitude each, a product of 16 k), nine additions to nearest
@@ -62,5 +60,7 @@ def test_what_is_not_served(kernels):
     assert not kernels.gemm_rows_supported(_rand((4, 264), 6), _rand((64, 264), 6))
     assert not kernels.gemm_rows_supported(_rand((4 * 256 + 1,), 6)[1:].reshape(4, 256), w), "rows that do not start on 16 bytes"
     assert not kernels.gemm_rows_supported(_rand((1, 1024), 6), _rand((151936, 1024), 6))
+    assert not kernels.gemm_rows_supported(_rand((1, 1024), 6), _rand((9480, 1024), 6)), "a row more than the processors hold"
+    assert not kernels.gemm_rows_supported(_rand((1, 1280), 6), _rand((64, 1280), 6)), "five pieces a warp"
     with pytest.raises(Exception):
         kernels.gemm_rows(_rand((17, 256), 6), w)

@@ -10,6 +10,7 @@ import pytest
 import torch
 
 from roost_b200.engine.executor import StepEntry, StepExecutor
+from roost_b200.kernels import library
 from tests import helpers as H
 from tests import vamatar_models as VM
 from tests.conftest import ROOT
@@ -97,6 +98,13 @@ def test_latent_attention_with_split_keys_against_the_plain_sum(kernels, dtype, 
     assert kernels.latent_splits_for(T, heads, window, 1024) > 1
     close(one, want, dtype, "latent attention, one block a token", bf16=1e-2)
     close(split, want, dtype, "latent attention, split keys", bf16=1e-2)
+    # more splits than this library's caller asks for, as the entry point takes them: another merge
+    for splits in (32, 33, 70):
+        out, part = torch.empty_like(one), torch.empty(T * heads * splits * (rank + 2), device="cuda")
+        ptr, stream = library._ptr, library._stream()
+        kernels._call("roost_latent_attention", ptr(q_latent), ptr(q), ptr(out), ptr(part), ptr(pool), ptr(positions), ptr(token_row), ptr(indptr), ptr(indices), T, heads,
+                      nope, rope, rank, page, scale, window or 0, splits, None, library.dtype_code(dtype), stream, launches=2)
+        close(out, want, dtype, f"latent attention, {splits} splits", bf16=1e-2)
 
 
 @pytest.mark.parametrize("rank", [32, 80, 272])

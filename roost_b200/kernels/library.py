@@ -508,7 +508,7 @@ class KernelLibrary:
         return out
 
     def gemm_simt(self, a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
-        """a [M, K] times w [N, K] transposed, 32-bit FFMA accumulation."""
+        """a [M, K] times w [N, K] transposed in 32 bits: on the tensor cores with all 24 bits of float32 operands where w allows it, else FFMAs."""
         _need(w, "w", a.dtype)
         if not a.is_cuda or a.dim() != 2 or (a.shape[1] > 1 and a.stride(1) != 1):       # rows may be strided (a column range of wider rows)
             raise KernelError("a is not a CUDA matrix with dense rows")
